@@ -433,7 +433,6 @@ static int bc_cores(const std::vector<CoreTask> &v) {
         if (t.RU) BC(t.RU, bc_span(t.K, t.K, t.ldru), "core RU", i);
         BC(t.RV, bc_span(t.K, t.K, t.ldrv), "core RV", i);
         BC(t.SU, bc_span(t.K, t.K, t.K), "core SU", i);
-        if (t.RUc) BC(t.RUc, bc_span(t.K, t.K, t.K), "core RU copy", i);
         if (t.work) BC(t.work, core_work_doubles(t.K) * sizeof(double), "core scratch", i);
         if (t.rank_out) BC(t.rank_out, sizeof(int), "core rank", i);
         if (t.rank_task) BC(t.rank_task, sizeof(int), "core task rank", i);
@@ -858,17 +857,30 @@ size_t recomp_ws_bytes(int nb, const RecompTask &t) {
     return b + 1024;
 }
 
-// Core-SVD launches bucketed by K so that small cores run several CTAs per SM.
+// Core-SVD launches bucketed by K, so that small cores run several CTAs per SM.
+// Buckets of the one-CTA kernel are merged upwards while the merged launch has
+// no more tasks than SMs: it is then one CTA per SM either way, and a launch
+// lasts as long as its slowest core.
 int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreParams &cp) {
-    static const int edges[] = {32, 64, 96, 128, 160, 1 << 30};
-    std::vector<CoreTask> bucket;
-    int lo = -1;
-    for (int e : edges) {
+    std::stable_sort(cores.begin(), cores.end(),
+                     [](const CoreTask &a, const CoreTask &b) { return core_bucket(a.K) < core_bucket(b.K); });
+    size_t i = 0;
+    while (i < cores.size()) {
+        size_t e = i;
+        int b = core_bucket(cores[i].K);
+        while (e < cores.size() && core_bucket(cores[e].K) == b) ++e;
+        while (e < cores.size() && core_bucket(cores[e].K) <= core_smem_kmax()) {
+            const int nb = core_bucket(cores[e].K);
+            size_t f = e;
+            while (f < cores.size() && core_bucket(cores[f].K) == nb) ++f;
+            if (f - i > (size_t)c->nsm) break;
+            e = f;
+        }
+        std::vector<CoreTask> bucket(cores.begin() + (long)i, cores.begin() + (long)e);
         int kmax = 0;
-        for (auto &t : cores)
-            if (t.K > lo && t.K <= e) { bucket.push_back(t); kmax = std::max(kmax, t.K); }
-        if (!bucket.empty()) TRY(run_core(c, bucket, kmax, cp));
-        lo = e;
+        for (auto &t : bucket) kmax = std::max(kmax, t.K);
+        TRY(run_core(c, bucket, kmax, cp));
+        i = e;
     }
     cores.clear();
     return 0;
@@ -1007,7 +1019,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 Vsrc = Vk;
             }
             ct.RU = RU; ct.ldru = K;
-            ct.SU = SU; ct.RUc = nullptr; ct.work = work;
+            ct.SU = SU; ct.work = work;
             (cq ? cores : coresS).push_back(ct);
             if (cq) {
                 // new U = Q_U U_r = X2 (R3^-1 U_r)
@@ -1954,7 +1966,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
                 cqw.push_back(CQTask{W, nullptr, nullptr, RW, nullptr, nb, s, 0, nb, nb});
                 CoreTask ct{};
                 ct.RU = nullptr; ct.RV = RW; ct.ldru = s; ct.ldrv = s;
-                ct.SU = SU; ct.RUc = nullptr; ct.work = nullptr;
+                ct.SU = SU; ct.work = nullptr;
                 ct.rank_out = t.rank_dst; ct.rank_task = rt; ct.K = s;
                 cores.push_back(ct);
                 GemmTask gU = make_gemm(0, 0, nb, std::min(s, maxrank), s, 1.0, Q, nb, SU, s, 0.0, t.outU, nb);
@@ -1983,7 +1995,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
             qw.push_back(QRTask{W, tauW, TW, nb, s, nb});
             CoreTask ct{};
             ct.RU = nullptr; ct.RV = W; ct.ldru = nb; ct.ldrv = nb;
-            ct.SU = SU; ct.RUc = nullptr; ct.work = work;
+            ct.SU = SU; ct.work = work;
             ct.rank_out = t.rank_dst; ct.rank_task = rt; ct.K = s;
             cores.push_back(ct);
             au.push_back(QApplyTask{Y, TY, SU, t.outU, rt, nb, s, nb, s, nb, maxrank});

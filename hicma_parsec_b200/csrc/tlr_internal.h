@@ -250,14 +250,12 @@ void launch_rcholqr_batched(const CQTask *d_tasks, int ntasks, int kmax, bool fo
 
 // ------------------------------------------------------------- core SVD -----
 // M = RU RV^T (RU, RV: K x K upper from the QRs; RU == nullptr means I),
-// one-sided Jacobi SVD, truncation and outputs SU = U_r, SV = V_r Sigma_r
-// (K x r each, ld K).  mode 0: absolute sigma >= tol (recompression);
+// one-sided Jacobi SVD, truncation and output SU = U_r (K x r, ld K).  mode 0: absolute sigma >= tol (recompression);
 // mode 1: relative Frobenius tol (generation, with reject rules).
 struct CoreTask {
     const double *RU;    // K x K upper (ld ldru), nullptr = identity
     const double *RV;    // K x K upper (ld ldrv)
-    double *SU;          // out: K x K, left singular vectors sorted by decreasing sigma
-    double *RUc;         // out (if RU): clean copy of RU, K x K, zeros below the diagonal
+    double *SU;          // out: left singular vectors sorted by decreasing sigma, rank columns (ld K)
     double *work;        // core_work_doubles(K) doubles when K > core_smem_kmax()
     int *rank_out;       // rank map entry (may be null)
     int *rank_task;      // per-task rank for the apply steps
@@ -275,7 +273,9 @@ struct CoreParams {
 int core_smem_kmax();
 // Global scratch (doubles) of one core with K > core_smem_kmax().
 size_t core_work_doubles(int K);
-// All tasks of one launch should have K <= kmax; shared memory is sized from kmax.
+// Launch bucket of a core (the widest K of its kernel instance or cluster size).
+int core_bucket(int K);
+// All tasks of one launch have K <= kmax; kernel and shared memory are chosen from kmax.
 void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p,
                              cudaStream_t st);
 
