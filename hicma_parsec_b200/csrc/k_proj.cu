@@ -27,62 +27,65 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-// Pr = C^T W (rc x ra, ld rc)
-__device__ void proj_gram(const double *__restrict__ C, const double *W, double *Pr, int nb, int rc, int ra,
-                          double *red) {
+// Block (bi, bj) of Pr = C^T W (rc x ra, ld ldp)
+__device__ void proj_block(const double *__restrict__ C, const double *W, double *Pr, int ldp, int nb, int rc, int ra,
+                           int bi, int bj, double *red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tig = lane & 3;
     int chunk = (nb + PW - 1) / PW;
     chunk = (chunk + 3) & ~3;
     const int r0 = warp * chunk, r1 = min(nb, r0 + chunk);
-    for (int bi = 0; bi < rc; bi += PB) {
-        for (int bj = 0; bj < ra; bj += PB) {
-            double acc[4][4][2];
+    double acc[4][4][2];
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-            // column offsets of this lane's C and W columns (-1: outside)
-            int co[4], wo[4];
+        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    // column offsets of this lane's C and W columns (-1: outside)
+    int co[4], wo[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int ci = bi + 8 * q + g, cj = bj + 8 * q + g;
-                co[q] = ci < rc ? ci * nb : -1;
-                wo[q] = cj < ra ? cj * nb : -1;
-            }
-#pragma unroll 2
-            for (int k = r0; k < r1; k += 4) {
-                const int row = k + tig;
-                const bool rv = row < r1;
-                double a[4], b[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    a[q] = (rv && co[q] >= 0) ? __ldg(C + co[q] + row) : 0.0;
-                    b[q] = (rv && wo[q] >= 0) ? W[wo[q] + row] : 0.0;
-                }
-#pragma unroll
-                for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
-            }
-            double *my = red + warp * PB * PB;
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) my[(8 * mi + g) * PB + 8 * ni + 2 * tig + e] = acc[mi][ni][e];
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < PB * PB; idx += PT) {
-                const int i = idx / PB, j = idx % PB;
-                double s = 0.0;
-#pragma unroll
-                for (int w = 0; w < PW; ++w) s += red[w * PB * PB + idx];
-                if (bi + i < rc && bj + j < ra) Pr[(size_t)(bi + i) + (size_t)(bj + j) * rc] = s;
-            }
-            __syncthreads();
-        }
+    for (int q = 0; q < 4; ++q) {
+        const int ci = bi + 8 * q + g, cj = bj + 8 * q + g;
+        co[q] = ci < rc ? ci * nb : -1;
+        wo[q] = cj < ra ? cj * nb : -1;
     }
+#pragma unroll 2
+    for (int k = r0; k < r1; k += 4) {
+        const int row = k + tig;
+        const bool rv = row < r1;
+        double a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            a[q] = (rv && co[q] >= 0) ? __ldg(C + co[q] + row) : 0.0;
+            b[q] = (rv && wo[q] >= 0) ? W[wo[q] + row] : 0.0;
+        }
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
+    }
+    double *my = red + warp * PB * PB;
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) my[(8 * mi + g) * PB + 8 * ni + 2 * tig + e] = acc[mi][ni][e];
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < PB * PB; idx += PT) {
+        const int i = idx % PB, j = idx / PB;   // down the columns of Pr
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < PW; ++w) s += red[w * PB * PB + i * PB + j];
+        if (bi + i < rc && bj + j < ra) Pr[(size_t)(bi + i) + (size_t)(bj + j) * ldp] = s;
+    }
+    __syncthreads();
+}
+
+// Pr = C^T W (rc x ra, ld rc)
+__device__ void proj_gram(const double *__restrict__ C, const double *W, double *Pr, int nb, int rc, int ra,
+                          double *red) {
+    for (int bi = 0; bi < rc; bi += PB)
+        for (int bj = 0; bj < ra; bj += PB) proj_block(C, W, Pr, rc, nb, rc, ra, bi, bj, red);
 }
 
 // W -= C Pr
@@ -140,13 +143,28 @@ __global__ void __launch_bounds__(PT, 2) k_bcgs2(const ProjTask *__restrict__ ta
     for (int idx = threadIdx.x; idx < t.rc * t.ra; idx += PT) t.P[idx] += t.P2[idx];
 }
 
-// P = C^T W for a batch (the inner product B_V^T A_V of a recompression):
-// the split-K DMMA reduction of the projection, one CTA per product.
+// P = C^T W for a batch (the inner product B_V^T A_V of a recompression, the
+// projections of the blocked QR): the split-K DMMA reduction of the projection,
+// one CTA per 32 x 32 block of a product (grid.x covers the largest product), so
+// that a few wide products still fill the device; each block reads its 64
+// columns once, from L2 after the first reader.
 __global__ void __launch_bounds__(PT, 2) k_gram_batched(const GramTask *__restrict__ tasks) {
     extern __shared__ double red[];
-    const GramTask t = tasks[blockIdx.x];
-    if (t.rc <= 0 || t.ra <= 0) return;
-    proj_gram(t.C, t.W, t.P, t.nb, t.rc, t.ra, red);
+    const GramTask t = tasks[blockIdx.y];
+    const int nbi = (t.rc + PB - 1) / PB, nbj = (t.ra + PB - 1) / PB;
+    if ((int)blockIdx.x >= nbi * nbj) return;
+    proj_block(t.C, t.W, t.P, t.ldp ? t.ldp : t.rc, t.nb, t.rc, t.ra, (int)(blockIdx.x % nbi) * PB,
+               (int)(blockIdx.x / nbi) * PB, red);
+}
+
+// R (K x K, ld K) <- the k0 x k0 identity in its top-left corner, zero elsewhere.
+__global__ void k_rinit(const RInitTask *__restrict__ tasks) {
+    const RInitTask t = tasks[blockIdx.y];
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < (long long)t.K * t.K;
+         idx += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(idx % t.K), j = (int)(idx / t.K);
+        t.R[idx] = i == j && i < t.k0 ? 1.0 : 0.0;
+    }
 }
 
 // Orthogonality check of formed Q factors (the generation range finder):
@@ -178,12 +196,19 @@ void launch_orth_check(const GramTask *d_tasks, int ntasks, double thr, int *fai
     k_orth_check<<<(ntasks + 7) / 8, 256, 0, st>>>(d_tasks, ntasks, thr, fail);
 }
 
-void launch_gram_batched(const GramTask *d_tasks, int ntasks, cudaStream_t st) {
+int gram_blocks(int rc, int ra) { return ((rc + PB - 1) / PB) * ((ra + PB - 1) / PB); }
+
+void launch_rinit(const RInitTask *d_tasks, int ntasks, int kmax, cudaStream_t st) {
     if (ntasks <= 0) return;
+    k_rinit<<<dim3((unsigned)((kmax * (long long)kmax + 1023) / 1024), (unsigned)ntasks), 256, 0, st>>>(d_tasks);
+}
+
+void launch_gram_batched(const GramTask *d_tasks, int ntasks, int max_blocks, cudaStream_t st) {
+    if (ntasks <= 0 || max_blocks <= 0) return;
     const int smem = PW * PB * PB * (int)sizeof(double);
     // per device and thread-safe: set on every launch (a host-side call, no synchronisation)
     cudaFuncSetAttribute(k_gram_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_gram_batched<<<ntasks, PT, smem, st>>>(d_tasks);
+    k_gram_batched<<<dim3((unsigned)max_blocks, (unsigned)ntasks), PT, smem, st>>>(d_tasks);
 }
 
 void launch_bcgs2(const ProjTask *d_tasks, int ntasks, cudaStream_t st) {

@@ -563,8 +563,15 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
     }
     double acc[NACC][2];
 
+    if (QF && t.plain) {
+        // X is nearly orthonormal already: R = I, one pass below without the substitution
+        for (int idx = tid; idx < KM * KM; idx += CQ_THREADS) {
+            const int j = idx / KM, k = idx % KM;
+            Rt[j * L + k] = j == k && j < K ? 1.0 : 0.0;
+        }
+        __syncthreads();
+    } else {
     // 1. the sketch: this thread's bucket is tid
-    {
         double s[KM];
 #pragma unroll
         for (int j = 0; j < KM; ++j) s[j] = 0.0;
@@ -638,7 +645,8 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
     }
 
     // 3. Y = X R^-1 and its Gram product; R <- chol(Y^T Y) R
-    const bool keep_y = QF || t.Rinv;
+    const bool plain = QF && t.plain;
+    const bool keep_y = (QF || t.Rinv) && !plain;
     for (int pass = 0;; ++pass) {
 #pragma unroll
         for (int q = 0; q < NACC; ++q) acc[q][0] = acc[q][1] = 0.0;
@@ -660,7 +668,7 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
             if (PREFETCH && r0 + CQ_THREADS < nb) load_row<KM>(t, row + CQ_THREADS, nb, k1, K, v);
             __syncwarp();
             // rd and R are zero past K, so the padding columns stay zero
-            warp_trsm<KM, P>(zb, Rt, rdt, K, lane);
+            if (!plain) warp_trsm<KM, P>(zb, Rt, rdt, K, lane);
             if (valid && keep_y) {
                 double *pz = t.Z + row;
                 for (int j = 0; j < K; ++j, pz += nb) *pz = zb[j * P + lane];
@@ -693,16 +701,17 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
         double gmax = 0.0;
 #pragma unroll
         for (int w = 0; w < CQ_WARPS; ++w) gmax = fmax(gmax, gmax_sh[w]);
-        const bool again = !(gmax <= CQ_GMAX) && pass + 1 < CQ_APPLY;
+        const bool again = !plain && !(gmax <= CQ_GMAX) && pass + 1 < CQ_APPLY;
         accumulate<KM>(Rr, Rt, G, rdt, K, tid);
         if (!again) break;
         if (tid == 0 && flags) atomicAdd(flags + 1, 1);
     }
 
     // outputs: R (column-major); Rc^-1 for a deferred Q; or Q = Y Rc^-1
+    const int ldr = t.ldr ? t.ldr : K;
     for (int idx = tid; idx < K * K; idx += CQ_THREADS) {
         const int i = idx % K, j = idx / K;
-        t.R[i + (size_t)j * K] = Rt[i * L + j];
+        t.R[i + (size_t)j * ldr] = Rt[i * L + j];
     }
     if (!QF && t.Rinv) {
         tri_inverse<KM>(Rr, rdg, G, Wsc, K, tid);

@@ -534,7 +534,7 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
         if (t.k1) BC(t.X1, bc_span(t.nb, t.k1, t.ld1), "cholqr X1", i);
         if (t.k2) BC(t.X2, bc_span(t.nb, t.k2, t.ld2), "cholqr X2", i);
         if (t.Q || t.Rinv) BC(t.Z, bc_span(t.nb, K, t.nb), "cholqr Y", i);
-        BC(t.R, bc_span(K, K, K), "cholqr R", i);
+        BC(t.R, bc_span(K, K, t.ldr ? t.ldr : K), "cholqr R", i);
         if (t.Q) BC(t.Q, bc_span(t.nb, K, t.nb), "cholqr Q", i);
         if (t.Rinv) BC(t.Rinv, bc_span(K, K, K), "cholqr R3 inverse", i);
     }
@@ -566,9 +566,9 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
             // pass over the rows (substitution and Gram product), and the Q substitution when Q
             // is formed
             const double K = t.k1 + t.k2, m = 256.0;
-            fl += 2.0 * t.nb * K + 5.0 * m * K * K + (t.Q ? 3.0 : 2.0) * t.nb * K * K;
+            fl += t.plain ? 2.0 * t.nb * K * K : 2.0 * t.nb * K + 5.0 * m * K * K + (t.Q ? 3.0 : 2.0) * t.nb * K * K;
             // X read twice; Y written when kept; Y read and Q written when Q is formed
-            by += 8.0 * t.nb * K * (2.0 + (t.Q || t.Rinv ? 1.0 : 0.0) + (t.Q ? 2.0 : 0.0));
+            by += 8.0 * t.nb * K * (t.plain ? 3.0 : 2.0 + (t.Q || t.Rinv ? 1.0 : 0.0) + (t.Q ? 2.0 : 0.0));
         }
         {
             Prof pf(c, P_CHOLQR, fl, by);
@@ -706,7 +706,7 @@ int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
         const GramTask &t = v[i];
         BC(t.C, bc_span(t.nb, t.rc, t.nb), "gram C", i);
         BC(t.W, bc_span(t.nb, t.ra, t.nb), "gram W", i);
-        BC(t.P, bc_span(t.rc, t.ra, t.rc), "gram P", i);
+        BC(t.P, bc_span(t.rc, t.ra, t.ldp ? t.ldp : t.rc), "gram P", i);
     }
 #endif
     double fl = 0.0, by = 0.0;
@@ -714,14 +714,117 @@ int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
         fl += 2.0 * g.nb * (double)g.rc * g.ra;
         by += 8.0 * g.nb * (double)(g.rc + g.ra);
     }
-    GramTask *d = stage(c, v.data(), v.size());
-    if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-    {
-        Prof pf(c, cls, fl, by);
-        launch_gram_batched(d, (int)v.size(), c->cur);
+    for (size_t i = 0; i < v.size(); i += GRAM_MAX_TASKS) {
+        const size_t n = std::min<size_t>(v.size() - i, GRAM_MAX_TASKS);
+        int blocks = 0;
+        for (size_t q = i; q < i + n; ++q) blocks = std::max(blocks, gram_blocks(v[q].rc, v[q].ra));
+        GramTask *d = stage(c, v.data() + i, n);
+        if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
+        {
+            Prof pf(c, cls, i ? 0.0 : fl, i ? 0.0 : by);
+            launch_gram_batched(d, (int)n, blocks, c->cur);
+        }
+        TRY(check_launch(c));
     }
     v.clear();
-    return check_launch(c);
+    return 0;
+}
+
+// QR of stacks wider than rcholqr_kmax() by block Gram-Schmidt with
+// reorthogonalisation (Barlow and Smoktunowicz, "Reorthogonalized block
+// classical Gram-Schmidt", Numer. Math. 2013).  Q (nb x K, ld nb) holds an
+// orthonormal basis in its first k0 columns and the columns to factor after
+// them; it becomes the orthonormal Q, and R (K x K, ld K) the factor of
+// [basis, columns].  A block of up to BQ_W columns is projected on the columns
+// before it, factored by the randomized CholeskyQR (whatever its condition),
+// projected again and factored by one plain CholeskyQR pass, which it is now
+// well enough conditioned for; R takes both rounds.  The products are batched
+// DMMA launches over all tasks, so a few wide stacks still fill the device (one
+// CTA per stack and SIMT reflectors before: 3 stacks of nb 1350 and K about 650
+// took 28 ms for the QRs and 18 ms for the Q application).
+// Scratch per task: Z nb x BQ_W, S2 K x BQ_W, R1 and R2 BQ_W x BQ_W.
+constexpr int BQ_W = 64;
+struct BQTask {
+    double *Q;
+    int nb, k0, K;
+    double *R;
+    double *Z, *S2, *R1, *R2;
+};
+
+size_t bq_ws_bytes(int nb, int K) {
+    return align_up(sizeof(double) * (size_t)nb * BQ_W + 1) + align_up(sizeof(double) * (size_t)K * BQ_W + 1) +
+           2 * align_up(sizeof(double) * BQ_W * BQ_W + 1);
+}
+
+// Allocates a task's scratch in the arena (false: exhausted).
+bool bq_make(hicma_tlr_ctx *c, BQTask &t, double *Q, int nb, int k0, int K, double *R) {
+    t.Q = Q; t.nb = nb; t.k0 = k0; t.K = K; t.R = R;
+    t.Z = ws_alloc<double>(c, (size_t)nb * BQ_W);
+    t.S2 = ws_alloc<double>(c, (size_t)K * BQ_W);
+    t.R1 = ws_alloc<double>(c, (size_t)BQ_W * BQ_W);
+    t.R2 = ws_alloc<double>(c, (size_t)BQ_W * BQ_W);
+    return t.Z && t.S2 && t.R1 && t.R2;
+}
+
+// Block width of n columns: equal blocks, a multiple of 8 wide.
+int bq_width(int n) {
+    const int nblk = (n + BQ_W - 1) / BQ_W;
+    return nblk ? ((n + nblk - 1) / nblk + 7) / 8 * 8 : BQ_W;
+}
+
+int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
+    if (v.empty()) return 0;
+    for (size_t i = 0; i < v.size(); i += GRAM_MAX_TASKS) {
+        std::vector<RInitTask> ri;
+        int kmax = 1;
+        for (size_t q = i; q < std::min(v.size(), i + GRAM_MAX_TASKS); ++q) {
+            ri.push_back(RInitTask{v[q].R, v[q].K, v[q].k0});
+            kmax = std::max(kmax, v[q].K);
+#ifdef TLR_BOUNDS_CHECK
+            BC(v[q].R, bc_span(v[q].K, v[q].K, v[q].K), "block QR R", q);
+#endif
+        }
+        RInitTask *d = stage(c, ri.data(), ri.size());
+        if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
+        launch_rinit(d, (int)ri.size(), kmax, c->cur);
+        TRY(check_launch(c));
+    }
+    for (int b = 0;; ++b) {
+        std::vector<GramTask> g1, g2;
+        std::vector<GemmTask> u1, u2, r2;
+        std::vector<CQTask> q1, q2;
+        for (const BQTask &t : v) {
+            const int bw = bq_width(t.K - t.k0), j = t.k0 + b * bw;
+            if (j >= t.K) continue;
+            const int w = std::min(bw, t.K - j), nb = t.nb, K = t.K;
+            double *W = t.Q + (size_t)nb * j, *Rj = t.R + (size_t)j * K;
+            CQTask f{W, nullptr, t.Z, j ? t.R1 : Rj, W, nb, w, 0, nb, nb};
+            f.ldr = j ? w : K;
+            q1.push_back(f);
+            if (!j) continue;
+            g1.push_back(GramTask{t.Q, W, Rj, nb, j, w, K});
+            u1.push_back(make_gemm(0, 0, nb, w, j, -1.0, t.Q, nb, Rj, K, 1.0, W, nb));
+            g2.push_back(GramTask{t.Q, W, t.S2, nb, j, w, j});
+            u2.push_back(make_gemm(0, 0, nb, w, j, -1.0, t.Q, nb, t.S2, j, 1.0, W, nb));
+            CQTask p{W, nullptr, W, t.R2, W, nb, w, 0, nb, nb};
+            p.ldr = w;
+            p.plain = 1;
+            q2.push_back(p);
+            // X_J = Q (S + S2 R1) + Q_J (R2 R1)
+            r2.push_back(make_gemm(0, 0, j, w, w, 1.0, t.S2, j, t.R1, w, 1.0, Rj, K));
+            r2.push_back(make_gemm(0, 0, w, w, w, 1.0, t.R2, w, t.R1, w, 0.0, Rj + j, K));
+        }
+        if (q1.empty()) break;
+        TRY(run_grams(c, g1, P_PROJ));
+        TRY(run_gemms(c, u1, false, P_PROJ));
+        TRY(run_rcholqr(c, q1, 0));
+        TRY(run_grams(c, g2, P_PROJ));
+        TRY(run_gemms(c, u2, false, P_PROJ));
+        TRY(run_rcholqr(c, q2, 0));
+        TRY(run_gemms(c, r2, false, P_PROJ));
+    }
+    v.clear();
+    return 0;
 }
 
 int run_copies(hicma_tlr_ctx *c, std::vector<CopyTask> &v) {
@@ -841,17 +944,21 @@ struct RecompTask {
 };
 
 // Workspace of one low-rank update (K = rc + ra).
-size_t recomp_ws_bytes(int nb, const RecompTask &t) {
+size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
     const int K = t.rc + t.ra, rc = t.rc, ra = t.ra;
-    const int pb = qr_panel_width(nb);
-    const size_t npk = (size_t)(K + pb - 1) / pb + 1, npa = (size_t)(ra + pb - 1) / pb + 1;
     auto A = [](size_t n) { return align_up(sizeof(double) * n + 1); };
     size_t b = 0;
-    b += A((size_t)nb * K) * 3;                          // Us = [Cu | Wu], Vs = [Cv | -Y], Vk
-    b += A(ra) + A(K) + A(npa * pb * pb) + A(npk * pb * pb);  // tau, T factors of Wu and Vs
-    b += A((size_t)rc * ra) * 2;                         // Pu, Pu2
-    b += A((size_t)nb * ra) + A((size_t)ra * ra);        // Q and R of the residual (CholeskyQR form)
-    b += A((size_t)K * K) * 6;                           // RU, SU, T1, RV, R3^-1 and R3^-1 U_r
+    b += A((size_t)nb * K) * 2;                          // Us (U side's Q), Vs = [Cv | -Y]
+    b += A((size_t)K * K) * 6;                           // RU, SU, T1, RV, Rc^-1 and Rc^-1 U_r
+    if (!c->cholqr) {                                    // Householder QRs
+        const int pb = qr_panel_width(nb);
+        const size_t npk = (size_t)(K + pb - 1) / pb + 1, npa = (size_t)(ra + pb - 1) / pb + 1;
+        b += A((size_t)nb * K);                          // Vk
+        b += A(ra) + A(K) + A(npa * pb * pb) + A(npk * pb * pb);  // tau, T factors of Wu and Vs
+        b += A((size_t)rc * ra) * 2;                     // Pu, Pu2
+    } else if (K > rcholqr_kmax()) {
+        b += A((size_t)nb * K) + 2 * bq_ws_bytes(nb, K); // Vk, block QRs
+    }
     if (K > core_smem_kmax()) b += A(core_work_doubles(K));
     if (t.Bv) b += A((size_t)t.rb * t.ra);
     return b + 1024;
@@ -887,15 +994,14 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
 }
 
 // Recompression of a batch of low-rank updates C = [Cu Au][Cv -Y]^T.
-// The old U is orthonormal, so on that side only the new columns need an
-// orthogonal factorisation: Au is projected twice against Cu (block classical
-// Gram-Schmidt, DMMA GEMMs) and the residual Wu (nb x ra) gets a Householder
-// QR, giving R_U = [[I, Pu], [0, R(Wu)]].  The old V = V Sigma is orthogonal
-// only up to the core solver's tolerance relative to its largest singular
-// value, which is not enough to project its weak columns, so [Cv, -Y] gets a
-// full Householder QR for R_V.  The core M = R_U R_V^T is decomposed and
-// truncated (core kernel), then new U = Cu U_top + Q(Wu) [U_bot; 0] and
-// new V = [Cv, -Y] (R_U^T U_r).
+// Both stacks get a QR: up to rcholqr_kmax() columns by the randomized
+// CholeskyQR in one CTA, wider ones by block Gram-Schmidt (run_block_qr).  There
+// the old U is orthonormal, so on that side only the new columns are factored,
+// R_U = [[I, P], [0, R]]; the old V = V Sigma is orthogonal only up to the core
+// solver's tolerance relative to its largest singular value, which is not enough
+// for its weak columns, so [Cv, -Y] is factored whole.  The core M = R_U R_V^T
+// is decomposed and truncated (core kernel), then new U = Q_U U_r and new
+// V = [Cv, -Y] (R_U^T U_r).
 // thr2 > 0 enables the precision policy: the products forming Y run in FP32
 // for updates whose factor tiles satisfy ||A||_F^2 ||B||_F^2 <= thr2.
 int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, double acc, int maxrank,
@@ -909,8 +1015,8 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         // CholeskyQR chain (F) there and the Householder chain of the wide
         // updates (S) on the side stream, joined at the end of the chunk
         std::vector<CopyTask> copies, copiesS, keeps;
-        std::vector<GemmTask> g1, g2, g1s, g2s, gTU, gU, g3, g4, gQS, gUS, g3S, g4S;
-        std::vector<CQTask> cqS;   // QRs of the wide updates' projected residuals (Q formed)
+        std::vector<GemmTask> g1, g2, g1s, g2s, gTU, gU, g3, g4, gUS, g3S, g4S;
+        std::vector<BQTask> bqs;   // block QRs of the wide updates
         std::vector<CoreTask> coresS;
         std::vector<ProjTask> projs;
         std::vector<SelTask> sels;
@@ -925,7 +1031,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         int *rank_task = d_rank_task_base;
         for (; i < tasks.size(); ++i) {
             const RecompTask &t = tasks[i];
-            if (recomp_ws_bytes(nb, t) > ws_free(c)) {
+            if (recomp_ws_bytes(c, nb, t) > ws_free(c)) {
                 if (i == i0) { set_err("workspace too small for one recompression (K=%d)", t.rc + t.ra); return HICMA_TLR_ERR_OOM; }
                 break;
             }
@@ -937,9 +1043,11 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             if (K == 0) { cores.push_back(ct); continue; }
             // Stacks up to rcholqr_kmax() columns: both QRs by randomized
             // CholeskyQR (U side [Cu, Au] read in place, Q_U = Y Rc^-1 kept
-            // factored; V side R only); wider stacks: block Gram-Schmidt +
-            // Householder on the U side and a Householder QR on the V side.
+            // factored; V side R only); wider stacks: block Gram-Schmidt QRs, on the
+            // U side starting from the orthonormal Cu.  With HICMA_TLR_QR=householder:
+            // Au projected on Cu + Householder on the U side, Householder on the V side.
             const bool cq = c->cholqr && K <= rcholqr_kmax();
+            const bool bq = c->cholqr && !cq;
             double *Vs = ws_alloc<double>(c, (size_t)nb * K);
             double *Us = ws_alloc<double>(c, (size_t)nb * K);    // CholeskyQR path: Y of the U side
             double *RU = ws_alloc<double>(c, (size_t)K * K);
@@ -979,6 +1087,21 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 vrs.push_back(u);
                 vrs.push_back(CQTask{Vs, nullptr, nullptr, RV, nullptr, nb, K, 0, nb, nb});
                 ct.RV = RV; ct.ldrv = K;
+            } else if (bq) {
+                // Us = [Cu | Au] becomes Q_U in place; the V side's Q is formed in a copy
+                double *Vk = ws_alloc<double>(c, (size_t)nb * K);
+                double *RV = ws_alloc<double>(c, (size_t)K * K);
+                if (rc > 0) copiesS.push_back(make_copy(t.Cu, nb, Us, nb, nb, rc));
+                if (ra > 0) copiesS.push_back(make_copy(t.Au, nb, Us + (size_t)nb * rc, nb, nb, ra));
+                keeps.push_back(make_copy(Vs, nb, Vk, nb, nb, K));
+                BQTask bu, bv;
+                if (!bq_make(c, bu, Us, nb, rc, K, RU) || !bq_make(c, bv, Vk, nb, 0, K, RV)) {
+                    set_err("workspace too small (block QR)");
+                    return HICMA_TLR_ERR_OOM;
+                }
+                bqs.push_back(bu);
+                bqs.push_back(bv);
+                ct.RV = RV; ct.ldrv = K;
             } else {
                 double *Vk = ws_alloc<double>(c, (size_t)nb * K);
                 const int pbw = qr_panel_width(nb);
@@ -987,34 +1110,17 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 double *TU = ws_alloc<double>(c, npa * pbw * pbw), *TV = ws_alloc<double>(c, npk * pbw * pbw);
                 double *Pu = ws_alloc<double>(c, (size_t)rc * ra), *Pu2 = ws_alloc<double>(c, (size_t)rc * ra);
                 double *Wu = Us + (size_t)nb * rc;
-                // R of the projected residual Wu, as the assembly reads it (top ra x ra, ld)
-                const double *Rw = Wu;
-                int ldrw = nb;
                 if (rc > 0) copiesS.push_back(make_copy(t.Cu, nb, Us, nb, nb, rc));
                 if (ra > 0) {
                     copiesS.push_back(make_copy(t.Au, nb, Wu, nb, nb, ra));
                     // two rounds of projection of Au against the old orthonormal U
                     if (rc > 0) projs.push_back(ProjTask{Us, Wu, Pu, Pu2, nb, rc, ra});
-                    if (c->cholqr && ra <= rcholqr_kmax()) {
-                        // residual up to 64 columns: randomized CholeskyQR with Q formed,
-                        // and the new U's Q(Wu) U_bot as one GEMM
-                        double *Qw = ws_alloc<double>(c, (size_t)nb * ra);
-                        double *Rq = ws_alloc<double>(c, (size_t)ra * ra);
-                        cqS.push_back(CQTask{Wu, nullptr, Qw, Rq, Qw, nb, ra, 0, nb, nb});
-                        Rw = Rq;
-                        ldrw = ra;
-                        GemmTask q = make_gemm(0, 0, nb, std::min(K, maxrank), ra, 1.0, Qw, nb, SU + rc, K, 0.0,
-                                               t.outU, nb);
-                        q.n_dev = ct.rank_task;
-                        gQS.push_back(q);
-                    } else {
-                        qrs.push_back(QRTask{Wu, tauU, TU, nb, ra, nb});
-                        apps.push_back(QApplyTask{Wu, TU, SU + rc, t.outU, ct.rank_task, nb, ra, nb, K, nb, maxrank});
-                    }
+                    qrs.push_back(QRTask{Wu, tauU, TU, nb, ra, nb});
+                    apps.push_back(QApplyTask{Wu, TU, SU + rc, t.outU, ct.rank_task, nb, ra, nb, K, nb, maxrank});
                 }
                 keeps.push_back(make_copy(Vs, nb, Vk, nb, nb, K));
                 qrs.push_back(QRTask{Vs, tauV, TV, nb, K, nb});
-                asm_.push_back(AssembleTask{Pu, Rw, RU, rc, ra, ldrw});
+                asm_.push_back(AssembleTask{Pu, Wu, RU, rc, ra, nb});
                 ct.RV = Vs; ct.ldrv = nb;
                 Vsrc = Vk;
             }
@@ -1031,6 +1137,11 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 GemmTask u = make_gemm(0, 0, nb, rcap, K, 1.0, Us, nb, TU, K, 0.0, t.outU, nb);
                 u.n_dev = ct.rank_task;
                 gU.push_back(u);
+            } else if (bq) {
+                // new U = Q_U U_r
+                GemmTask u = make_gemm(0, 0, nb, std::min(K, maxrank), K, 1.0, Us, nb, SU, K, 0.0, t.outU, nb);
+                u.n_dev = ct.rank_task;
+                gUS.push_back(u);
             } else if (rc > 0) {
                 // new U = Q(Wu) [U_bot; 0] + Cu U_top (beta 1 after the Q application when ra > 0)
                 GemmTask u = make_gemm(0, 0, nb, std::min(K, maxrank), rc, 1.0, Us, nb, SU, K, ra > 0 ? 1.0 : 0.0, t.outU, nb);
@@ -1080,7 +1191,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             TRY(check_launch(c));
         }
         TRY(run_qr(c, qrs, nb));
-        TRY(run_rcholqr(c, cqS, 0));
+        TRY(run_block_qr(c, bqs));
         if (!asm_.empty()) {
             AssembleTask *d = stage(c, asm_.data(), asm_.size());
             if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
@@ -1090,7 +1201,6 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         CoreParams cp{0, acc, maxrank, fixed_rank, nb, c->d_flags + 1, c->d_flags + 2};
         TRY(run_core_buckets(c, coresS, cp));
         TRY(run_qapply(c, apps, nb));
-        TRY(run_gemms(c, gQS));   // Q(Wu) U_bot before gUS adds Cu U_top
         TRY(run_gemms(c, gUS));
         TRY(run_gemms(c, g3S));
         TRY(run_gemms(c, g4S));
@@ -1910,7 +2020,8 @@ static size_t compress_ws_bytes(int nb, int s) {
     b += align_up(sizeof(double) * (size_t)nb * s + 1) * 4;   // Y, Q, W, Wkeep
     b += align_up(sizeof(double) * (size_t)s + 1) * 2;
     b += align_up(sizeof(double) * npan * pb * pb + 1) * 2;
-    b += align_up(sizeof(double) * (size_t)s * s + 1) * 3;    // SU (+ R_Y, R_W of the CholeskyQR path)
+    b += align_up(sizeof(double) * (size_t)s * s + 1) * 4;    // SU (+ R_Y, R_W, Q^T Q of the CholeskyQR path)
+    if (s > rcholqr_kmax()) b += 2 * bq_ws_bytes(nb, s);      // block QRs
     if (s > core_smem_kmax()) b += align_up(sizeof(double) * core_work_doubles(s) + 1);
     return b + 1024;
 }
@@ -1942,9 +2053,10 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         std::vector<CQTask> cqy, cqw;
         std::vector<GemmTask> gu;
         std::vector<GramTask> gq;
-        // up to rcholqr_kmax() samples: both QRs by randomized CholeskyQR (Q of
-        // Y formed, R of W only), U = Q_Y U_r as a GEMM
-        const bool cq = c->cholqr && s <= rcholqr_kmax() && !force_hh;
+        // both QRs by randomized CholeskyQR (Q of Y formed, R of W only; above
+        // rcholqr_kmax() samples by block Gram-Schmidt), U = Q_Y U_r as a GEMM
+        const bool cq = c->cholqr && !force_hh;
+        std::vector<BQTask> bqy, bqw;
         size_t i = i0;
         for (; i < tasks.size(); ++i) {
             if (compress_ws_bytes(nb, s) > ws_free(c)) {
@@ -1952,6 +2064,37 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
                 break;
             }
             const CompressTask &t = tasks[i];
+            if (cq && s > rcholqr_kmax()) {
+                double *Y = ws_alloc<double>(c, (size_t)nb * s);      // becomes Q_Y
+                double *W = ws_alloc<double>(c, (size_t)nb * s), *Wk = ws_alloc<double>(c, (size_t)nb * s);
+                double *RY = ws_alloc<double>(c, (size_t)s * s), *RW = ws_alloc<double>(c, (size_t)s * s);
+                double *SU = ws_alloc<double>(c, (size_t)s * s);
+                BQTask by, bw;
+                if (!bq_make(c, by, Y, nb, 0, s, RY) || !bq_make(c, bw, Wk, nb, 0, s, RW)) {
+                    set_err("workspace too small (block QR)");
+                    return HICMA_TLR_ERR_OOM;
+                }
+                int *rt = d_rank_task_base + (i - i0);
+                gy.push_back(make_gemm(0, 0, nb, s, nb, 1.0, t.A, nb, Omega, nb, 0.0, Y, nb));
+                bqy.push_back(by);
+                if (d_fail) gq.push_back(GramTask{Y, Y, ws_alloc<double>(c, (size_t)s * s), nb, s, s});
+                gw.push_back(make_gemm(1, 0, nb, s, nb, 1.0, t.A, nb, Y, nb, 0.0, W, nb));
+                keeps.push_back(make_copy(W, nb, Wk, nb, nb, s));
+                bqw.push_back(bw);
+                CoreTask ct{};
+                ct.RU = nullptr; ct.RV = RW; ct.ldru = s; ct.ldrv = s;
+                ct.SU = SU;
+                ct.work = s > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(s)) : nullptr;
+                ct.rank_out = t.rank_dst; ct.rank_task = rt; ct.K = s;
+                cores.push_back(ct);
+                GemmTask gU = make_gemm(0, 0, nb, std::min(s, maxrank), s, 1.0, Y, nb, SU, s, 0.0, t.outU, nb);
+                gU.n_dev = rt;
+                gu.push_back(gU);
+                GemmTask g = make_gemm(0, 0, nb, std::min(s, maxrank), s, 1.0, W, nb, SU, s, 0.0, t.outV, nb);
+                g.n_dev = rt;
+                gv.push_back(g);
+                continue;
+            }
             if (cq) {
                 double *Y = ws_alloc<double>(c, (size_t)nb * s);
                 double *Q = ws_alloc<double>(c, (size_t)nb * s);
@@ -2007,15 +2150,13 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         TRY(run_gemms(c, gy, false, P_GEMM_GEN));
         TRY(run_qr(c, qy, nb));
         TRY(run_rcholqr(c, cqy, 0));
+        TRY(run_block_qr(c, bqy));
         if (!gq.empty()) {
             // Q^T Q of every formed Q, then the orthogonality flags of this sub-batch
+            std::vector<GramTask> gc = gq;
+            TRY(run_grams(c, gc, P_GRAM));
             GramTask *dq = stage(c, gq.data(), gq.size());
             if (!dq) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-            {
-                Prof pf(c, P_GRAM, 2.0 * nb * (double)s * s * gq.size(), 8.0 * nb * (double)s * gq.size());
-                launch_gram_batched(dq, (int)gq.size(), c->cur);
-            }
-            TRY(check_launch(c));
             launch_orth_check(dq, (int)gq.size(), GEN_ORTH_THR, d_fail + i0, c->cur);
             TRY(check_launch(c));
         }
@@ -2024,6 +2165,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         TRY(run_copies(c, keeps));
         TRY(run_qr(c, qw, nb));
         TRY(run_rcholqr(c, cqw, 0));
+        TRY(run_block_qr(c, bqw));
         CoreParams cp{1, tol, maxrank, 0, nb, nullptr, nullptr};
         TRY(run_core_buckets(c, cores, cp));
         TRY(run_qapply(c, au, nb));
@@ -2060,7 +2202,7 @@ int hicma_tlr_generate(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, int *Ar, c
     // The reference samples min(maxrank + 10, NB) columns for every tile
     // (STARSH_gen.jdf:262-266); the sampled singular values only matter up to
     // the rank, so tiles start with s = min(64, s_full) samples (the CholeskyQR
-    // path; 160 with the Householder path) and a tile whose rank comes within
+    // path; 160 with HICMA_TLR_QR=householder) and a tile whose rank comes within
     // max(32, s/4) of s is generated again with twice the samples, up to
     // s_full.  Rejected tiles (2r >= NB) stay rejected: more samples can only
     // raise the rank.
@@ -2081,7 +2223,7 @@ int hicma_tlr_generate(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, int *Ar, c
     bool force_hh = false;
     while (!pending.empty()) {
         const size_t mark_round = c->ar->off;
-        const bool cq_round = c->cholqr && s <= rcholqr_kmax() && !force_hh;
+        const bool cq_round = c->cholqr && !force_hh;
         int *dfail = cq_round ? ws_alloc<int>(c, pending.size()) : nullptr;
         if (cq_round && !dfail) { set_err("workspace too small"); return HICMA_TLR_ERR_OOM; }
         launch_set_identity(Ident, s, s, c->stream);

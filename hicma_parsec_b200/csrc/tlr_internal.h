@@ -146,14 +146,25 @@ struct ProjTask {
     int nb, rc, ra;
 };
 void launch_bcgs2(const ProjTask *d_tasks, int ntasks, cudaStream_t st);
-// P = C^T W (rc x ra, ld rc) with C nb x rc and W nb x ra (ld nb): one CTA per
-// product, split-K over its warps, fixed-order reduction.
+// P = C^T W (rc x ra, ld ldp; 0 means rc) with C nb x rc and W nb x ra (ld nb):
+// one CTA per 32 x 32 block, split-K over its warps, fixed-order reduction.
+// max_blocks: the largest gram_blocks() of the tasks; ntasks <= GRAM_MAX_TASKS.
 struct GramTask {
     const double *C, *W;
     double *P;
     int nb, rc, ra;
+    int ldp = 0;
 };
-void launch_gram_batched(const GramTask *d_tasks, int ntasks, cudaStream_t st);
+int gram_blocks(int rc, int ra);
+constexpr int GRAM_MAX_TASKS = 32768;     // grid.y
+void launch_gram_batched(const GramTask *d_tasks, int ntasks, int max_blocks, cudaStream_t st);
+// R (K x K, ld K) <- k0 x k0 identity in the top-left corner, zero elsewhere;
+// kmax: the largest K; ntasks <= GRAM_MAX_TASKS.
+struct RInitTask {
+    double *R;
+    int K, k0;
+};
+void launch_rinit(const RInitTask *d_tasks, int ntasks, int kmax, cudaStream_t st);
 // fail[i] = 1 when the P of task i (a Q^T Q, rc == ra) is not the identity to
 // within thr between nonzero columns, else 0 (one warp per task).
 void launch_orth_check(const GramTask *d_tasks, int ntasks, double thr, int *fail, cudaStream_t st);
@@ -241,6 +252,9 @@ struct CQTask {
     double *Q;
     int nb, k1, k2, ld1, ld2;
     double *Rinv = nullptr;
+    int ldr = 0;        // leading dimension of R (0: K)
+    int plain = 0;      // one CholeskyQR pass without the sketch, for an X that is nearly
+                        // orthonormal already: Q = X chol(X^T X)^-1 (Z = X1, k2 = 0; Q may be X)
 };
 int rcholqr_kmax();
 int rcholqr_bucket(int K);   // width of the kernel instance that takes K
