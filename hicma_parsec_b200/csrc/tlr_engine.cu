@@ -3208,57 +3208,87 @@ int hicma_tlr_logdet(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *logdet) {
 }
 
 // Forward (L z = b) then backward (L^T x = z) substitution over tiles with
-// the stored L_kk^-1; off-diagonal updates of one step are batched.
-static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, int nrhs) {
-    const int NT = A->NT, NB = A->NB;
-    const size_t N = A->N;
-    double *tmp = ws_alloc<double>(c, (size_t)NB * nrhs);
-    double *T2 = ws_alloc<double>(c, (size_t)NT * A->maxrank * nrhs + 1);
-    if (!tmp || !T2) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
-    std::vector<GemmTask> g1, g2;
-    std::vector<CopyTask> cp;
-    for (int k = 0; k < NT; ++k) {
-        double *xk = X + (size_t)k * NB;
-        g1.push_back(make_gemm(0, 0, NB, nrhs, NB, 1.0, A->linv(k), NB, xk, (int)N, 0.0, tmp, NB));
-        g1.back().tri = 1;   // L^-1 lower triangular
-        TRY(run_gemms(c, g1));
-        cp.push_back(make_copy(tmp, NB, xk, (int)N, NB, nrhs));
-        TRY(run_copies(c, cp));
-        for (int m = k + 1; m < NT; ++m) {
-            double *xm = X + (size_t)m * NB;
-            if (A->is_dense(m, k)) {
-                g2.push_back(make_gemm(0, 0, NB, nrhs, NB, -1.0, A->dense(m, k), NB, xk, (int)N, 1.0, xm, (int)N));
-            } else {
-                const int r = A->rank(m, k);
-                if (r == 0) continue;
-                double *t = T2 + (size_t)m * A->maxrank * nrhs;
-                g1.push_back(make_gemm(1, 0, r, nrhs, NB, 1.0, A->V(m, k), NB, xk, (int)N, 0.0, t, r));
-                g2.push_back(make_gemm(0, 0, NB, nrhs, r, -1.0, A->U(m, k), NB, t, r, 1.0, xm, (int)N));
-            }
+// the stored L_kk^-1, on n columns (X: N x n, ld N, in and out; Z: the same, scratch;
+// T: NT x maxrank x n scratch).  Three launches a step: the diagonal solve (into
+// the other of X and Z, so nothing is copied), the products V^T z of the column's
+// low-rank tiles with the dense tiles' updates, and the low-rank updates.  The
+// tasks of all steps are staged at once: their sizes are known on the host.
+static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, double *T, int n) {
+    const int NT = A->NT, NB = A->NB, N = A->N;
+    struct Step { size_t first; int cnt, mmax, kmax; };
+    std::vector<SkinnyTask> all;
+    std::vector<Step> steps;
+    auto close = [&](size_t first) {
+        Step s{first, (int)(all.size() - first), 0, 0};
+        for (size_t i = first; i < all.size(); ++i) {
+            s.mmax = std::max(s.mmax, all[i].m);
+            s.kmax = std::max(s.kmax, all[i].k);
         }
-        TRY(run_gemms(c, g1));
-        TRY(run_gemms(c, g2));
+        if (s.cnt) steps.push_back(s);
+    };
+    for (int sweep = 0; sweep < 2; ++sweep) {
+        const bool fw = sweep == 0;
+        double *src = fw ? X : Z, *dst = fw ? Z : X;   // updated right-hand sides, solved blocks
+        for (int q = 0; q < NT; ++q) {
+            const int k = fw ? q : NT - 1 - q;
+            const double *yk = dst + (size_t)k * NB;
+            size_t first = all.size();
+            all.push_back(SkinnyTask{A->linv(k), src + (size_t)k * NB, dst + (size_t)k * NB, NB, n, NB, NB, N, N,
+                                     fw ? 0 : 1, fw ? 1 : 2, 1.0, 0.0});
+            close(first);
+            std::vector<SkinnyTask> upd;
+            first = all.size();
+            for (int o = fw ? k + 1 : 0; o < (fw ? NT : k); ++o) {
+                const int m = fw ? o : k, j = fw ? k : o;   // tile (m, j)
+                double *xo = src + (size_t)o * NB;
+                if (A->is_dense(m, j)) {
+                    all.push_back(SkinnyTask{A->dense(m, j), yk, xo, NB, n, NB, NB, N, N, fw ? 0 : 1, 0, -1.0, 1.0});
+                    continue;
+                }
+                const int r = A->rank(m, j);
+                if (r == 0) continue;
+                double *t = T + (size_t)o * A->maxrank * n;
+                all.push_back(SkinnyTask{fw ? A->V(m, j) : A->U(m, j), yk, t, r, n, NB, NB, N, r, 1, 0, 1.0, 0.0});
+                upd.push_back(SkinnyTask{fw ? A->U(m, j) : A->V(m, j), t, xo, NB, n, r, NB, r, N, 0, 0, -1.0, 1.0});
+            }
+            close(first);
+            first = all.size();
+            all.insert(all.end(), upd.begin(), upd.end());
+            close(first);
+        }
     }
-    for (int k = NT - 1; k >= 0; --k) {
-        double *xk = X + (size_t)k * NB;
-        g1.push_back(make_gemm(1, 0, NB, nrhs, NB, 1.0, A->linv(k), NB, xk, (int)N, 0.0, tmp, NB));
-        TRY(run_gemms(c, g1));
-        cp.push_back(make_copy(tmp, NB, xk, (int)N, NB, nrhs));
-        TRY(run_copies(c, cp));
-        for (int j = 0; j < k; ++j) {
-            double *xj = X + (size_t)j * NB;
-            if (A->is_dense(k, j)) {
-                g2.push_back(make_gemm(1, 0, NB, nrhs, NB, -1.0, A->dense(k, j), NB, xk, (int)N, 1.0, xj, (int)N));
-            } else {
-                const int r = A->rank(k, j);
-                if (r == 0) continue;
-                double *t = T2 + (size_t)j * A->maxrank * nrhs;
-                g1.push_back(make_gemm(1, 0, r, nrhs, NB, 1.0, A->U(k, j), NB, xk, (int)N, 0.0, t, r));
-                g2.push_back(make_gemm(0, 0, NB, nrhs, r, -1.0, A->V(k, j), NB, t, r, 1.0, xj, (int)N));
+#ifdef TLR_BOUNDS_CHECK
+    for (size_t i = 0; i < all.size(); ++i) {
+        const SkinnyTask &t = all[i];
+        BC(t.A, t.opA ? bc_span(t.k, t.m, t.lda) : bc_span(t.m, t.k, t.lda), "solve A", i);
+        BC(t.B, bc_span(t.k, t.n, t.ldb), "solve B", i);
+        BC(t.C, bc_span(t.m, t.n, t.ldc), "solve C", i);
+    }
+#endif
+    // staged in pieces of whole steps where the ring is too small for all of them
+    const size_t cap = c->stage_bytes / 2 / sizeof(SkinnyTask);
+    for (size_t s = 0; s < steps.size();) {
+        size_t e = s, cnt = 0;
+        while (e < steps.size() && (e == s || cnt + steps[e].cnt <= cap)) cnt += steps[e++].cnt;
+        SkinnyTask *d = stage(c, all.data() + steps[s].first, cnt);
+        if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
+        const size_t base = steps[s].first;
+        for (; s < e; ++s) {
+            const Step &st = steps[s];
+            double fl = 0, by = 0;
+            if (c->prof)
+                for (size_t i = st.first; i < st.first + st.cnt; ++i) {
+                    const double mk = (double)all[i].m * all[i].k * (all[i].tri ? 0.5 : 1.0);
+                    fl += 2.0 * mk * all[i].n;
+                    by += 8.0 * (mk + (double)all[i].n * (all[i].k + 2.0 * all[i].m));
+                }
+            Prof pf(c, P_GEMM, fl, by);
+            for (int o = 0; o < st.cnt; o += SKINNY_MAX_TASKS) {
+                launch_skinny_batched(d + (st.first - base) + o, std::min(st.cnt - o, SKINNY_MAX_TASKS), st.mmax, n,
+                                      st.kmax, c->cur);
+                TRY(check_launch(c));
             }
         }
-        TRY(run_gemms(c, g1));
-        TRY(run_gemms(c, g2));
     }
     return 0;
 }
@@ -3272,10 +3302,20 @@ int hicma_tlr_solve(hicma_tlr_ctx *c, hicma_tlr_desc *A, int nrhs, double *B, lo
     ws_reset(c);
     const size_t N = A->N;
     double *X = ws_alloc<double>(c, N * nrhs);
-    if (!X) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
+    double *T = ws_alloc<double>(c, (size_t)A->NT * A->maxrank * nrhs + 1);
+    if (!X || !T || !ws_alloc<double>(c, (size_t)A->NB * nrhs)) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
+    // the second right-hand-side buffer: as many columns as the arena has left (the
+    // critical-path arena, idle here, when that is not one)
+    int cols = (int)std::min<size_t>((size_t)nrhs, ws_free(c) / (N * sizeof(double) + 256));
+    double *Z = cols > 0 ? ws_alloc<double>(c, N * cols) : nullptr;
+    if (!Z) {
+        cols = (int)std::min<size_t>((size_t)nrhs, c->hi_ar.bytes / (N * sizeof(double)));
+        Z = (double *)c->hi_ar.base;
+        if (cols < 1) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
+    }
     CUDA_TRY(cudaMemcpy2DAsync(X, N * sizeof(double), B, ldb * sizeof(double), N * sizeof(double), nrhs,
                                cudaMemcpyHostToDevice, c->stream));
-    TRY(solve_dev(c, A, X, nrhs));
+    for (int j = 0; j < nrhs; j += cols) TRY(solve_dev(c, A, X + N * j, Z, T, std::min(cols, nrhs - j)));
     CUDA_TRY(cudaMemcpy2DAsync(B, ldb * sizeof(double), X, N * sizeof(double), N * sizeof(double), nrhs,
                                cudaMemcpyDeviceToHost, c->stream));
     TRY(ctx_sync(c));

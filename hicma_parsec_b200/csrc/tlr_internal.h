@@ -84,6 +84,22 @@ inline GemmTask make_gemm(int opA, int opB, int m, int n, int k, double alpha, c
     return t;
 }
 
+// ----------------------------------------------------- few right-hand sides --
+// C (m x n, ldc) = alpha op(A) B + beta C with few columns n; opA: 0 = N, 1 = T.
+// tri: A is lower triangular with zeros above (1: op N, 2: op T).  C must not
+// alias A or B.  mmax, nmax, kmax: the largest of the tasks; ntasks <=
+// SKINNY_MAX_TASKS.
+struct SkinnyTask {
+    const double *A, *B;
+    double *C;
+    int m, n, k;
+    int lda, ldb, ldc;
+    int opA, tri;
+    double alpha, beta;
+};
+constexpr int SKINNY_MAX_TASKS = 32768;   // grid.y
+void launch_skinny_batched(const SkinnyTask *d_tasks, int ntasks, int mmax, int nmax, int kmax, cudaStream_t st);
+
 // ------------------------------------------------------------ generation ----
 struct CovTask {
     double *out;
