@@ -7,17 +7,27 @@
 // products inside HCORE (low-rank SYRK/GEMM, QR/SVD recompression).
 //
 // CTA tile 64 x 64 x 16 (or 128 x 32 x 16 for outputs a rank wide), 4 warps
-// (2 x 2 or 4 x 1, 32 x 32 each = 4 x 4 DMMA tiles),
-// operands staged in shared memory by cp.async (2 stages, zero-filled at the
-// edges).  op(A)/op(B) transposes are handled by the load mapping so every
-// global load walks the contiguous dimension.  A batch is a list of tasks
-// whose output tiles are flattened into one grid (prefix sums in tile_off).
+// (2 x 2 or 4 x 1, 32 x 32 each = 4 x 4 DMMA tiles).  Operands are staged in
+// shared memory by cp.async in three stages with one barrier per 16-wide step,
+// zero-filled at the edges: 16-byte copies where base and leading dimension
+// allow, 8-byte ones otherwise.  An operand is stored along its contiguous
+// dimension, [k][x] or [x][k], with a pitch == 4 mod 16 doubles, so that copies
+// walk global memory and the DMMA fragment reads are free of bank conflicts in
+// either form; the four op combinations are separate instances.  Bound by the
+// DMMA rate (37 TFLOP/s) and by the last wave of CTAs.  Measured for C -= A op(B)
+// on a B200, against two stages, two barriers, 8-byte copies and a pitch of 72
+// (2-way conflicts): 2700^3 NT 22.8 -> 30.0, NN 20.8 -> 29.7, TN 17.4 -> 30.5
+// TFLOP/s; 10800^3 27.5 -> 33.4, 23.6 -> 33.2, 20.1 -> 34.3; 1000^3 13 -> 23.
+// Larger tiles (128 x 64, 128 x 128, 96 x 96) were slower at every size.
+// A batch is a list of tasks whose output tiles are flattened into one grid
+// (prefix sums in tile_off).
 #include "tlr_internal.h"
 
 namespace tlr {
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, PAD = 8, NT = 128;
+constexpr int BM = 64, BN = 64, BK = 16, NT = 128;
+constexpr int STAGES = 3;
 
 __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -25,10 +35,13 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void cp_async8(void *smem, const double *gmem, bool pred) {
-    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    int sz = pred ? 8 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
+__device__ __forceinline__ void cp_async8(unsigned smem, const double *gmem, bool pred) {
+    const int sz = pred ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem), "l"(gmem), "r"(sz));
+}
+// bytes: 16, 8 or 0 read from gmem (16-byte aligned), the rest zero-filled
+__device__ __forceinline__ void cp_async16(unsigned smem, const double *gmem, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -36,55 +49,46 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-template <int BM_, int BN_>
-struct Smem {
-    double A[2][BK][BM_ + PAD];
-    double B[2][BK][BN_ + PAD];
+// Shared layout of an operand with BX outer rows: KC (contiguous along k in
+// global memory) [x][BK + 4], else [k][BX + 4].
+template <int BX, bool KC>
+struct OpTile {
+    static constexpr int P = KC ? BK + 4 : BX + 4;
+    static constexpr int D = KC ? BX * P : BK * P;
 };
-
+template <int BX>
+constexpr int op_doubles() { return OpTile<BX, true>::D > OpTile<BX, false>::D ? OpTile<BX, true>::D : OpTile<BX, false>::D; }
 template <int BM_, int BN_>
-__device__ __forceinline__ void load_stage(Smem<BM_, BN_> &sm, int s, const GemmTask &t, int i0, int j0,
-                                           int k0) {
-    const int tid = threadIdx.x;
+constexpr size_t gemm_smem() { return sizeof(double) * STAGES * (op_doubles<BM_>() + op_doubles<BN_>()); }
+
+// Rows x0.. (below xe) and inner indices k0.. (below ke) of an operand into its stage.
+template <int BX, bool KC, bool V16>
+__device__ __forceinline__ void load_operand(double *sm, const double *X, int ld, int x0, int xe, int k0, int ke) {
+    constexpr int P = OpTile<BX, KC>::P, INNER = KC ? BK : BX, W = V16 ? 2 : 1;
+    const unsigned s0 = (unsigned)__cvta_generic_to_shared(sm);
+    const int ei = KC ? ke : xe, eo = KC ? xe : ke;
 #pragma unroll
-    for (int q = 0; q < (BM_ * BK) / NT; ++q) {
-        const int e = tid + q * NT;
-        int i, kk;
-        if (t.opA == 0) { i = e & (BM_ - 1); kk = e / BM_; }
-        else            { kk = e & (BK - 1); i = e / BK; }
-        const int gi = i0 + i, gk = k0 + kk;
-        const bool p = gi < t.m && gk < t.k;
-        const double *src = t.A;
-        if (p) src += (t.opA == 0) ? ((size_t)gi + (size_t)gk * t.lda) : ((size_t)gk + (size_t)gi * t.lda);
-        cp_async8(&sm.A[s][kk][i], src, p);
+    for (int q = 0; q < BX * BK / W / NT; ++q) {
+        const int e = threadIdx.x + q * NT;
+        const int in = (e % (INNER / W)) * W, ou = e / (INNER / W);
+        const int gi = (KC ? k0 : x0) + in, go = (KC ? x0 : k0) + ou;
+        const bool p = go < eo && gi < ei;
+        const double *src = p ? X + (size_t)gi + (size_t)go * ld : X;
+        const unsigned d = s0 + (unsigned)((ou * P + in) * sizeof(double));
+        if (V16) cp_async16(d, src, p ? (gi + 1 < ei ? 16 : 8) : 0);
+        else cp_async8(d, src, p);
     }
-#pragma unroll
-    for (int q = 0; q < (BN_ * BK) / NT; ++q) {
-        const int e = tid + q * NT;
-        int j, kk;
-        if (t.opB == 0) { kk = e & (BK - 1); j = e / BK; }
-        else            { j = e & (BN_ - 1); kk = e / BN_; }
-        const int gj = j0 + j, gk = k0 + kk;
-        const bool p = gj < t.n && gk < t.k;
-        const double *src = t.B;
-        if (p) src += (t.opB == 0) ? ((size_t)gk + (size_t)gj * t.ldb) : ((size_t)gj + (size_t)gk * t.ldb);
-        cp_async8(&sm.B[s][kk][j], src, p);
-    }
-    cp_async_commit();
 }
 
 // One BM_ x BN_ output tile; four warps of 32 x 32 (2 x 2 for 64 x 64,
-// 4 x 1 for the narrow 128 x 32 tile used when n is a rank).
-template <int BM_, int BN_>
-__device__ __forceinline__ void gemm_tile(Smem<BM_, BN_> &sm, GemmTask t, int tm, int tn) {
+// 4 x 1 for the narrow 128 x 32 tile used when n is a rank).  AK / BKC: op(A) /
+// op(B) is contiguous along the inner dimension (opA = 1, opB = 0).
+template <int BM_, int BN_, bool AK, bool BKC, bool V16>
+__device__ __forceinline__ void gemm_tile_op(double *sm, const GemmTask &t, int n, int i0, int j0) {
+    using OA = OpTile<BM_, AK>;
+    using OB = OpTile<BN_, BKC>;
     constexpr int WM = BM_ / 32;
-    const int i0 = tm * BM_, j0 = tn * BN_;
-    if (t.lower && j0 >= i0 + BM_) return;
-    if (t.n_dev) {
-        const int nd = *t.n_dev;
-        t.n = nd < t.n ? nd : t.n;
-    }
-    if (j0 >= t.n) return;
+    constexpr int SI = AK ? OA::P : 1, SKA = AK ? 1 : OA::P, SJ = BKC ? OB::P : 1, SKB = BKC ? 1 : OB::P;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tig = lane & 3;
     const int wm = warp % WM, wn = warp / WM;
@@ -100,29 +104,37 @@ __device__ __forceinline__ void gemm_tile(Smem<BM_, BN_> &sm, GemmTask t, int tm
     if (t.tri == 1) kend = min(kend, i0 + BM_);
     else if (t.tri == 2) kend = min(kend, j0 + BN_);
     const int ktiles = (kend + BK - 1) / BK;
-    if (ktiles > 0) load_stage<BM_, BN_>(sm, 0, t, i0, j0, 0);
+    auto load = [&](int s, int kt) {
+        double *sa = sm + s * (OA::D + OB::D);
+        load_operand<BM_, AK, V16>(sa, t.A, t.lda, i0, t.m, kt * BK, t.k);
+        load_operand<BN_, BKC, V16>(sa + OA::D, t.B, t.ldb, j0, n, kt * BK, t.k);
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < ktiles) load(s, s);
+        cp_async_commit();
+    }
+    int s = 0;
     for (int kt = 0; kt < ktiles; ++kt) {
-        const int s = kt & 1;
-        if (kt + 1 < ktiles) {
-            load_stage<BM_, BN_>(sm, s ^ 1, t, i0, j0, (kt + 1) * BK);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();   // the stage is complete, and the one loaded next is no longer read
+        if (kt + STAGES - 1 < ktiles) load(s == 0 ? STAGES - 1 : s - 1, kt + STAGES - 1);
+        cp_async_commit();
+        const double *sa = sm + s * (OA::D + OB::D), *sb = sa + OA::D;
+        const double *pa = sa + (wm * 32 + g) * SI + tig * SKA, *pb = sb + (wn * 32 + g) * SJ + tig * SKB;
 #pragma unroll
         for (int k4 = 0; k4 < BK; k4 += 4) {
             double a[4], b[4];
 #pragma unroll
-            for (int mi = 0; mi < 4; ++mi) a[mi] = sm.A[s][k4 + tig][wm * 32 + mi * 8 + g];
+            for (int mi = 0; mi < 4; ++mi) a[mi] = pa[mi * 8 * SI + k4 * SKA];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) b[ni] = sm.B[s][k4 + tig][wn * 32 + ni * 8 + g];
+            for (int ni = 0; ni < 4; ++ni) b[ni] = pb[ni * 8 * SJ + k4 * SKB];
 #pragma unroll
             for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
         }
-        __syncthreads();
+        s = s + 1 == STAGES ? 0 : s + 1;
     }
 
     const double alpha = t.alpha, beta = t.beta;
@@ -135,13 +147,33 @@ __device__ __forceinline__ void gemm_tile(Smem<BM_, BN_> &sm, GemmTask t, int tm
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int col = j0 + wn * 32 + ni * 8 + tig * 2 + e;
-                if (col >= t.n) continue;
+                if (col >= n) continue;
                 double *c = t.C + (size_t)row + (size_t)col * t.ldc;
                 double v = alpha * acc[mi][ni][e];
                 if (beta != 0.0) v += beta * (*c);
                 *c = v;
             }
         }
+    }
+}
+
+template <int BM_, int BN_>
+__device__ __forceinline__ void gemm_tile(double *sm, const GemmTask &t, int tm, int tn) {
+    const int i0 = tm * BM_, j0 = tn * BN_;
+    if (t.lower && j0 >= i0 + BM_) return;
+    int n = t.n;
+    if (t.n_dev) n = min(n, *t.n_dev);
+    if (j0 >= n) return;
+    const bool v16 = (((size_t)t.A | (size_t)t.B) & 15) == 0 && ((t.lda | t.ldb) & 1) == 0;
+    switch ((t.opA ? 4 : 0) | (t.opB ? 2 : 0) | (v16 ? 1 : 0)) {
+        case 0: gemm_tile_op<BM_, BN_, false, true, false>(sm, t, n, i0, j0); break;
+        case 1: gemm_tile_op<BM_, BN_, false, true, true>(sm, t, n, i0, j0); break;
+        case 2: gemm_tile_op<BM_, BN_, false, false, false>(sm, t, n, i0, j0); break;
+        case 3: gemm_tile_op<BM_, BN_, false, false, true>(sm, t, n, i0, j0); break;
+        case 4: gemm_tile_op<BM_, BN_, true, true, false>(sm, t, n, i0, j0); break;
+        case 5: gemm_tile_op<BM_, BN_, true, true, true>(sm, t, n, i0, j0); break;
+        case 6: gemm_tile_op<BM_, BN_, true, false, false>(sm, t, n, i0, j0); break;
+        default: gemm_tile_op<BM_, BN_, true, false, true>(sm, t, n, i0, j0); break;
     }
 }
 
@@ -156,7 +188,7 @@ __device__ __forceinline__ int task_of(const int *__restrict__ tile_off, int nta
 template <int BM_, int BN_>
 __global__ void __launch_bounds__(NT, 3) k_gemm_batched(const GemmTask *__restrict__ tasks,
                                                      const int *__restrict__ tile_off, int ntasks) {
-    __shared__ __align__(16) Smem<BM_, BN_> sm;
+    extern __shared__ __align__(16) double sm[];
     const int bid = blockIdx.x;
     const int lo = task_of(tile_off, ntasks, bid);
     const GemmTask t = tasks[lo];
@@ -164,8 +196,8 @@ __global__ void __launch_bounds__(NT, 3) k_gemm_batched(const GemmTask *__restri
     gemm_tile<BM_, BN_>(sm, t, local % t.tiles_m, local / t.tiles_m);
 }
 
-__global__ void __launch_bounds__(NT) k_gemm_single(GemmTask t) {
-    __shared__ __align__(16) Smem<BM, BN> sm;
+__global__ void __launch_bounds__(NT, 3) k_gemm_single(GemmTask t) {
+    extern __shared__ __align__(16) double sm[];
     gemm_tile<BM, BN>(sm, t, blockIdx.x, blockIdx.y);
 }
 
@@ -264,20 +296,26 @@ void launch_gemm_batched(const GemmTask *d_tasks, const int *d_tile_off, int nta
     if (ntasks <= 0 || total_tiles <= 0) return;
     if (fp32)
         k_sgemm_batched<<<total_tiles, 256, 0, st>>>(d_tasks, d_tile_off, ntasks);
-    else
-        k_gemm_batched<BM, BN><<<total_tiles, NT, 0, st>>>(d_tasks, d_tile_off, ntasks);
+    else {
+        // per device and thread-safe: set on every launch (a host-side call, no synchronisation)
+        cudaFuncSetAttribute(k_gemm_batched<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<BM, BN>());
+        k_gemm_batched<BM, BN><<<total_tiles, NT, gemm_smem<BM, BN>(), st>>>(d_tasks, d_tile_off, ntasks);
+    }
 }
 
 void launch_gemm_batched_narrow(const GemmTask *d_tasks, const int *d_tile_off, int ntasks, int total_tiles,
                                 cudaStream_t st) {
     if (ntasks <= 0 || total_tiles <= 0) return;
-    k_gemm_batched<GEMM_NARROW_M, GEMM_NARROW_N><<<total_tiles, NT, 0, st>>>(d_tasks, d_tile_off, ntasks);
+    constexpr size_t smem = gemm_smem<GEMM_NARROW_M, GEMM_NARROW_N>();
+    cudaFuncSetAttribute(k_gemm_batched<GEMM_NARROW_M, GEMM_NARROW_N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_gemm_batched<GEMM_NARROW_M, GEMM_NARROW_N><<<total_tiles, NT, smem, st>>>(d_tasks, d_tile_off, ntasks);
 }
 
 void launch_gemm_single(const GemmTask &t, cudaStream_t st) {
     if (t.m <= 0 || t.n <= 0) return;
     dim3 grid((t.m + BM - 1) / BM, (t.n + BN - 1) / BN);
-    k_gemm_single<<<grid, NT, 0, st>>>(t);
+    cudaFuncSetAttribute(k_gemm_single, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<BM, BN>());
+    k_gemm_single<<<grid, NT, gemm_smem<BM, BN>(), st>>>(t);
 }
 
 }  // namespace tlr
