@@ -83,33 +83,86 @@ __device__ __forceinline__ bool pair_scaled(double &aa, double &bb, double &cc, 
 // Rotation that makes the pair orthogonal: x' = cs x - sn y, y' = sn x + cs y.
 // With h = sqrt((bb - aa)^2 + 4 cc^2): cs^2 = (1 + |bb - aa| / h) / 2 and
 // sn cs = |cc| / h (the small angle).  cs = 1, sn = 0 where none is needed.
-__device__ __forceinline__ bool pair_rotation(double aa, double bb, double cc, double tau2, double tol2, double &cs,
-                                              double &sn) {
-    cs = 1.0;
-    sn = 0.0;
-    if (!pair_scaled(aa, bb, cc, tau2, tol2)) return false;
-    const double d = bb - aa;
-    const double rh = rsqrt(fma(d, d, 4.0 * cc * cc));
+// On the critical path of a round: the test runs beside the rotation, and the
+// scaling only where a square could over- or underflow.
+__device__ __forceinline__ double2 pair_rotation(double aa, double bb, double cc, double tau2, double tol2) {
+    bool need = aa > tau2 && bb > tau2 && cc * cc > tol2 * aa * bb;
+    if (!(fmin(aa, bb) > 1e-120 && fmax(aa, bb) < 1e140)) need = pair_scaled(aa, bb, cc, tau2, tol2);
+    const double d = bb - aa, c2x = cc + cc;
+    const double rh = rsqrt(fma(d, d, c2x * c2x));
     const double c2 = fma(0.5 * fabs(d), rh, 0.5);
     const double rc = rsqrt(c2);
-    cs = c2 * rc;
-    sn = copysign(1.0, d) * cc * rh * rc;
-    return true;
+    return make_double2(need ? c2 * rc : 1.0, need ? copysign(cc, d * cc) * rh * rc : 0.0);
 }
 
-// 2 x 2 block of G at rows (a0, b0) and columns (a1, b1): rotated by the row
-// pair's (c0, s0) and the column pair's (c1, s1).
-__device__ __forceinline__ void rotate_block(double *G, int ld, int a0, int b0, double c0, double s0, int a1, int b1,
-                                             double c1, double s1, bool diag) {
-    double *pa = G + a0 * ld, *pb = G + b0 * ld;
-    const double gaa = pa[a1], gab = pa[b1], gba = pb[a1], gbb = pb[b1];
-    const double u0 = c1 * gaa - s1 * gab, u1 = s1 * gaa + c1 * gab;
-    const double v0 = c1 * gba - s1 * gbb, v1 = s1 * gba + c1 * gbb;
-    pa[a1] = c0 * u0 - s0 * v0;
-    pb[b1] = s0 * u1 + c0 * v1;
-    // a diagonal block holds its own pair: the rotation made it zero
-    pa[b1] = diag ? 0.0 : c0 * u1 - s0 * v1;
-    pb[a1] = diag ? 0.0 : s0 * u0 + c0 * v0;
+// G is symmetric: entry (x, y) of the lower triangle stored.
+__device__ __forceinline__ int low(int x, int y, int ld) { return x > y ? x * ld + y : y * ld + x; }
+
+// Blocks (I, J), I >= J, of G's lower triangle by pairs, in the order of a
+// linear index (J of 16 bits above I of 16 bits).
+__device__ __forceinline__ int tri_block(int q) {
+    int i = 0;
+    while ((i + 1) * (i + 2) / 2 <= q) ++i;
+    return i | ((q - i * (i + 1) / 2) << 16);
+}
+
+// G <- J^T G J on the NB blocks blk[] of a thread (2 x 2 blocks of G at
+// the pairs I and J, a | b << 16, rotations rot[]), all loaded before any is
+// written, without branches.  A diagonal block belongs to one pair: the rotation
+// makes its off-diagonal entry zero.
+template <int NB>
+__device__ __forceinline__ void rotate_blocks(double *G, int ld, const int (&blk)[NB], const double2 *rot,
+                                              const int *pab) {
+    double2 cr[NB], cc[NB];
+    double gaa[NB], gab[NB], gba[NB], gbb[NB];
+    int iaa[NB], iab[NB], iba[NB], ibb[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int I = blk[q] & 0xffff, J = blk[q] >> 16;
+        cr[q] = rot[I];
+        cc[q] = rot[J];
+        const int pi = pab[I], pj = pab[J];
+        const int a0 = pi & 0xffff, b0 = pi >> 16, a1 = pj & 0xffff, b1 = pj >> 16;
+        iaa[q] = low(a0, a1, ld);
+        iab[q] = low(a0, b1, ld);
+        iba[q] = low(b0, a1, ld);
+        ibb[q] = low(b0, b1, ld);
+        gaa[q] = G[iaa[q]];
+        gab[q] = G[iab[q]];
+        gba[q] = G[iba[q]];
+        gbb[q] = G[ibb[q]];
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const double u0 = cc[q].x * gaa[q] - cc[q].y * gab[q], u1 = cc[q].y * gaa[q] + cc[q].x * gab[q];
+        const double v0 = cc[q].x * gba[q] - cc[q].y * gbb[q], v1 = cc[q].y * gba[q] + cc[q].x * gbb[q];
+        const bool diag = (blk[q] & 0xffff) == blk[q] >> 16;
+        G[iaa[q]] = cr[q].x * u0 - cr[q].y * v0;
+        G[ibb[q]] = cr[q].y * u1 + cr[q].x * v1;
+        // (on a diagonal block that needed no rotation the entry stays)
+        const double vab = cr[q].x * u1 - cr[q].y * v1, vba = cr[q].y * u0 + cr[q].x * v0;
+        const bool zero = diag && cr[q].y != 0.0;
+        G[iab[q]] = zero ? 0.0 : vab;
+        G[iba[q]] = zero ? 0.0 : vba;
+    }
+}
+
+// Rotates the column pair ab (rotation r) in R rows of M from row c0 on, step rows
+// apart (row-major, pitch ld), all loaded before any is written.
+template <int R>
+__device__ __forceinline__ void rotate_rows(double *M, int ld, int ab, double2 r, int c0, int step) {
+    double *pa = M + c0 * ld + (ab & 0xffff), *pb = M + c0 * ld + (ab >> 16);
+    double xa[R], xb[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        xa[q] = pa[q * step * ld];
+        xb[q] = pb[q * step * ld];
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        pa[q * step * ld] = r.x * xa[q] - r.y * xb[q];
+        pb[q * step * ld] = r.y * xa[q] + r.x * xb[q];
+    }
 }
 
 // Truncation floor on squared norms: 1e-3 of the absolute threshold
@@ -157,23 +210,34 @@ __device__ __forceinline__ int core_rank(const CoreParams &p, int K, int k, doub
 // from the norms in shared memory, and the two barriers of a step are after
 // the norms and after the pivot column is published.  Bound by the latency of
 // those steps and of the Jacobi rounds; several CTAs share an SM.
-// Against one CTA with dot products reduced over 8 or 16 lanes and two to three
-// shuffles a value (the form before): the cores of the 60 x 60 tiles of 2700 2D
-// workload (34,220 of K up to 100) 142 -> 74 ms, 20 x 20 tiles of 1350 90 -> 33 ms.
+// In a Jacobi round the first warps find the next round's rotations (about 600
+// cycles of dependent FP64 operations) while the others rotate the rows of X; G is
+// stored by its lower triangle with an odd pitch, since its blocks are read along
+// rows and columns alike.  Latency of one core with k = 0.83 K: K = 32, 64, 80 107,
+// 405, 791 us (145, 499, 1146 with the rotations found before both updates and G
+// full with 4-way conflicts).  Against one CTA with dot products reduced over 8 or
+// 16 lanes and two to three shuffles a value: the cores of the 60 x 60 tiles of
+// 2700 2D workload (34,220 of K up to 100) 142 -> 74 ms, 20 x 20 tiles of 1350 90
+// -> 33 ms.
 template <int KM>
 struct SmallCore {
     static constexpr int NT = 4 * KM;
     static constexpr int NW = NT / 32;
-    static constexpr int P = KM + 4;          // == 4 mod 16: conflict-free DMMA fragments
+    static constexpr int P = KM + 4;          // pitch of X, == 4 mod 16: conflict-free DMMA fragments
+    static constexpr int PG = KM + 1;         // pitch of G, odd: its rows and columns are read alike
     static constexpr int NT8 = KM / 8;
-    static constexpr size_t doubles = 2 * (size_t)KM * P + 2 * KM + KM;   // X, G, sig, hv, (cs, sn)
-    static constexpr size_t bytes = sizeof(double) * doubles + sizeof(int) * 2 * KM;
+    static constexpr int NBLK = (KM / 2) * (KM / 2 + 1) / 2;   // 2 x 2 blocks of G's lower triangle
+    static constexpr int BPT = (NBLK + NT - 1) / NT;           // of them a thread rotates
+    static constexpr int XR = KM + 4 * NW;                     // rows of X: batches of four a warp
+    // X, G and an idle entry, sig, hv, 2 x (cs, sn) of KM / 2 pairs and the idle pair
+    static constexpr size_t doubles = (size_t)XR * P + (KM + 1) * PG + 1 + 2 * KM + 2 * (KM + 2);
+    static constexpr size_t bytes = sizeof(double) * doubles + sizeof(int) * (2 * KM + 2);
 };
 
 template <int KM>
 __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restrict__ tasks, CoreParams p) {
     using S = SmallCore<KM>;
-    constexpr int NT = S::NT, NW = S::NW, P = S::P, NT8 = S::NT8;
+    constexpr int NT = S::NT, NW = S::NW, P = S::P, PG = S::PG, NT8 = S::NT8;
     constexpr int Q = KM / 4;                 // rows a lane holds
     constexpr int NSLOT = (KM + 31) / 32;     // columns a lane scans for the pivot
     extern __shared__ __align__(16) double sm[];
@@ -190,11 +254,12 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
         return;
     }
     double *X = sm;                           // X(c, i) at c * P + i; T(r, c) at c * P + r before the QR
-    double *G = X + KM * P;
-    double *sig = G + KM * P;
+    double *G = X + S::XR * P;
+    double *sig = G + (KM + 1) * PG + 1;      // keeps what follows 16-byte aligned: PG is odd
     double *hv = sig + KM;
-    double2 *rot = (double2 *)(hv + KM);      // KM / 2 rotations of a round
-    int *order = (int *)(rot + KM / 2);
+    double2 *rot = (double2 *)(hv + KM);      // KM / 2 rotations of this and of the next round, an idle one each
+    constexpr int RP = KM / 2 + 1;
+    int *order = (int *)(rot + 2 * RP);
     int *pab = order + KM;                    // their column pairs, a | b << 16
 
     // 1. T = M^T: T(i, c) = sum_{l >= max(i, c)} RU(c, l) RV(i, l), the entries
@@ -241,19 +306,11 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
     if (sub == 0) sig[col] = s2;
     bool active = col < K;
     __syncthreads();
-    // largest squared norm (scale of the pivot keys) and their sum
-    double nmax = 0.0, total = 0.0;
+    double total = 0.0;
 #pragma unroll
-    for (int s = 0; s < NSLOT; ++s) {
-        const double v = lane + 32 * s < KM ? sig[lane + 32 * s] : 0.0;
-        nmax = fmax(nmax, v);
-        total += v;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nmax = fmax(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
+    for (int s = 0; s < NSLOT; ++s) total += lane + 32 * s < KM ? sig[lane + 32 * s] : 0.0;
     total = group_sum<32>(total);
     const double tau2 = trunc_floor(p, total);
-    const double kscale = nmax > 1e-290 && nmax < 1e290 ? 1.0 / nmax : 1.0;
 
     // 2. pivoted Householder QR of T, stopped when the trailing mass <= tau2
     unsigned done[NSLOT];                     // columns this lane scans that were pivots already
@@ -262,8 +319,8 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
     int k = K;
     double dropped = 0.0;
     for (int j = 0; j < K; ++j) {
-        // pivot: the column of largest norm (single-precision keys of the
-        // scaled norms; the lowest index of equal ones)
+        // pivot: the column of largest norm, by the upper half of the double
+        // (20 bits of mantissa; the lowest index of equal ones)
         unsigned best = 0u;
         int bc = 0;
         double tr = 0.0;
@@ -272,7 +329,7 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
             if (!done[s]) {
                 const double v = sig[lane + 32 * s];
                 tr += v;
-                const unsigned key = __float_as_uint((float)(v * kscale)) + 1u;
+                const unsigned key = (unsigned)__double2hiint(v) + 1u;
                 if (key > best) { best = key; bc = lane + 32 * s; }
             }
         }
@@ -281,7 +338,7 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
         tr = group_sum<32>(tr);
         if (!(tr > tau2)) { k = j; dropped = tr; break; }    // the same in every warp
         pc = min(pc, KM - 1);
-        const double n2 = sig[pc];
+        const double n2 = sig[pc], sn = sqrt(n2);
         if ((pc & 31) == lane) {
 #pragma unroll
             for (int s = 0; s < NSLOT; ++s)
@@ -294,7 +351,7 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
         __syncthreads();
         // H = I - v v^T / (n2 - alpha beta), v = x - beta e_j, beta = -sign(alpha) ||x||
         const double alpha = hv[j];
-        const double beta = -copysign(sqrt(n2), alpha);
+        const double beta = -copysign(sn, alpha);
         const double den = fma(-alpha, beta, n2);
         const double th = den > 0.0 ? 1.0 / den : 0.0;
         double v[Q], w0 = 0.0, w1 = 0.0;
@@ -336,9 +393,33 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
     // columns k .. 8 nk8 take part in the Gram tiles: zero
     for (int idx = tid; idx < KM * (8 * nk8 - k); idx += NT) X[(idx % KM) * P + k + idx / KM] = 0.0;
     __syncthreads();
-    const int L = np <= 8 ? 8 : np <= 16 ? 16 : 32;   // lanes over pairs
+    // the first warps find the rotations of the next round while the others
+    // rotate the rows of X, lanes over pairs
+    const int nwa = np > 32 && NW > 2 ? 2 : 1;
+    const int L = np <= 8 ? 8 : np <= 16 ? 16 : 32;
     const int RS = 32 / L;                            // rows a warp takes at a time
-    const int li = lane % L, lr = warp * RS + lane / L, rstep = NW * RS;
+    const int li = lane % L, lr = (warp - nwa) * RS + lane / L, rstep = (NW - nwa) * RS;
+    int blk[S::BPT];                                  // this thread's blocks of G, -1: none
+#pragma unroll
+    for (int q = 0; q < S::BPT; ++q) {
+        const int e = tid + q * NT;
+        blk[q] = e < np * (np + 1) / 2 ? tri_block(e) : (KM / 2) | ((KM / 2) << 16);
+    }
+    // the idle pair of threads without a block: no rotation, of the idle entry
+    if (tid < 2) {
+        rot[tid * RP + KM / 2] = make_double2(1.0, 0.0);
+        pab[tid * RP + KM / 2] = KM | (KM << 16);
+        G[KM * PG + KM] = 0.0;
+    }
+    auto angles = [&](int round, int buf) {
+        for (int pr = tid; pr < np; pr += 32 * nwa) {
+            const int a = tourney(pr, round, kp), b = tourney(kp - 1 - pr, round, kp);
+            rot[buf * RP + pr] = max(a, b) < k
+                                           ? pair_rotation(G[a * PG + a], G[b * PG + b], G[low(a, b, PG)], tau2, tol2)
+                                           : make_double2(1.0, 0.0);
+            pab[buf * RP + pr] = a | (b << 16);
+        }
+    };
     while (k > 0) {
         // G = X^T X (rows past K are zero)
         for (int q = warp; q < nk8 * (nk8 + 1) / 2; q += NW) {
@@ -354,11 +435,7 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
             }
             if (c < K) dmma884(a0, X[(c + tig) * P + 8 * I + g], X[(c + tig) * P + 8 * J + g]);
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const double v = a0[e] + a1[e];
-                G[(8 * I + g) * P + 8 * J + 2 * tig + e] = v;
-                G[(8 * J + 2 * tig + e) * P + 8 * I + g] = v;
-            }
+            for (int e = 0; e < 2; ++e) G[(8 * I + g) * PG + 8 * J + 2 * tig + e] = a0[e] + a1[e];
         }
         __syncthreads();
         if (sweeps >= MAX_SWEEPS) break;
@@ -366,36 +443,33 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
         for (int idx = tid; idx < k * k; idx += NT) {
             const int i = idx / k, jj = idx - i * k;
             if (jj < i) {
-                double aa = G[i * P + i], bb = G[jj * P + jj], cc = G[i * P + jj];
+                double aa = G[i * PG + i], bb = G[jj * PG + jj], cc = G[i * PG + jj];
                 need |= pair_scaled(aa, bb, cc, tau2, tol2);
             }
         }
         if (!__syncthreads_or(need)) break;
         ++sweeps;
+        if (warp < nwa) angles(0, 0);
+        __syncthreads();
         for (int round = 0; round < kp - 1; ++round) {
-            for (int pr = tid; pr < np; pr += NT) {
-                const int a = tourney(pr, round, kp), b = tourney(kp - 1 - pr, round, kp);
-                double cs = 1.0, sn = 0.0;
-                if (max(a, b) < k) pair_rotation(G[a * P + a], G[b * P + b], G[a * P + b], tau2, tol2, cs, sn);
-                rot[pr] = make_double2(cs, sn);
-                pab[pr] = a | (b << 16);
-            }
+            const double2 *rr = rot + (round & 1) * RP;
+            const int *pp = pab + (round & 1) * RP;
+            rotate_blocks<S::BPT>(G, PG, blk, rr, pp);
             __syncthreads();
-            for (int I = li; I < np; I += L) {
-                const double2 ri = rot[I];
-                const int ab = pab[I], a = ab & 0xffff, b = ab >> 16;
-                for (int J = lr; J < np; J += rstep) {
-                    const double2 rj = rot[J];
-                    if (ri.y == 0.0 && rj.y == 0.0) continue;
-                    const int abj = pab[J];
-                    rotate_block(G, P, abj & 0xffff, abj >> 16, rj.x, rj.y, a, b, ri.x, ri.y, I == J);
-                }
-                if (ri.y != 0.0) {
-                    for (int c = lr; c < K; c += rstep) {
-                        const double xa = X[c * P + a], xb = X[c * P + b];
-                        X[c * P + a] = ri.x * xa - ri.y * xb;
-                        X[c * P + b] = ri.y * xa + ri.x * xb;
-                    }
+            if (warp < nwa) {
+                if (round + 1 < kp - 1) angles(round + 1, (round + 1) & 1);
+            } else {
+                for (int I = li; I < np; I += L) {
+                    const double2 r = rr[I];
+                    const int ab = pp[I];
+                    if (r.y == 0.0) continue;
+                    // batches of four rows a warp; a last batch past K ends in X's padding
+                    if (RS == 1)
+                        for (int c = lr; c < K; c += 4 * rstep) rotate_rows<4>(X, P, ab, r, c, rstep);
+                    else if (RS == 2)
+                        for (int c = lr; c < K; c += 2 * rstep) rotate_rows<2>(X, P, ab, r, c, rstep);
+                    else
+                        for (int c = lr; c < K; c += rstep) rotate_rows<1>(X, P, ab, r, c, rstep);
                 }
             }
             __syncthreads();
@@ -404,7 +478,7 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
 
     // 4. singular values (from the fresh Gram matrix), descending order, rank
     for (int c = tid; c < k; c += NT) {
-        sig[c] = sqrt(G[c * P + c]);
+        sig[c] = sqrt(G[c * PG + c]);
         order[c] = c;
     }
     __syncthreads();
@@ -450,11 +524,15 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
 // matrix, rotations of the Gram matrix with the rotations accumulated in J,
 // then the columns times J.  Bound by the latency of the rounds: the 31
 // rotation rounds of a pair problem take about as long as its two products.
-// Two launches of three cores and one of K about 650 (k about 430): 470 -> 38 ms
-// against one warp per column pair reading its columns through L2.
+// Pairs within a block are rotated once a sweep, pairs across two blocks in the
+// round that brings the blocks together (16 rotation rounds of about 800 cycles).
+// One core of K = 96, 256, 400: 0.52, 2.4, 9.0 ms.  Two launches of three cores and
+// one of K about 650 (k about 430): 470 -> 32 ms against one warp per column pair
+// reading its columns through L2.
 constexpr int WB = 16;                        // columns of a block
 constexpr int WP = 2 * WB;                    // columns of a pair problem
-constexpr int WLD = WP + 4;                   // pitch of its G and J
+constexpr int WLD = WP + 4;                   // pitch of its J (conflict-free DMMA fragments)
+constexpr int WGD = WP + 1;                   // pitch of its G (rows and columns read alike)
 constexpr int W_CT = 256;
 constexpr int W_NW = W_CT / 32;
 constexpr int W_TILES = 10;                   // lower 8 x 8 tiles of the 32 x 32 Gram matrix
@@ -478,8 +556,8 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) double sm[];
     __shared__ WidePub pub[2][W_CSMAX];
-    __shared__ double2 rot[WP / 2];
-    __shared__ int pab[WP / 2];
+    __shared__ double2 rot[2][WP / 2];
+    __shared__ int pab[2][WP / 2];
     __shared__ int rank_sh;
     const int CS = (int)cl.num_blocks(), crank = (int)cl.block_rank();
     const CoreTask t = tasks[blockIdx.x / CS];
@@ -500,7 +578,7 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
     double *sig = X + (size_t)K * (K + WP);
     double *Tg = sig + K;
     int *rotf = (int *)(Tg + (size_t)K * (K + W_CSMAX));  // [sweep]: a pair was rotated
-    const int ncl = wide_ncl(K, CS);
+    const int ncl = wide_ncl(K, CS), lcs = __ffs(CS) - 1;   // CS is a power of two
     double *hv = sm;                          // K
     double *sigl = hv + K;                    // ncl: squared norms of the CTA's columns, -1 once pivots
     double *Ts = sigl + ncl + ((K + ncl) & 1);
@@ -562,41 +640,45 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
     for (int j = 0; j < K; ++j) {
         const int par = j & 1;
         if (warp == 0) {
-            double tr = 0.0, best = -1.0;
-            int bc = 0x7fffffff;
+            // the CTA's best column (by the upper half of the norm) and its sum of norms
+            double tr = 0.0;
+            unsigned best = 0u;
+            int bq = 0x7fffffff;
             for (int q = lane; q < nc; q += 32) {
                 const double v = sigl[q];
                 if (v < 0.0) continue;
                 tr += v;
-                if (v > best) { best = v; bc = crank + CS * q; }
+                const unsigned key = (unsigned)__double2hiint(v) + 1u;
+                if (key > best) { best = key; bq = q; }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                tr += __shfl_xor_sync(0xffffffffu, tr, o);
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
-                if (ob > best || (ob == best && oc < bc)) { best = ob; bc = oc; }
-            }
+            const unsigned top = __reduce_max_sync(0xffffffffu, best);
+            bq = __reduce_min_sync(0xffffffffu, best == top ? bq : 0x7fffffff);
+            tr = group_sum<32>(tr);
             if (lane < CS) {
                 WidePub *d = cl.map_shared_rank(&pub[par][crank], lane);
-                d->norm = best;
+                d->norm = top ? sigl[bq] : -1.0;
                 d->sum = tr;
-                d->col = bc;
+                d->col = top ? crank + CS * bq : 0x7fffffff;
             }
         }
         cl.sync();
+        // best of the CTAs: the same comparison in every warp of the cluster
         double tr = 0.0, n2 = -1.0;
         int pc = 0x7fffffff;
-        for (int r = 0; r < CS; ++r) {
-            const double v = pub[par][r].norm;
-            const int c = pub[par][r].col;
-            tr += pub[par][r].sum;
-            if (v > n2 || (v == n2 && c < pc)) { n2 = v; pc = c; }
+        {
+            const WidePub e = pub[par][lane & (CS - 1)];
+            tr = lane < CS ? e.sum : 0.0;
+            const unsigned key = e.norm >= 0.0 || e.norm != e.norm ? (unsigned)__double2hiint(e.norm) + 1u : 0u;
+            const unsigned top = __reduce_max_sync(0xffffffffu, key);
+            pc = __reduce_min_sync(0xffffffffu, key == top ? e.col : 0x7fffffff);
+            tr = group_sum<32>(tr);
         }
         if (j == 0) tau2 = trunc_floor(p, tr);
         if (!(tr > tau2) || pc >= K) { k = j; dropped = tr; break; }   // the same in every CTA
         // the pivot column, from its owner's memory (nothing writes it any more)
-        const int owner = pc % CS, lp = pc / CS;
+        const int owner = pc & (CS - 1), lp = pc >> lcs;
+        n2 = pub[par][owner].norm;
+        const double sn = sqrt(n2);
         if (t_in_smem) {
             const double *src = cl.map_shared_rank(Ts, owner) + (size_t)lp * K;
             for (int r = j + tid; r < K; r += W_CT) hv[r] = src[r];
@@ -606,35 +688,50 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
         }
         __syncthreads();
         const double alpha = hv[j];
-        const double beta = -copysign(sqrt(n2), alpha);
+        const double beta = -copysign(sn, alpha);
         const double den = fma(-alpha, beta, n2);
         const double th = den > 0.0 ? 1.0 / den : 0.0;
-        for (int q = warp; q < nc; q += W_NW) {
-            const int c = crank + CS * q;
-            const bool act = sigl[q] >= 0.0;
-            double rj = 0.0;
-            if (c == pc) {
-                rj = beta;
-            } else if (act) {
-                double *tc = Tl + (size_t)q * K;
-                double w = 0.0;
-#pragma unroll 4
-                for (int r = j + lane; r < K; r += 32) w = fma(r == j ? alpha - beta : hv[r], tc[r], w);
-                w = group_sum<32>(w) * th;
-                double s2 = 0.0;
-#pragma unroll 4
-                for (int r = j + lane; r < K; r += 32) {
-                    const double x = fma(-w, r == j ? alpha - beta : hv[r], tc[r]);
-                    tc[r] = x;
-                    if (r == j) rj = x;
-                    else s2 = fma(x, x, s2);
+        // eight lanes a column, four columns a warp; row j apart (v_j = alpha - beta)
+        const int gl = lane & 7;
+        for (int q0 = 4 * warp; q0 < nc; q0 += 4 * W_NW) {
+            const int q = q0 + (lane >> 3), c = crank + CS * q;
+            const bool act = q < nc && c != pc && sigl[q] >= 0.0;
+            double *tc = Tl + (size_t)q * K;
+            double tj = act ? tc[j] : 0.0, w0 = 0.0, w1 = 0.0;
+            int r = j + 1 + gl;
+            if (act) {
+#pragma unroll 2
+                for (; r + 8 < K; r += 16) {
+                    w0 = fma(hv[r], tc[r], w0);
+                    w1 = fma(hv[r + 8], tc[r + 8], w1);
                 }
-                s2 = group_sum<32>(s2);
-                if (lane == 0) sigl[q] = s2;
+                if (r < K) w0 = fma(hv[r], tc[r], w0);
             }
-            if (lane == 0) {
-                X[(size_t)j * K + c] = rj;       // row j of R: zero at the earlier pivots
-                if (c == pc) sigl[q] = -1.0;
+            double w = group_sum<8>(w0 + w1);
+            w = fma(alpha - beta, tj, w) * th;
+            double s0 = 0.0, s1 = 0.0;
+            r = j + 1 + gl;
+            if (act) {
+#pragma unroll 2
+                for (; r + 8 < K; r += 16) {
+                    const double x0 = fma(-w, hv[r], tc[r]), x1 = fma(-w, hv[r + 8], tc[r + 8]);
+                    tc[r] = x0;
+                    tc[r + 8] = x1;
+                    s0 = fma(x0, x0, s0);
+                    s1 = fma(x1, x1, s1);
+                }
+                if (r < K) {
+                    const double x0 = fma(-w, hv[r], tc[r]);
+                    tc[r] = x0;
+                    s0 = fma(x0, x0, s0);
+                }
+            }
+            const double s2 = group_sum<8>(s0 + s1);
+            __syncwarp();
+            if (gl == 0 && q < nc) {
+                // row j of R: beta at the pivot, zero at the earlier pivots
+                X[(size_t)j * K + c] = c == pc ? beta : (act ? fma(-w, alpha - beta, tj) : 0.0);
+                sigl[q] = act ? s2 : -1.0;
             }
         }
         __syncthreads();
@@ -647,6 +744,7 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
 
     // 3. block Jacobi on the columns of X
     double *G = sm, *Jm = G + WP * WLD, *red = Jm + WP * WLD;   // the QR's shared memory is free
+    const int gblk[1] = {tri_block(min(tid, WP / 2 * (WP / 2 + 1) / 2 - 1))};      // this thread's block of G
     const double tolj = 4.4e-16 * (double)(K > 16 ? K : 16), tol2 = tolj * tolj;
     int sweeps = 0;
     while (k > 1 && sweeps < MAX_SWEEPS) {
@@ -685,8 +783,7 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
                     for (int w = 0; w < W_NW; ++w) v += red[w * W_TILES * 64 + idx];
                     const int q = idx >> 6, I = q >= 6 ? 3 : q >= 3 ? 2 : q >= 1 ? 1 : 0, J = q - I * (I + 1) / 2;
                     const int i = 8 * I + ((idx & 63) >> 3), jj = 8 * J + (idx & 7);
-                    G[i * WLD + jj] = v;
-                    G[jj * WLD + i] = v;
+                    if (jj <= i) G[i * WGD + jj] = v;
                 }
                 for (int idx = tid; idx < WP * WP; idx += W_CT)
                     Jm[(idx >> 5) * WLD + (idx & 31)] = (idx >> 5) == (idx & 31) ? 1.0 : 0.0;
@@ -695,33 +792,41 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
                 for (int idx = tid; idx < WP * WP; idx += W_CT) {
                     const int i = idx >> 5, jj = idx & 31;
                     if (jj < i) {
-                        double va = G[i * WLD + i], vb = G[jj * WLD + jj], vc = G[i * WLD + jj];
+                        double va = G[i * WGD + i], vb = G[jj * WGD + jj], vc = G[i * WGD + jj];
                         need |= pair_scaled(va, vb, vc, tau2, tol2);
                     }
                 }
                 if (!__syncthreads_or(need)) continue;
                 if (tid == 0) atomicExch(rotf + sweeps, 1);
-                for (int rr = 0; rr < WP - 1; ++rr) {
-                    if (tid < WP / 2) {
-                        const int a = tourney(tid, rr, WP), b = tourney(WP - 1 - tid, rr, WP);
-                        double cs, sn;
-                        pair_rotation(G[a * WLD + a], G[b * WLD + b], G[a * WLD + b], tau2, tol2, cs, sn);
-                        rot[tid] = make_double2(cs, sn);
-                        pab[tid] = a | (b << 16);
-                    }
+                // rotations: every pair in the sweep's first round (each block is in one
+                // problem then; with an odd number of blocks the one left out is in the
+                // second round's), the pairs across the two blocks in the others; warp 0
+                // finds the next round's while the other warps rotate J
+                const bool full = round == 0 || (round == 1 && (nblk & 1));
+                const int nr = full ? WP - 1 : WB;
+                auto angles = [&](int rr) {
+                    if (tid >= WP / 2) return;
+                    const int a = full ? tourney(tid, rr, WP) : tid;
+                    const int b = full ? tourney(WP - 1 - tid, rr, WP) : WB + ((tid + rr) & (WB - 1));
+                    rot[rr & 1][tid] = pair_rotation(G[a * WGD + a], G[b * WGD + b], G[low(a, b, WGD)], tau2, tol2);
+                    pab[rr & 1][tid] = a | (b << 16);
+                };
+                angles(0);
+                __syncthreads();
+                for (int rr = 0; rr < nr; ++rr) {
+                    const double2 *rt = rot[rr & 1];
+                    const int *pp = pab[rr & 1];
+                    if (tid < WP / 2 * (WP / 2 + 1) / 2) rotate_blocks<1>(G, WGD, gblk, rt, pp);
                     __syncthreads();
-                    const int I = tid & 15, r0 = tid >> 4;
-                    const double2 ri = rot[I], rj = rot[r0];
-                    const int a = pab[I] & 0xffff, b = pab[I] >> 16;
-                    if (ri.y != 0.0 || rj.y != 0.0)
-                        rotate_block(G, WLD, pab[r0] & 0xffff, pab[r0] >> 16, rj.x, rj.y, a, b, ri.x, ri.y, I == r0);
-                    if (ri.y != 0.0) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            double *jr = Jm + (r0 + 16 * h) * WLD;
-                            const double xa = jr[a], xb = jr[b];
-                            jr[a] = ri.x * xa - ri.y * xb;
-                            jr[b] = ri.y * xa + ri.x * xb;
+                    if (warp == 0) {
+                        if (rr + 1 < nr) angles(rr + 1);
+                    } else {
+                        const double2 r = rt[tid & 15];
+                        // seven warps, two rows a warp: rows 0..27, then 28..31
+                        const int c = 2 * (warp - 1) + (lane >> 4);
+                        if (r.y != 0.0) {
+                            rotate_rows<2>(Jm, WLD, pp[tid & 15], r, c, 2 * (W_NW - 1));
+                            if (c < WP - 4 * (W_NW - 1)) rotate_rows<1>(Jm, WLD, pp[tid & 15], r, c + 4 * (W_NW - 1), 1);
                         }
                     }
                     __syncthreads();
@@ -832,25 +937,29 @@ int wide_cluster(int K) { return K <= 160 ? 4 : K <= 448 ? 8 : W_CSMAX; }
 
 }  // namespace
 
-int core_smem_kmax() { return SMALL_KMAX; }
+// One CTA beats a cluster at any width when the launch fills the device, but its
+// latency grows with K (K = 80: 0.79 ms against 0.5 ms on four CTAs): cores of
+// 65 to SMALL_KMAX columns take either kernel, so they bring scratch.
+int core_smem_kmax() { return 64; }
 
 size_t core_work_doubles(int K) { return (size_t)K * (K + WP) + (size_t)K * (K + W_CSMAX) + (size_t)K + 64; }
 
-int core_bucket(int K) {
+int core_bucket(int K, bool cluster) {
     if (K <= 64) return K <= 16 ? 16 : K <= 32 ? 32 : K <= 48 ? 48 : 64;
-    if (K <= SMALL_KMAX) return K <= 80 ? 80 : 96;
+    if (K <= SMALL_KMAX && !cluster) return K <= 80 ? 80 : SMALL_KMAX;
     return K <= 160 ? 160 : K <= 448 ? 448 : 1 << 30;
 }
+int core_one_cta_kmax() { return SMALL_KMAX; }
 
-void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p,
+void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p, bool cluster,
                              cudaStream_t st) {
     if (ntasks <= 0) return;
     if (kmax <= 16) return launch_small<16>(d_tasks, ntasks, p, st);
     if (kmax <= 32) return launch_small<32>(d_tasks, ntasks, p, st);
     if (kmax <= 48) return launch_small<48>(d_tasks, ntasks, p, st);
     if (kmax <= 64) return launch_small<64>(d_tasks, ntasks, p, st);
-    if (kmax <= 80) return launch_small<80>(d_tasks, ntasks, p, st);
-    if (kmax <= SMALL_KMAX) return launch_small<96>(d_tasks, ntasks, p, st);
+    if (kmax <= 80 && !cluster) return launch_small<80>(d_tasks, ntasks, p, st);
+    if (kmax <= SMALL_KMAX && !cluster) return launch_small<96>(d_tasks, ntasks, p, st);
     int cs = wide_cluster(kmax);
     for (;;) {
     // T in the cluster's shared memory where a CTA's share fits

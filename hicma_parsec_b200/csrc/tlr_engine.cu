@@ -595,14 +595,14 @@ int run_qapply(hicma_tlr_ctx *c, std::vector<QApplyTask> &v, int m_max) {
     return check_launch(c);
 }
 
-int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CoreParams &cp) {
+int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CoreParams &cp, bool cluster) {
     if (v.empty()) return 0;
     TRY(bc_cores(v));
     CoreTask *d = stage(c, v.data(), v.size());
     if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
     {
         Prof pf(c, P_CORE, 0, 0);
-        launch_core_svd_batched(d, (int)v.size(), std::max(kmax, 1), cp, c->cur);
+        launch_core_svd_batched(d, (int)v.size(), std::max(kmax, 1), cp, cluster, c->cur);
     }
     v.clear();
     return check_launch(c);
@@ -967,26 +967,31 @@ size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
 // Core-SVD launches bucketed by K, so that small cores run several CTAs per SM.
 // Buckets of the one-CTA kernel are merged upwards while the merged launch has
 // no more tasks than SMs: it is then one CTA per SM either way, and a launch
-// lasts as long as its slowest core.
+// lasts as long as its slowest core.  Cores of 65 to 96 columns run on clusters of
+// four CTAs, with the wider ones, while those clusters fit the device at once.
 int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreParams &cp) {
+    int mid = 0;
+    for (auto &t : cores) mid += t.K > core_smem_kmax() && t.K <= core_one_cta_kmax();
+    const bool cluster = 4 * mid <= c->nsm;
+    auto bucket_of = [&](const CoreTask &t) { return core_bucket(t.K, cluster); };
     std::stable_sort(cores.begin(), cores.end(),
-                     [](const CoreTask &a, const CoreTask &b) { return core_bucket(a.K) < core_bucket(b.K); });
+                     [&](const CoreTask &a, const CoreTask &b) { return bucket_of(a) < bucket_of(b); });
     size_t i = 0;
     while (i < cores.size()) {
         size_t e = i;
-        int b = core_bucket(cores[i].K);
-        while (e < cores.size() && core_bucket(cores[e].K) == b) ++e;
-        while (e < cores.size() && core_bucket(cores[e].K) <= core_smem_kmax()) {
-            const int nb = core_bucket(cores[e].K);
+        const int b = bucket_of(cores[i]);
+        while (e < cores.size() && bucket_of(cores[e]) == b) ++e;
+        while (e < cores.size() && bucket_of(cores[e]) <= core_one_cta_kmax()) {
+            const int nb = bucket_of(cores[e]);
             size_t f = e;
-            while (f < cores.size() && core_bucket(cores[f].K) == nb) ++f;
+            while (f < cores.size() && bucket_of(cores[f]) == nb) ++f;
             if (f - i > (size_t)c->nsm) break;
             e = f;
         }
         std::vector<CoreTask> bucket(cores.begin() + (long)i, cores.begin() + (long)e);
         int kmax = 0;
         for (auto &t : bucket) kmax = std::max(kmax, t.K);
-        TRY(run_core(c, bucket, kmax, cp));
+        TRY(run_core(c, bucket, kmax, cp, cluster));
         i = e;
     }
     cores.clear();

@@ -300,13 +300,17 @@ struct CoreParams {
     int *overflow;       // device counter of capped recompressions
     int *sweeps;         // device counter of Jacobi sweeps (diagnostics, may be null)
 };
+// Cores up to this K need no scratch in global memory.
 int core_smem_kmax();
 // Global scratch (doubles) of one core with K > core_smem_kmax().
 size_t core_work_doubles(int K);
 // Launch bucket of a core (the widest K of its kernel instance or cluster size).
-int core_bucket(int K);
+// Cores between core_smem_kmax() and core_one_cta_kmax() run on a cluster of
+// CTAs each if `cluster` is set, else on one CTA.
+int core_bucket(int K, bool cluster);
+int core_one_cta_kmax();
 // All tasks of one launch have K <= kmax; kernel and shared memory are chosen from kmax.
-void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p,
+void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p, bool cluster,
                              cudaStream_t st);
 
 // ---------------------------------------------------------------- misc ------
