@@ -2,30 +2,37 @@
 //
 // Replaces HCORE_dpotrf on a diagonal tile (hicma_parsec/HiCMA_dpotrf_L_2flow.jdf
 // :233-242) together with the inverse L^-1 that the panel solves of this
-// engine apply as a GEMM.  The tile is split into 64 x 64 blocks and the
-// blocked right-looking algorithm becomes a list of block tasks:
+// engine apply as a GEMM.  The tile is split into 64 x 64 blocks, and a blocked
+// left-looking algorithm becomes a list of tasks:
 //   CHAIN        the critical path, run by one CTA from start to end: for each
 //                block column j, Cholesky of A_jj and D_j = L_jj^-1, then
-//                L_j+1,j = A_j+1,j D_j^T and A_j+1,j+1 -= L_j+1,j L_j+1,j^T,
+//                L_j+1,j = S_j+1,j D_j^T and S_j+1,j+1 -= L_j+1,j L_j+1,j^T,
 //                the next diagonal block staying in shared memory
-//   PANEL(j,i)   L_ij = A_ij D_j^T                        (i >= j + 2)
-//   UPD(j,i,k)   A_ik -= L_ij L_kj^T         (j < k <= i, (i,k) != (j+1,j+1))
-//   XDIAG(j,k)   X_jk = D_j B_jk                           (k < j)
-//   XUPD(j,i,k)  B_ik -= L_ij X_jk                         (k <= j < i)
-// where X = L^-1 is produced by block forward substitution on the identity
-// (B starts as zero off the diagonal).  The chain is the first task; the rest
-// of the list is in a topological order and CTAs take tasks from it with an
-// atomic ticket, so every task waits only on the chain or on tasks already
-// held by running CTAs, and the chain waits only on tasks of earlier block
-// columns, which the other CTAs take in list order: the kernel makes progress
-// with two or more CTAs, whether or not they are resident together, and needs
-// no cooperative launch.  Dependencies are per-block counters released
-// with a fence after the block is written and acquired by one thread before
-// the CTA reads (through L2: ld.global.cg).  Every wait is bounded; a wait
+//   PRE(k)       S_k+1,{k,k+1} = A_k+1,{k,k+1} - sum_{j<k} L_k+1,j L_{k,k+1},j^T
+//   LT(i,k)      L_{i,i+1},k = (A_{i,i+1},k - sum_{j<k} L_{i,i+1},j L_kj^T) D_k^T
+//                                                               (i >= k + 2)
+//   XT(i,p)      X_i,{2p,2p+1} = -D_i sum_{2p<=j<i} L_ij X_j,{2p,2p+1}
+// where X = L^-1 is produced by block forward substitution.  A task keeps its
+// 128 x 64 or 64 x 128 tile in the accumulators over all of its sum, reading
+// each block once as it becomes final, so that the tile is read and written
+// once and the waits overlap the products of the blocks before them.  The chain
+// is the first task; the rest of the list is in a topological order and CTAs
+// take tasks from it with an atomic ticket, so every task waits only on the
+// chain or on tasks already held by running CTAs, and the chain waits only on
+// tasks of earlier block columns, which the other CTAs take in list order: the
+// kernel makes progress with two or more CTAs, whether or not they are resident
+// together, and needs no cooperative launch.  Dependencies are per-block flags
+// released with a fence after the block is written and acquired by one thread
+// before the CTA reads (through L2: ld.global.cg).  Every wait is bounded; a wait
 // that gives up sets the timeout flag and the abort flag, and every CTA leaves
-// at its next task.  A non-positive pivot sets the reference's INFO
+// at its next wait or task.  A non-positive pivot sets the reference's INFO
 // (k*NB + iinfo) and aborts the same way.  The block products run on the FP64
 // tensor cores (mma.sync m8n8k4 f64).
+// Bound by the chain (43 steps of about 24 us for a tile of 2700) when one CTA runs
+// on every SM, by the DMMA rate of its CTAs below about 100.  Against one task per
+// 64 x 64 x 64 block product (right-looking, C read and written for each of them, 20k
+// cycles a product of which DMMA 4.1k): tile of 2700 with its inverse 2.00 -> 1.13 ms
+// on 148 CTAs, 4.1 -> 1.67 ms on 64, 7.8 -> 3.05 ms on 32; tile of 1350 0.64 -> 0.54 ms.
 #include "tlr_internal.h"
 
 #include <map>
@@ -36,14 +43,14 @@ namespace tlr {
 namespace {
 
 constexpr int TB = 64;          // block edge
-constexpr int TPITCH = 72;      // shared pitch of DMMA operand tiles
 constexpr int CP = TB + 4;      // shared pitch of the chain CTA's blocks (conflict-free DMMA fragments)
 constexpr int NTH = 256;
+constexpr int XLAG = 6;         // block columns by which the inverse's rows follow the factor's (0: 6 % slower, 2: 3 %)
 constexpr long long SPIN_LIMIT = 1LL << 24;
 
-enum { IT_CHAIN = 0, IT_PANEL, IT_UPD, IT_XDIAG, IT_XUPD };
+enum { IT_CHAIN = 0, IT_PRE, IT_LT, IT_XT };
 struct PItem {
-    unsigned short type, j, i, k;
+    unsigned short type, i, k, pad;   // k: block column, or column pair of XT
 };
 
 struct PotrfParams {
@@ -54,10 +61,11 @@ struct PotrfParams {
     double *D;          // nblk x (64 x 64) block inverses when X is null
     const PItem *items;
     int nitems;
-    int *cnt;           // [0] ticket [1] abort, then ver, pdone, xver, xdone (nblk^2 each), ddone (nblk)
+    int *cnt;           // [0] ticket [1] abort, then pdone, xdone (nblk^2 each), ddone, vpre (nblk each)
     int *info;
     int info_base;
     int *timeout;
+    int v16;                // A and X are 16-byte aligned, with even leading dimensions
     long long spin_limit;   // polls before a wait gives up (SPIN_LIMIT in production)
 };
 
@@ -86,84 +94,365 @@ __device__ bool wait_ge(const int *p, int v, const PotrfParams &P) {
 
 __device__ __forceinline__ int bsz(int b, int n) { return min(TB, n - b * TB); }
 
-// C (m x nn, ldc) = beta C + alpha opA(A) opB(B), inner dimension kk <= 64.
-// Operands are staged in shared memory before C is written, so C may alias
-// A or B when beta = 0 (with beta != 0, C is read before the products and
-// must not alias them).  The operand loads go out in two rounds of 16 per
-// thread, and C's entries are fetched ahead of the products.
-__device__ void blk_gemm(double *sm, double *C, int ldc, int m, int nn, int kk, double alpha, double beta,
-                         const double *A, int lda, int opA, const double *B, int ldb, int opB) {
-    double *As = sm;                 // As[k][i]
-    double *Bs = sm + TB * TPITCH;   // Bs[k][j]
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, tig = lane & 3;
-    const int wm = warp & 1, wn = warp >> 1;   // 2 x 4 warps, 32 x 16 each
-    constexpr int HALF = (TB * TB) / NTH / 2;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        double va[HALF], vb[HALF];
-#pragma unroll
-        for (int q = 0; q < HALF; ++q) {
-            const int e = tid + (h * HALF + q) * NTH;
-            int i, k;
-            if (opA == 0) { i = e & (TB - 1); k = e >> 6; } else { k = e & (TB - 1); i = e >> 6; }
-            va[q] = (i < m && k < kk) ? __ldcg(opA == 0 ? A + i + (size_t)k * lda : A + k + (size_t)i * lda) : 0.0;
-            int j;
-            if (opB == 0) { k = e & (TB - 1); j = e >> 6; } else { j = e & (TB - 1); k = e >> 6; }
-            vb[q] = (j < nn && k < kk) ? __ldcg(opB == 0 ? B + k + (size_t)j * ldb : B + j + (size_t)k * ldb) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < HALF; ++q) {
-            const int e = tid + (h * HALF + q) * NTH;
-            int i, k, j;
-            if (opA == 0) { i = e & (TB - 1); k = e >> 6; } else { k = e & (TB - 1); i = e >> 6; }
-            As[k * TPITCH + i] = va[q];
-            if (opB == 0) { k = e & (TB - 1); j = e >> 6; } else { j = e & (TB - 1); k = e >> 6; }
-            Bs[k * TPITCH + j] = vb[q];
-        }
+// Flags of the task queue.
+struct PFlags {
+    int *pdone, *xdone, *ddone, *vpre;
+    int nb;
+    __device__ PFlags(const PotrfParams &P) : nb(P.nblk) {
+        pdone = P.cnt + 8;
+        xdone = pdone + nb * nb;
+        ddone = xdone + nb * nb;
+        vpre = ddone + nb;
     }
-    double cv[4][2][2];
+    __device__ int *p(int i, int j) const { return pdone + i * nb + j; }   // L_ij is final
+    __device__ int *x(int i, int q) const { return xdone + i * nb + q; }   // X_i,{2q,2q+1} is final
+};
+
+// ------------------------------------------------------------ bulk tasks ----
+// Inner step: 32 with cp.async (fewer barriers, against which one CTA per SM has
+// nothing to run), 16 where the next step waits in registers.
+template <bool V16>
+__host__ __device__ constexpr int pk() { return V16 ? 32 : 16; }
+
+// Flags (at most three) that release inner block j of a task.
+struct JDeps {
+    const int *a, *b, *c;
+};
+__device__ __forceinline__ bool deps_ready(const JDeps &d) {
+    const int r = ld_volatile(d.a) & ld_volatile(d.b) & ld_volatile(d.c);
+    if (r) __threadfence();
+    return r;
+}
+__device__ bool deps_wait(const JDeps &d, const PotrfParams &P) {
+    for (long long it = 0; it < P.spin_limit; ++it) {
+        if (deps_ready(d)) return true;
+        if (ld_volatile(P.cnt + 1)) return false;
+        __nanosleep(it < 256 ? 32 : 256);
+    }
+    atomicExch(P.timeout, 1);
+    atomicExch(P.cnt + 1, 1);
+    return false;
+}
+
+// Warp-wide: how many of the inner blocks j, j + 1, ... below j1 are released (up
+// to 32 looked at, so that a task with a backlog polls once for many blocks).
+template <class Deps>
+__device__ __forceinline__ int deps_count(int j, int j1, int lane, Deps deps) {
+    bool r = false;
+    if (j + lane < j1) {
+        const JDeps d = deps(j + lane);
+        r = ld_volatile(d.a) & ld_volatile(d.b) & ld_volatile(d.c);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, r);
+    if (m & 1u) __threadfence();
+    return m == 0xffffffffu ? 32 : __ffs(~m) - 1;
+}
+
+// bytes (16, 8 or 0) from gmem through L2, the rest of the 16 zero-filled
+__device__ __forceinline__ void cp_async16(unsigned smem, const double *gmem, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(bytes));
+}
+// acc += A B over the inner blocks j0 <= j < j1 (64 each) for an MT x NL tile:
+// A (rows x inner, mrows of them valid) column-major; B by op: BKC = false: B^T
+// is stored (rows, column-major, nrows valid), true: B is stored (columns,
+// contiguous along the inner dimension, nrows valid).  Eight warps of 32 x 32.
+// Two shared stages: V16 (bases and leading dimensions 16-byte aligned) filled by
+// cp.async through L2, otherwise with the next step's operands in registers
+// (8-byte cp.async would go through L1, which may hold a neighbouring block's older
+// rows).  The flags of a block are looked at when its first
+// step comes up for loading, and waited for only when the products have caught up.
+// Each block's 64-term sum is formed on its own before it is added: one running sum
+// over up to 2700 terms rounds 2.3 times as far off (tile of 2700, 7.9e-14 against
+// 3.4e-14).  A step's loads are issued in parts between its products: as one burst after the
+// barrier they held up the fragment reads behind them (12.7k cycles a 128 x 64 x 64
+// block against 8.2k of DMMA).  Returns false if a wait gave up or the run was
+// aborted.
+template <int MT, int NL, bool BKC, bool V16, class Deps>
+__device__ bool acc_blocks(double *sm, double (&acc)[4][4][2], const PotrfParams &P, const double *A, int lda,
+                           int mrows, const double *B, int ldb, int nrows, int j0, int j1, Deps deps) {
+    constexpr int PK = pk<V16>(), PA = MT + 4, PB = BKC ? PK + 4 : NL + 4;
+    constexpr int SA = PK * PA, SB = BKC ? NL * PB : PK * PB;
+    constexpr int ST = 2, SPB = TB / PK;
+    constexpr int W = V16 ? 2 : 1, QA = MT * PK / W / NTH, QB = NL * PK / W / NTH;
+    __shared__ int poll_sh[2], wait_sh;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tig = lane & 3, wm = warp % (MT / 32), wn = warp / (MT / 32);
+    if (j0 >= j1) return true;
+    const int S = (j1 - j0) * SPB;
+    double blk[4][4][2];                  // this block's sum
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
+        for (int ni = 0; ni < 4; ++ni) blk[mi][ni][0] = blk[mi][ni][1] = 0.0;
+    double ra[V16 ? 1 : QA], rb[V16 ? 1 : QB];
+    const unsigned s0 = (unsigned)__cvta_generic_to_shared(sm);
+    // part t of NP of step s's operands
+    constexpr int NP = PK / 4;
+    auto load_part = [&](int s, int t) {
+        const int kb = j0 * TB + s * PK;
+        const unsigned st = s0 + (unsigned)((s % ST) * (SA + SB) * sizeof(double));
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int row = wm * 32 + mi * 8 + g, col = wn * 16 + ni * 8 + 2 * tig + e;
-                cv[mi][ni][e] = (beta != 0.0 && row < m && col < nn) ? __ldcg(C + row + (size_t)col * ldc) : 0.0;
+        for (int q = 0; q < QA; ++q) {
+            if (q < t * QA / NP || q >= (t + 1) * QA / NP) continue;
+            const int e = tid + q * NTH, x = (e % (MT / W)) * W, kk = e / (MT / W);
+            const double *src = A + x + (size_t)(kb + kk) * lda;
+            if constexpr (V16) cp_async16(st + (unsigned)((kk * PA + x) * sizeof(double)), x < mrows ? src : A,
+                                          x + 1 < mrows ? 16 : x < mrows ? 8 : 0);
+            else ra[q] = x < mrows ? __ldcg(src) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < QB; ++q) {
+            if (q < t * QB / NP || q >= (t + 1) * QB / NP) continue;
+            const int e = tid + q * NTH;
+            if (BKC) {
+                const int kk = (e % (PK / W)) * W, x = e / (PK / W);
+                const double *src = B + kb + kk + (size_t)x * ldb;
+                if constexpr (V16) cp_async16(st + (unsigned)((SA + x * PB + kk) * sizeof(double)), x < nrows ? src : B,
+                                              x < nrows ? 16 : 0);
+                else rb[q] = x < nrows ? __ldcg(src) : 0.0;
+            } else {
+                const int x = (e % (NL / W)) * W, kk = e / (NL / W);
+                const double *src = B + x + (size_t)(kb + kk) * ldb;
+                if constexpr (V16) cp_async16(st + (unsigned)((SA + kk * PB + x) * sizeof(double)), x < nrows ? src : B,
+                                              x + 1 < nrows ? 16 : x < nrows ? 8 : 0);
+                else rb[q] = x < nrows ? __ldcg(src) : 0.0;
             }
+        }
+    };
+    auto load = [&](int s) {
+#pragma unroll
+        for (int t = 0; t < NP; ++t) load_part(s, t);
+    };
+    if (tid == 0) wait_sh = deps_wait(deps(j0), P);
     __syncthreads();
-    double acc[4][2][2];
+    if (!wait_sh) return false;
+    int issued = 0, ready = j0 + 1;       // steps loaded or on their way; blocks known to be released
+    load(issued++);
+    for (int s = 0; s < S; ++s) {
+        double *As = sm + (s % ST) * (SA + SB), *Bs = As + SA;
+        if constexpr (V16) {
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+        } else {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+            for (int q = 0; q < QA; ++q) {
+                const int e = tid + q * NTH;
+                As[(e / MT) * PA + e % MT] = ra[q];
+            }
 #pragma unroll
-        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    const int k4end = (kk + 3) & ~3;
-    for (int k4 = 0; k4 < k4end; k4 += 4) {
-        double a[4], b[2];
+            for (int q = 0; q < QB; ++q) {
+                const int e = tid + q * NTH;
+                if (BKC) Bs[(e / PK) * PB + e % PK] = rb[q];
+                else Bs[(e / NL) * PB + e % NL] = rb[q];
+            }
+        }
+        // the step to load now starts a block not known to be released: look again
+        const int jn = j0 + issued / SPB;
+        const bool look = issued < S && jn >= ready;
+        if (look && warp == 0) {
+            const int n = deps_count(jn, j1, lane, deps);
+            if (lane == 0) poll_sh[s & 1] = jn + n;
+        }
+        __syncthreads();                  // step s is in shared memory, step s - 1 has been read
+        if (look) ready = poll_sh[s & 1];
+        const bool now = issued < S && jn < ready;
+        const double *pa = As + tig * PA + wm * 32 + g;
+        const double *pb = BKC ? Bs + (wn * 32 + g) * PB + tig : Bs + tig * PB + wn * 32 + g;
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi) a[mi] = As[(k4 + tig) * TPITCH + wm * 32 + mi * 8 + g];
+        for (int k4 = 0; k4 < PK; k4 += 4) {
+            double a[4], b[4];
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni) b[ni] = Bs[(k4 + tig) * TPITCH + wn * 16 + ni * 8 + g];
+            for (int mi = 0; mi < 4; ++mi) a[mi] = pa[k4 * PA + 8 * mi];
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni) b[ni] = BKC ? pb[8 * ni * PB + k4] : pb[k4 * PB + 8 * ni];
+            if (now) load_part(issued, k4 / 4);
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni) dmma884(blk[mi][ni], a[mi], b[ni]);
+        }
+        if (s % SPB == SPB - 1) {
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        acc[mi][ni][e] += blk[mi][ni][e];
+                        blk[mi][ni][e] = 0.0;
+                    }
+        }
+        if (now) ++issued;
+        if (s + 1 < S && issued == s + 1) {
+            if (tid == 0) wait_sh = deps_wait(deps(jn), P);
+            __syncthreads();
+            if (!wait_sh) return false;
+            ready = jn + 1;
+            load(issued++);
+        }
+    }
+    return true;
+}
+
+// One bulk task; false if a wait gave up or the run was aborted.
+// Not inlined, as the chain, so that each has the registers to itself.
+template <bool V16>
+__device__ __noinline__ bool run_bulk(double *sm, const PItem it, const PotrfParams &P) {
+    __shared__ int d_sh;
+    const PFlags F(P);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tig = lane & 3;
+    const int n = P.n, lda = P.lda, nb = P.nblk, i = it.i, k = it.k;
+    auto Aij = [&](int r, int c) { return P.A + (size_t)r * TB + (size_t)c * TB * lda; };
+    double acc[4][4][2];
+    const bool lt = it.type == IT_LT;
+    const int WMN = lt ? 4 : 2;               // warps down the tile
+    const int wm = warp % WMN, wn = warp / WMN;
+    auto row_of = [&](int mi) { return wm * 32 + 8 * mi + g; };
+    auto col_of = [&](int ni, int e) { return wn * 32 + 8 * ni + 2 * tig + e; };
+    if (it.type == IT_XT) {
+        const int c0 = 2 * k;                 // first block column of the pair
 #pragma unroll
         for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-            for (int ni = 0; ni < 2; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
+            for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        const int mrows = bsz(i, n), ncols = min(2 * TB, i * TB - c0 * TB);   // columns left of the diagonal block
+        auto deps = [&](int j) {
+            return JDeps{F.p(i, j), j == c0 ? F.ddone + j : F.x(j, k), j <= c0 + 1 ? F.ddone + j : F.p(i, j)};
+        };
+        if (!acc_blocks<TB, 2 * TB, true, V16>(sm, acc, P, Aij(i, 0), lda, mrows, P.X + (size_t)c0 * TB * P.ldx, P.ldx, ncols,
+                                          c0, i, deps))
+            return false;
+        // X = -D_i acc
+        double *Ds = sm, *Ss = sm + TB * (TB + 4);
+        if (tid == 0) d_sh = wait_ge(F.ddone + i, 1, P);
+        __syncthreads();
+        if (!d_sh) return false;
+        const double *D = P.X + (size_t)i * TB + (size_t)i * TB * P.ldx;
+#pragma unroll
+        for (int q = 0; q < TB * TB / NTH; ++q) {
+            const int e = tid + q * NTH, x = e % TB, kk = e / TB;
+            Ds[kk * (TB + 4) + x] = x < mrows && kk < mrows ? __ldcg(D + x + (size_t)kk * P.ldx) : 0.0;
+        }
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    Ss[col_of(ni, e) * (TB + 4) + row_of(mi)] = -acc[mi][ni][e];
+                    acc[mi][ni][e] = 0.0;
+                }
+        __syncthreads();
+        const int ke = wm * 32 + 32;          // D_i is lower triangular
+        for (int k4 = 0; k4 < ke; k4 += 4) {
+            double a[4], b[4];
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi) a[mi] = Ds[(k4 + tig) * (TB + 4) + row_of(mi)];
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni) b[ni] = Ss[(wn * 32 + 8 * ni + g) * (TB + 4) + k4 + tig];
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
+        }
+        double *O = P.X + (size_t)i * TB + (size_t)c0 * TB * P.ldx;
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if (row_of(mi) < mrows && col_of(ni, e) < ncols)
+                        O[row_of(mi) + (size_t)col_of(ni, e) * P.ldx] = acc[mi][ni][e];
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicExch(F.x(i, k), 1);
+        }
+        return true;
+    }
+    // rows of the tile: blocks i, i + 1 (LT) or block k + 1 (PRE); columns: block k (LT) or k, k + 1 (PRE)
+    const int r0 = lt ? i : k + 1;
+    const int mrows = min(lt ? 2 * TB : TB, n - r0 * TB), ncols = lt ? TB : min(2 * TB, n - k * TB);
+    double *C = Aij(r0, k);
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                acc[mi][ni][e] = row_of(mi) < mrows && col_of(ni, e) < ncols
+                                     ? -__ldcg(C + row_of(mi) + (size_t)col_of(ni, e) * lda) : 0.0;   // acc = sum - C
+    if (!lt) {
+        auto deps = [&](int j) { return JDeps{F.p(k + 1, j), F.p(k, j), F.p(k, j)}; };
+        if (!acc_blocks<TB, 2 * TB, false, V16>(sm, acc, P, Aij(k + 1, 0), lda, mrows, Aij(k, 0), lda, ncols, 0, k, deps))
+            return false;
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if (row_of(mi) < mrows && col_of(ni, e) < ncols)
+                        C[row_of(mi) + (size_t)col_of(ni, e) * lda] = -acc[mi][ni][e];
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicExch(F.vpre + k, 1);
+        }
+        return true;
+    }
+    const bool two = i + 1 < nb;
+    auto deps = [&](int j) { return JDeps{F.p(i, j), F.p(two ? i + 1 : i, j), F.p(k, j)}; };
+    if (!acc_blocks<2 * TB, TB, false, V16>(sm, acc, P, Aij(i, 0), lda, mrows, Aij(k, 0), lda, TB, 0, k, deps)) return false;
+    // L = -acc D_k^T
+    double *Ss = sm, *Ds = sm + TB * (2 * TB + 4);
+    if (tid == 0) d_sh = wait_ge(F.ddone + k, 1, P);
+    __syncthreads();
+    if (!d_sh) return false;
+    const double *D = P.X ? P.X + (size_t)k * TB + (size_t)k * TB * P.ldx : P.D + (size_t)k * TB * TB;
+    const int ldd = P.X ? P.ldx : TB;
+#pragma unroll
+    for (int q = 0; q < TB * TB / NTH; ++q) {
+        const int e = tid + q * NTH, x = e % TB, kk = e / TB;
+        Ds[kk * (TB + 4) + x] = __ldcg(D + x + (size_t)kk * ldd);
     }
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi) {
-        const int row = wm * 32 + mi * 8 + g;
-        if (row >= m) continue;
+    for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
+        for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int col = wn * 16 + ni * 8 + 2 * tig + e;
-                if (col >= nn) continue;
-                C[row + (size_t)col * ldc] = alpha * acc[mi][ni][e] + beta * cv[mi][ni][e];
+                Ss[col_of(ni, e) * (2 * TB + 4) + row_of(mi)] = -acc[mi][ni][e];
+                acc[mi][ni][e] = 0.0;
             }
+    __syncthreads();
+    const int ke = wn * 32 + 32;              // D_k^T is upper triangular
+    for (int k4 = 0; k4 < ke; k4 += 4) {
+        double a[4], b[4];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) a[mi] = Ss[(k4 + tig) * (2 * TB + 4) + row_of(mi)];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) b[ni] = Ds[(k4 + tig) * (TB + 4) + wn * 32 + 8 * ni + g];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
     }
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (row_of(mi) < mrows) C[row_of(mi) + (size_t)col_of(ni, e) * lda] = acc[mi][ni][e];
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        atomicExch(F.p(i, k), 1);
+        if (two) atomicExch(F.p(i + 1, k), 1);
+    }
+    return true;
 }
 
 // ------------------------------------------------------------ the chain ----
@@ -173,6 +462,11 @@ __device__ void blk_gemm(double *sm, double *C, int ldc, int m, int nn, int kk, 
 // than 64 are padded: with the identity on the diagonal of S, with zeros in
 // Pn, so the padded parts factor to the identity and never reach the tile.
 constexpr int CHAIN_SMEM_DOUBLES = 3 * TB * CP;
+constexpr int SMEM_DOUBLES = 2 * (pk<true>() * (TB + 4) + 2 * TB * (pk<true>() + 4));   // two stages of an XT task
+static_assert(SMEM_DOUBLES >= CHAIN_SMEM_DOUBLES, "the chain's blocks");
+static_assert(SMEM_DOUBLES >= 2 * pk<true>() * (2 * TB + 4 + TB + 4), "two stages of an LT or PRE task");
+static_assert(SMEM_DOUBLES >= TB * (2 * TB + 4) + TB * (TB + 4), "S and D of an LT task");
+static_assert(SMEM_DOUBLES >= TB * (TB + 4) + 2 * TB * (TB + 4), "D and S of an XT task");
 
 // M(r, c) = G(r, c) for r < rows, c < cols, else (r == c && pad_id); all of a
 // thread's loads are issued before its shared stores.
@@ -259,18 +553,17 @@ __device__ int chain_panel(double *S, double *Xs, int p0, int warp, int lane) {
     return -1;
 }
 
-// Cholesky of S in place and its inverse in Xs (Pn is scratch).  Blocked by
+// Cholesky of S in place and its inverse in Xs (its blocks above the diagonal are
+// zero on entry and stay so; Pn is scratch).  Blocked by
 // 8-column panels (chain_panel, which also inverts the panel's diagonal
 // block), then every warp applies the panel's rank-8 update to the lower 8 x 8
 // tiles of the trailing block on the tensor cores.  The inverse's diagonal
 // blocks are then merged in pairs as X21 = -X22 (L21 X11) at widths 8, 16, 32.
 // Returns the column (0..63) of a non-positive pivot, or -1.
-__device__ int chain_diag(double *S, double *Xs, double *Pn) {
+__device__ int chain_diag(double *S, double *Xs, double *Pn, const int *flag, int *seen) {
     __shared__ int bad_sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    for (int e = tid; e < TB * CP; e += NTH) Xs[e] = 0.0;
-    __syncthreads();
     for (int p0 = 0; p0 < TB; p0 += 8) {
         if (warp < 3) {
             const int b = chain_panel(S, Xs, p0, warp, lane);
@@ -278,20 +571,37 @@ __device__ int chain_diag(double *S, double *Xs, double *Pn) {
         }
         __syncthreads();
         if (bad_sh >= 0) return bad_sh;
-        const int nbt = (TB - p0 - 8) / 8;   // trailing 8 x 8 block rows
-        for (int t = warp; t < nbt * (nbt + 1) / 2; t += NTH / 32) {
-            int bi = 0;
-            while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-            const int bj = t - bi * (bi + 1) / 2;
-            const int m0 = p0 + 8 + 8 * bi, n0 = p0 + 8 + 8 * bj;
-            double acc[2] = {S[(n0 + 2 * tig) * CP + m0 + g], S[(n0 + 2 * tig + 1) * CP + m0 + g]};
+        // rank-8 update of the trailing lower 8 x 8 tiles: warp w takes tile row w,
+        // its tiles independent of each other
+        if (8 * warp >= p0 + 8) {
+            const int m0 = 8 * warp;
+            double u[7][2];
+            const double a0 = -S[(p0 + tig) * CP + m0 + g], a1 = -S[(p0 + 4 + tig) * CP + m0 + g];
 #pragma unroll
-            for (int k = 0; k < 8; k += 4)
-                dmma884(acc, -S[(p0 + k + tig) * CP + m0 + g], S[(p0 + k + tig) * CP + n0 + g]);
-            S[(n0 + 2 * tig) * CP + m0 + g] = acc[0];
-            S[(n0 + 2 * tig + 1) * CP + m0 + g] = acc[1];
+            for (int c = 0; c < 7; ++c) {
+                const int n0 = p0 + 8 + 8 * c;
+                if (n0 <= m0) {
+                    u[c][0] = S[(n0 + 2 * tig) * CP + m0 + g];
+                    u[c][1] = S[(n0 + 2 * tig + 1) * CP + m0 + g];
+                    dmma884(u[c], a0, S[(p0 + tig) * CP + n0 + g]);
+                    dmma884(u[c], a1, S[(p0 + 4 + tig) * CP + n0 + g]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 7; ++c) {
+                const int n0 = p0 + 8 + 8 * c;
+                if (n0 <= m0) {
+                    S[(n0 + 2 * tig) * CP + m0 + g] = u[c][0];
+                    S[(n0 + 2 * tig + 1) * CP + m0 + g] = u[c][1];
+                }
+            }
         }
         __syncthreads();
+    }
+    if (tid == NTH - 1) {
+        const int v = ld_volatile(flag);
+        if (v) __threadfence();
+        *seen = v;
     }
     for (int h = 8; h < TB; h *= 2) {
         const int hb = h / 8, tpp = hb * hb, nt = (TB / (2 * h)) * tpp;
@@ -349,13 +659,13 @@ __device__ __forceinline__ void chain_mm_nt(double (&acc)[4][2][2], const double
 // (written, released as pdone(j+1, j)) and S = A_j+1,j+1 - L_j+1,j L_j+1,j^T,
 // each after the block's updates from the earlier columns are in.  Returns
 // false if a wait gave up or a pivot failed (the abort flag is then set).
-__device__ bool run_chain(double *sm, const PotrfParams &P) {
-    __shared__ int ok_c;
+__device__ __noinline__ bool run_chain(double *sm, const PotrfParams &P) {
+    __shared__ int ok_c, pre_c;
     double *S = sm, *Xs = sm + TB * CP, *Pn = sm + 2 * TB * CP;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tig = lane & 3, wm = warp & 1, wn = warp >> 1;
     const int nb = P.nblk, n = P.n, lda = P.lda;
-    int *ver = P.cnt + 8, *pdone = ver + nb * nb, *ddone = pdone + 3 * nb * nb;
+    const PFlags F(P);
     auto Ablk = [&](int r, int c) { return P.A + (size_t)r * TB + (size_t)c * TB * lda; };
     auto wait_all = [&](const int *p, int v) {
         if (tid == 0) ok_c = wait_ge(p, v, P);
@@ -363,10 +673,14 @@ __device__ bool run_chain(double *sm, const PotrfParams &P) {
         return ok_c != 0;
     };
     load_frame(S, Ablk(0, 0), lda, bsz(0, n), bsz(0, n), true);
+    for (int e = tid; e < TB * CP; e += NTH) Xs[e] = 0.0;
     __syncthreads();
+    constexpr int FR = (TB * TB) / NTH;
+    double fp[FR], fs[FR];                // the next panel and diagonal block, on their way
     for (int j = 0; j < nb; ++j) {
         const int jb = bsz(j, n);
-        const int bad = chain_diag(S, Xs, Pn);
+        // an idle thread looks for S_j+1,{j,j+1} while the diagonal block is factored
+        const int bad = chain_diag(S, Xs, Pn, F.vpre + j, &pre_c);
         if (bad >= 0) {
             if (tid == 0) {
                 // a pivot of the padding is 1: bad < jb
@@ -375,6 +689,17 @@ __device__ bool run_chain(double *sm, const PotrfParams &P) {
             }
             return false;
         }
+        const int i = j + 1, ib = i < nb ? bsz(i, n) : 0;
+        auto fetch = [&]() {
+#pragma unroll
+            for (int q = 0; q < FR; ++q) {
+                const int e = tid + q * NTH, r = e & (TB - 1), c = e >> 6;
+                fp[q] = r < ib ? __ldcg(Ablk(i, j) + r + (size_t)c * lda) : 0.0;
+                fs[q] = r < ib && c < ib ? __ldcg(Ablk(i, i) + r + (size_t)c * lda) : (r == c ? 1.0 : 0.0);
+            }
+        };
+        const bool early = i < nb && (j == 0 || pre_c);
+        if (early) fetch();               // they cross the write-out of L_jj and D_j
         double *Dj = P.X ? P.X + (size_t)j * TB + (size_t)j * TB * P.ldx : P.D + (size_t)j * TB * TB;
         const int ldd = P.X ? P.ldx : TB;
         double *Ajj = Ablk(j, j);
@@ -389,14 +714,20 @@ __device__ bool run_chain(double *sm, const PotrfParams &P) {
         __syncthreads();
         if (tid == 0) {
             __threadfence();
-            atomicExch(ddone + j, 1);
+            atomicExch(F.ddone + j, 1);
         }
-        const int i = j + 1;
         if (i >= nb) break;
-        const int ib = bsz(i, n);
         // L_ij = A_ij D_j^T (D_j^T upper: k stops at the warp's last column)
-        if (!wait_all(ver + i * nb + j, j)) return false;
-        load_frame(Pn, Ablk(i, j), lda, ib, TB, false);
+        if (!early) {
+            if (!wait_all(F.vpre + j, 1)) return false;
+            fetch();
+        }
+#pragma unroll
+        for (int q = 0; q < FR; ++q) {
+            const int e = tid + q * NTH;
+            Pn[(e >> 6) * CP + (e & (TB - 1))] = fp[q];
+            S[(e >> 6) * CP + (e & (TB - 1))] = fs[q];
+        }
         __syncthreads();
         double acc[4][2][2];
 #pragma unroll
@@ -419,14 +750,12 @@ __device__ bool run_chain(double *sm, const PotrfParams &P) {
                 }
         }
         __syncthreads();
-        if (tid == 0) {
+        // (a thread of a warp that is idle in the update below)
+        if (tid == 4 * 32) {
             __threadfence();
-            atomicExch(pdone + i * nb + j, 1);
+            atomicExch(F.p(i, j), 1);
         }
-        // S = A_ii - L_ij L_ij^T (lower tiles; the warps above the diagonal skip)
-        if (!wait_all(ver + i * nb + i, j)) return false;
-        load_frame(S, Ablk(i, i), lda, ib, ib, true);
-        __syncthreads();
+        // S = S_ii - L_ij L_ij^T (lower tiles; the warps above the diagonal skip)
         if (wm * 32 + 31 >= wn * 16) {
 #pragma unroll
             for (int mi = 0; mi < 4; ++mi)
@@ -449,12 +778,10 @@ __device__ bool run_chain(double *sm, const PotrfParams &P) {
     return true;
 }
 
-__global__ void __launch_bounds__(NTH, 2) k_potrf_tile(PotrfParams P) {
+__global__ void __launch_bounds__(NTH, 1) k_potrf_tile(PotrfParams P) {
     extern __shared__ double sm[];
-    __shared__ int item_sh, ok_sh;
+    __shared__ int item_sh;
     const int tid = threadIdx.x;
-    const int nb2 = P.nblk * P.nblk;
-    int *ver = P.cnt + 8, *pdone = ver + nb2, *xver = pdone + nb2, *xdone = xver + nb2, *ddone = xdone + nb2;
     for (;;) {
         if (tid == 0) {
             int t = -1;
@@ -468,93 +795,27 @@ __global__ void __launch_bounds__(NTH, 2) k_potrf_tile(PotrfParams P) {
         const int t = item_sh;
         if (t < 0) break;
         const PItem it = P.items[t];
-        if (it.type == IT_CHAIN) {
-            if (!run_chain(sm, P)) break;
-            __syncthreads();
-            continue;
-        }
-        const int j = it.j, i = it.i, k = it.k, n = P.n, nb = P.nblk;
-        if (tid == 0) {
-            bool ok = true;
-            switch (it.type) {
-                case IT_PANEL: ok = wait_ge(ddone + j, 1, P) && wait_ge(ver + i * nb + j, j, P); break;
-                case IT_UPD:
-                    ok = wait_ge(pdone + i * nb + j, 1, P) && wait_ge(pdone + k * nb + j, 1, P) &&
-                         wait_ge(ver + i * nb + k, j, P);
-                    break;
-                case IT_XDIAG: ok = wait_ge(ddone + j, 1, P) && wait_ge(xver + j * nb + k, j - k, P); break;
-                default:
-                    ok = wait_ge(pdone + i * nb + j, 1, P) &&
-                         (k == j ? wait_ge(ddone + j, 1, P) : wait_ge(xdone + j * nb + k, 1, P)) &&
-                         wait_ge(xver + i * nb + k, j - k, P);
-                    break;
-            }
-            ok_sh = ok;
-        }
+        if (!(it.type == IT_CHAIN ? run_chain(sm, P) : P.v16 ? run_bulk<true>(sm, it, P) : run_bulk<false>(sm, it, P)))
+            break;
         __syncthreads();
-        if (!ok_sh) break;
-        const int lda = P.lda;
-        auto Ablk = [&](int r, int c) { return P.A + (size_t)r * TB + (size_t)c * TB * lda; };
-        auto Xblk = [&](int r, int c) { return P.X + (size_t)r * TB + (size_t)c * TB * P.ldx; };
-        double *Dj = P.X ? Xblk(j, j) : P.D + (size_t)j * TB * TB;
-        const int ldd = P.X ? P.ldx : TB;
-        switch (it.type) {
-            case IT_PANEL:
-                blk_gemm(sm, Ablk(i, j), lda, bsz(i, n), bsz(j, n), bsz(j, n), 1.0, 0.0, Ablk(i, j), lda, 0, Dj, ldd, 1);
-                break;
-            case IT_UPD:
-                blk_gemm(sm, Ablk(i, k), lda, bsz(i, n), bsz(k, n), bsz(j, n), -1.0, 1.0, Ablk(i, j), lda, 0,
-                         Ablk(k, j), lda, 1);
-                break;
-            case IT_XDIAG:
-                blk_gemm(sm, Xblk(j, k), P.ldx, bsz(j, n), bsz(k, n), bsz(j, n), 1.0, 0.0, Dj, ldd, 0, Xblk(j, k),
-                         P.ldx, 0);
-                break;
-            default:
-                blk_gemm(sm, Xblk(i, k), P.ldx, bsz(i, n), bsz(k, n), bsz(j, n), -1.0, 1.0, Ablk(i, j), lda, 0,
-                         Xblk(j, k), P.ldx, 0);
-                break;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            switch (it.type) {
-                case IT_PANEL: atomicExch(pdone + i * nb + j, 1); break;
-                case IT_UPD: atomicExch(ver + i * nb + k, j + 1); break;
-                case IT_XDIAG: atomicExch(xdone + j * nb + k, 1); break;
-                default: atomicExch(xver + i * nb + k, j - k + 1); break;
-            }
-        }
     }
 }
 
-// The bulk tasks column by column (right-looking order: the updates of one
-// block come from different columns, so they never queue behind each other).
-// Each column starts with the three tasks the chain's step after next waits
-// on: PANEL(j, j+2), UPD(j, j+2, j+1) and UPD(j, j+2, j+2).
+// The bulk tasks column by column: PRE(k), which the chain's step k waits on,
+// LT(i,k), then the inverse's row k - XLAG, which the factorization does not wait
+// on (a row of it is as much work as a column of L, so it may lag behind).
 std::vector<PItem> build_items(int nblk, bool inv) {
     std::vector<PItem> v;
-    auto add = [&](int t, int j, int i, int k) {
-        v.push_back(PItem{(unsigned short)t, (unsigned short)j, (unsigned short)i, (unsigned short)k});
-    };
-    add(IT_CHAIN, 0, 0, 0);
-    for (int j = 0; j < nblk; ++j) {
-        // the chain does PANEL(j, j+1) and UPD(j, j+1, j+1)
-        if (j + 2 < nblk) {
-            add(IT_PANEL, j, j + 2, 0);
-            add(IT_UPD, j, j + 2, j + 1);
-            add(IT_UPD, j, j + 2, j + 2);
+    auto add = [&](int t, int i, int k) { v.push_back(PItem{(unsigned short)t, (unsigned short)i, (unsigned short)k, 0}); };
+    add(IT_CHAIN, 0, 0);
+    for (int k = 0; k < nblk + XLAG; ++k) {
+        if (k < nblk) {
+            if (k > 0 && k + 1 < nblk) add(IT_PRE, 0, k);
+            for (int i = k + 2; i < nblk; i += 2) add(IT_LT, i, k);
         }
-        for (int i = j + 3; i < nblk; ++i) add(IT_PANEL, j, i, 0);
-        for (int i = j + 3; i < nblk; ++i) add(IT_UPD, j, i, j + 1);
-        for (int k = j + 2; k < nblk; ++k)
-            for (int i = k; i < nblk; ++i)
-                if (i != j + 2 || k != j + 2) add(IT_UPD, j, i, k);
-        if (inv) {
-            for (int k = 0; k < j; ++k) add(IT_XDIAG, j, 0, k);
-            for (int i = j + 1; i < nblk; ++i)
-                for (int k = 0; k <= j; ++k) add(IT_XUPD, j, i, k);
-        }
+        const int r = k - XLAG;
+        if (inv && r >= 0)
+            for (int p = 0; 2 * p < r; ++p) add(IT_XT, r, p);
     }
     return v;
 }
@@ -603,7 +864,7 @@ int potrf_tile_max_n() { return 128 * TB; }
 
 size_t potrf_tile_scratch_ints(int n) {
     const size_t nb = (size_t)(n + TB - 1) / TB;
-    return 8 + 4 * nb * nb + nb;
+    return 8 + 2 * nb * nb + 2 * nb;
 }
 
 // The caller provides cnt (potrf_tile_scratch_ints(n) ints, any content) and,
@@ -614,10 +875,11 @@ int launch_potrf_tile(double *A, int lda, int n, double *X, int ldx, double *D, 
     const ItemList *L = get_items(nblk, X != nullptr, st);
     if (!L) return -1;
     if (cudaMemsetAsync(cnt, 0, potrf_tile_scratch_ints(n) * sizeof(int), st) != cudaSuccess) return -1;
-    const int smem = (int)sizeof(double) * (2 * TB * TPITCH > CHAIN_SMEM_DOUBLES ? 2 * TB * TPITCH : CHAIN_SMEM_DOUBLES);
+    const int smem = (int)sizeof(double) * SMEM_DOUBLES;
     // per device and thread-safe: set on every launch (a host-side call, no synchronisation)
     cudaFuncSetAttribute(k_potrf_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    PotrfParams P{A, lda, n, nblk, X, ldx, D, L->d, L->n, cnt, info, info_base, timeout, SPIN_LIMIT};
+    const int v16 = (((size_t)A | (size_t)X) & 15) == 0 && ((lda | (X ? ldx : 0)) & 1) == 0;
+    PotrfParams P{A, lda, n, nblk, X, ldx, D, L->d, L->n, cnt, info, info_base, timeout, v16, SPIN_LIMIT};
     // the chain waits on bulk tasks of earlier block columns, which only the
     // other CTAs take: with any bulk task in the list the launch has two CTAs
     // or more (they need not be resident at the same time)

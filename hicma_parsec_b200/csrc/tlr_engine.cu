@@ -851,12 +851,14 @@ CopyTask make_copy(const double *src, int lds, double *dst, int ldd, int rows, i
 }
 
 // ----------------------------------------------------------- tile POTRF ----
-// Blocked right-looking Cholesky of an n x n tile (64-column panels): the
+// Cholesky of an n x n tile and, with Linv, its inverse: the persistent kernel up
+// to potrf_tile_max_n(); above it blocked right-looking with 64-column panels (the
 // diagonal block is factored and inverted in one CTA, the panel below is
-// multiplied by the block inverse, the trailing matrix gets a lower DMMA
-// SYRK.  With Linv, L^-1 is then assembled block row by block row.
+// multiplied by the block inverse, the trailing matrix gets a lower DMMA SYRK, and
+// L^-1 is assembled block row by block row).
+// overlapped: other work of the factorization runs beside it.
 int potrf_tile(hicma_tlr_ctx *c, double *A, int n, int lda, double *Linv, int ldl, int *d_info,
-               int info_base) {
+               int info_base, bool overlapped = false) {
 #ifdef TLR_BOUNDS_CHECK
     BC(A, bc_span(n, n, lda), "potrf tile", 0);
     if (Linv) BC(Linv, bc_span(n, n, ldl), "potrf inverse", 0);
@@ -873,7 +875,12 @@ int potrf_tile(hicma_tlr_ctx *c, double *A, int n, int lda, double *Linv, int ld
         double *D = Linv ? nullptr : ws_alloc<double>(c, (size_t)nblk * DBK * DBK);
         if (!cnt || (!Linv && !D)) { set_err("workspace exhausted (potrf)"); return HICMA_TLR_ERR_OOM; }
         if (Linv) CUDA_TRY(cudaMemset2DAsync(Linv, (size_t)ldl * sizeof(double), 0, sizeof(double) * n, n, st));
-        const int grid = c->potrf_grid > 0 ? c->potrf_grid : c->nsm;
+        // One CTA per SM when it runs alone.  Beside a panel's updates half of that: its
+        // CTAs hold 106 KB of shared memory, which keeps the CholeskyQR kernels off their
+        // SMs, and the tile is on the critical path of small panels only (2D, tile 2700:
+        // 60 x 60 tiles 449 ms with 148 CTAs, 428 to 430 with 48 to 80, 447 with 24;
+        // 36 x 36 tiles 380, 365, 373; the tile alone 1.13, 1.7 to 1.5, 4.1 ms).
+        const int grid = c->potrf_grid > 0 ? c->potrf_grid : overlapped ? c->nsm / 2 : c->nsm;
         if (launch_potrf_tile(A, lda, n, Linv, ldl, D, cnt, d_info, info_base, c->d_flags + 3, grid, st)) {
             set_err("tile POTRF launch failed: %s", cudaGetErrorString(cudaGetLastError()));
             return HICMA_TLR_ERR_CUDA;
@@ -2777,7 +2784,8 @@ static int factorize(hicma_tlr_ctx *c, hicma_tlr_desc *A, double acc, int fixed_
                 TRY(run_syrk_lazy(c, A, k + 1, syrk_from[k + 1], k + 1));
                 syrk_from[k + 1] = k + 1;
                 CUDA_TRY(cudaEventRecord(ev[P0], c->cur));
-                TRY(potrf_tile(c, A->dense(k + 1, k + 1), NB, NB, A->linv(k + 1), NB, d_info, (k + 1) * NB));
+                TRY(potrf_tile(c, A->dense(k + 1, k + 1), NB, NB, A->linv(k + 1), NB, d_info, (k + 1) * NB,
+                               NT - (k + 1) >= 6));
                 CUDA_TRY(cudaEventRecord(ev[P1], c->cur));
                 CUDA_TRY(cudaEventRecord(evP, c->cur));
                 // the next diagonal tile's low-rank contributions of columns 0..k (all
