@@ -26,10 +26,12 @@ OBJ_CHECKED = os.path.join(OBJ, "checked")
 CHECKED_SOURCES = ["tlr_engine.cu", "serve.cu", "k_potrf.cu"]
 CLI_SRC = os.path.join(HERE, "cli", "testing_dpotrf_tlr.c")
 CLI = os.path.join(LIBDIR, "testing_dpotrf_tlr")
-SOURCES = ["k_gemm.cu", "k_tile.cu", "k_potrf.cu", "k_potrf_tile.cu", "k_qr.cu", "k_rcholqr.cu", "k_proj.cu", "k_svd.cu",
+SOURCES = ["k_gemm.cu", "k_tile.cu", "k_potrf.cu", "k_potrf_tile.cu", "k_qr.cu", "k_rcholqr.cu", "k_rcholqr_c2.cu",
+           "k_rcholqr_c4.cu", "k_proj.cu", "k_svd.cu",
            "k_skinny.cu",
            "tlr_engine.cu", "serve.cu"]
 HEADERS = ["tlr_internal.h"]
+INCLUDED = {"k_rcholqr_c2.cu": "k_rcholqr.cu", "k_rcholqr_c4.cu": "k_rcholqr.cu"}   # sources that include another
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
@@ -52,7 +54,8 @@ def _newer(target: str, deps: list[str]) -> bool:
 
 def _compile(nvcc: str, src: str, force: bool, checked: bool = False) -> tuple[str, str]:
     out = os.path.join(OBJ_CHECKED if checked else OBJ, os.path.basename(src).replace(".cu", ".o"))
-    deps = [src] + [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "hicma_tlr.h")]
+    included = [INCLUDED[f] for f in (os.path.basename(src),) if f in INCLUDED]
+    deps = [src] + [os.path.join(CSRC, h) for h in HEADERS + included] + [os.path.join(ROOT, "include", "hicma_tlr.h")]
     if not force and _newer(out, deps):
         return out, ""
     cmd = [nvcc, *ARCH, *NVCC_FLAGS, *(["-DTLR_BOUNDS_CHECK"] if checked else []), "-c", src, "-o", out]

@@ -1,5 +1,5 @@
 // QR factorization of a tall-skinny matrix by randomized CholeskyQR, one CTA
-// per matrix, FP64 (Gram products on the FP64 tensor cores).
+// or a cluster of CTAs per matrix, FP64 (Gram products on the FP64 tensor cores).
 //
 // Replaces both QRs of HCORE_dgemm_qr_svd (call sites
 // hicma_parsec/HiCMA_dpotrf_L_2flow.jdf:830-903,985-1058): the U side
@@ -49,12 +49,28 @@
 // per-warp partials are added in warp order (deterministic).  Width 64: the
 // CTA stages 256-row chunks and each warp accumulates the tiles it owns.  The
 // K x K Cholesky factorizations run on the whole CTA.  Kernels are
-// instantiated per width bucket (KM = 16, 32, 48, 64 columns); wider stacks
-// take the Householder path.
+// instantiated per width bucket (KM = 16, 32, 48, 64 columns); wider stacks are
+// factored block by block.
+//
+// One CTA per matrix when a launch has enough of them.  With few, a cluster of CS =
+// 2 or 4 CTAs shares one: each takes a slice of the rows in both passes, the
+// sketches and the Gram matrices are summed over the cluster through distributed
+// shared memory in rank order (every CTA the same sums), and the K x K work runs in
+// every CTA.  This file is compiled once per CS (CQ_CS).  Latency of one matrix of
+// 2700 rows on 1, 2, 4 CTAs: K = 64 348, 277, 224 us (R only), 476, 340, 245 us (Q
+// formed); K = 48 203, 165, 136 and 304, 213, 159 us.  What stays is the K x K work:
+// four factorizations of 15 us and three 256-row Gram products at K = 64.
+#ifndef CQ_CS
+#define CQ_CS 1
+#endif
 #include "tlr_internal.h"
+
+#include <cooperative_groups.h>
 
 namespace tlr {
 namespace {
+
+constexpr int CS = CQ_CS;
 
 constexpr int CQ_WARPS = 8;
 constexpr int CQ_THREADS = CQ_WARPS * 32;
@@ -547,9 +563,14 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
     double *ivp = dsc + KM;                        // inverse pivots of the elimination
     double *Wsc = sm + S::CHUNK - S::WS;           // per-warp 8 x 8 scratch
 
-    const CQTask t = tasks[blockIdx.x];
+    namespace cg = cooperative_groups;
+    const CQTask t = tasks[blockIdx.x / CS];
     const int k1 = t.k1, K = t.k1 + t.k2, nb = t.nb;
     if (K <= 0) return;
+    // this CTA's rows
+    const int rank = CS > 1 ? (int)(blockIdx.x % CS) : 0;
+    const int rows = CS > 1 ? ((nb + CS - 1) / CS + 31) / 32 * 32 : nb;
+    const int rbeg = min(nb, rank * rows), rend = min(nb, rbeg + rows);
 
     // tiles owned by this warp in the CTA-staged form
     int tmi[S::TPW], tni[S::TPW];
@@ -576,7 +597,7 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
 #pragma unroll
         for (int j = 0; j < KM; ++j) s[j] = 0.0;
 #pragma unroll 1
-        for (int row = tid; row < nb; row += CQ_THREADS) {
+        for (int row = rbeg + ((tid - rbeg) & (CQ_THREADS - 1)); row < rend; row += CQ_THREADS) {
             const double sg = row_sign((unsigned)row);
             const double *p1 = t.X1 + row, *p2 = t.X2 + row;
             // the row in batches of CQ_SKB loads issued back to back (the sketch
@@ -600,6 +621,27 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
 #pragma unroll
                 for (int jj = 0; jj < CQ_SKB; ++jj) s[j0 + jj] += sg * v[jj];
             }
+        }
+
+        if constexpr (CS > 1) {
+            // the cluster's sketches, summed in rank order in every CTA
+            cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+            for (int j = 0; j < KM; ++j)
+                if (j < K) sm[j * CQ_LDZ + tid] = s[j];
+            cl.sync();
+            const double *part[CS];
+#pragma unroll
+            for (int r = 0; r < CS; ++r) part[r] = cl.map_shared_rank(sm, r) + tid;
+#pragma unroll
+            for (int j = 0; j < KM; ++j) {
+                if (j >= K) continue;
+                double v = part[0][j * CQ_LDZ];
+#pragma unroll
+                for (int r = 1; r < CS; ++r) v += part[r][j * CQ_LDZ];
+                s[j] = v;
+            }
+            cl.sync();
         }
 
         // 2. shifted CholeskyQR3 of the sketch rows
@@ -657,15 +699,15 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
         constexpr bool PREFETCH = KM >= 48;
         double *zb = STAGED ? sm + warp * 32 : sm + warp * S::W;
         double v[KM];
-        if (PREFETCH) load_row<KM>(t, STAGED ? tid : warp * 32 + lane, nb, k1, K, v);
+        if (PREFETCH) load_row<KM>(t, rbeg + tid, rend, k1, K, v);
 #pragma unroll 1
-        for (int r0 = STAGED ? 0 : warp * 32; r0 < nb; r0 += CQ_THREADS) {
+        for (int r0 = rbeg + (STAGED ? 0 : warp * 32); r0 < rend; r0 += CQ_THREADS) {
             const int row = r0 + (STAGED ? tid : lane);
-            const bool valid = row < nb;
-            if (!PREFETCH) load_row<KM>(t, row, nb, k1, K, v);
+            const bool valid = row < rend;
+            if (!PREFETCH) load_row<KM>(t, row, rend, k1, K, v);
 #pragma unroll
             for (int j = 0; j < KM; ++j) zb[j * P + lane] = v[j];
-            if (PREFETCH && r0 + CQ_THREADS < nb) load_row<KM>(t, row + CQ_THREADS, nb, k1, K, v);
+            if (PREFETCH && r0 + CQ_THREADS < rend) load_row<KM>(t, row + CQ_THREADS, rend, k1, K, v);
             __syncwarp();
             // rd and R are zero past K, so the padding columns stay zero
             if (!plain) warp_trsm<KM, P>(zb, Rt, rdt, K, lane);
@@ -683,6 +725,28 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
             }
         }
         gram_reduce<KM>(acc, G, sm, tid, tmi, tni);
+        if constexpr (CS > 1) {
+            // the cluster's Gram matrices, summed in rank order in every CTA
+            cg::cluster_group cl = cg::this_cluster();
+            constexpr int E = KM * KM / CQ_THREADS;
+            cl.sync();
+            double v[E];
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const int idx = tid + q * CQ_THREADS;
+                v[q] = 0.0;
+                if (idx % KM < K && idx / KM < K)
+#pragma unroll
+                    for (int r = 0; r < CS; ++r) v[q] += cl.map_shared_rank(G, r)[idx];
+            }
+            cl.sync();
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const int idx = tid + q * CQ_THREADS;
+                if (idx % KM < K && idx / KM < K) G[idx] = v[q];
+            }
+            __syncthreads();
+        }
         {
             // ||G||_inf: warp w sums the rows i = w, w + 8, ... (column i of the
             // symmetric G, lanes over its entries), then the max over the warps
@@ -697,23 +761,24 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
             if (lane == 0) gmax_sh[warp] = mx;
         }
         const int nnull = factor<KM>(G, Rr, rdg, ivp, K, (double)nb, false, tid);   // barriers: gmax_sh visible
-        if (nnull && tid == 0 && flags) atomicAdd(flags, nnull);
+        if (nnull && tid == 0 && rank == 0 && flags) atomicAdd(flags, nnull);
         double gmax = 0.0;
 #pragma unroll
         for (int w = 0; w < CQ_WARPS; ++w) gmax = fmax(gmax, gmax_sh[w]);
         const bool again = !plain && !(gmax <= CQ_GMAX) && pass + 1 < CQ_APPLY;
         accumulate<KM>(Rr, Rt, G, rdt, K, tid);
         if (!again) break;
-        if (tid == 0 && flags) atomicAdd(flags + 1, 1);
+        if (tid == 0 && rank == 0 && flags) atomicAdd(flags + 1, 1);
     }
 
     // outputs: R (column-major); Rc^-1 for a deferred Q; or Q = Y Rc^-1
     const int ldr = t.ldr ? t.ldr : K;
-    for (int idx = tid; idx < K * K; idx += CQ_THREADS) {
-        const int i = idx % K, j = idx / K;
-        t.R[i + (size_t)j * ldr] = Rt[i * L + j];
-    }
-    if (!QF && t.Rinv) {
+    if (rank == 0)
+        for (int idx = tid; idx < K * K; idx += CQ_THREADS) {
+            const int i = idx % K, j = idx / K;
+            t.R[i + (size_t)j * ldr] = Rt[i * L + j];
+        }
+    if (!QF && t.Rinv && rank == 0) {
         tri_inverse<KM>(Rr, rdg, G, Wsc, K, tid);
         for (int idx = tid; idx < K * K; idx += CQ_THREADS) {
             const int i = idx % K, c = idx / K;
@@ -722,7 +787,7 @@ __global__ void __launch_bounds__(CQ_THREADS, KM <= 32 ? 2 : 1) k_rcholqr(const 
     }
     if constexpr (QF) {
 #pragma unroll 1
-        for (int row = tid; row < nb; row += CQ_THREADS) {
+        for (int row = rbeg + tid; row < rend; row += CQ_THREADS) {
             double x[KM];
             const double *pz = t.Z + row;
 #pragma unroll
@@ -741,13 +806,29 @@ void launch_cq(const CQTask *d_tasks, int ntasks, int *flags, cudaStream_t st) {
     const size_t smem = CQSmem<KM>::bytes();
     // per device and thread-safe: set on every launch (a host-side call, no synchronisation)
     cudaFuncSetAttribute(k_rcholqr<KM, QF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_rcholqr<KM, QF><<<ntasks, CQ_THREADS, smem, st>>>(d_tasks, flags);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ntasks * CS);
+    cfg.blockDim = dim3(CQ_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = CS > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_rcholqr<KM, QF>, d_tasks, flags);
 }
 
 template <bool QF>
 void launch_bucket(const CQTask *d_tasks, int ntasks, int kmax, int *flags, cudaStream_t st) {
     switch (rcholqr_bucket(kmax)) {
+#if CQ_CS == 1
         case 16: launch_cq<16, QF>(d_tasks, ntasks, flags, st); break;
+#else
+        case 16:   // the width of 32 on clusters
+#endif
         case 32: launch_cq<32, QF>(d_tasks, ntasks, flags, st); break;
         case 48: launch_cq<48, QF>(d_tasks, ntasks, flags, st); break;
         default: launch_cq<64, QF>(d_tasks, ntasks, flags, st); break;
@@ -756,17 +837,26 @@ void launch_bucket(const CQTask *d_tasks, int ntasks, int kmax, int *flags, cuda
 
 }  // namespace
 
-int rcholqr_kmax() { return 64; }
-
-int rcholqr_bucket(int K) { return K <= 16 ? 16 : K <= 32 ? 32 : K <= 48 ? 48 : 64; }
-
-void launch_rcholqr_batched(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags,
-                            cudaStream_t st) {
-    if (ntasks <= 0) return;
+#define CQ_NAME2(n) launch_rcholqr_cs##n
+#define CQ_NAME(n) CQ_NAME2(n)
+void CQ_NAME(CQ_CS)(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags, cudaStream_t st) {
     if (form_q)
         launch_bucket<true>(d_tasks, ntasks, kmax, flags, st);
     else
         launch_bucket<false>(d_tasks, ntasks, kmax, flags, st);
 }
+
+#if CQ_CS == 1
+int rcholqr_kmax() { return 64; }
+
+int rcholqr_bucket(int K) { return K <= 16 ? 16 : K <= 32 ? 32 : K <= 48 ? 48 : 64; }
+
+void launch_rcholqr_batched(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int cluster, int *flags,
+                            cudaStream_t st) {
+    if (ntasks <= 0) return;
+    (cluster >= 4 ? launch_rcholqr_cs4 : cluster >= 2 ? launch_rcholqr_cs2 : launch_rcholqr_cs1)(d_tasks, ntasks, kmax,
+                                                                                              form_q, flags, st);
+}
+#endif
 
 }  // namespace tlr

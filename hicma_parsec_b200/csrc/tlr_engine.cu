@@ -547,16 +547,24 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
             set_err("CholeskyQR batch mixes tasks that form Q with tasks that do not");
             return HICMA_TLR_ERR_ARG;
         }
-    // one launch per width bucket (the kernel is instantiated per bucket)
+    // one launch per width bucket (the kernel is instantiated per bucket); a bucket
+    // joins the next wider one while both together leave half of the SMs free: the
+    // launch then lasts as long as its widest matrix instead of one after the other.
+    // Few matrices share clusters of CTAs while those fit three quarters of the SMs
+    // (the tile POTRF holds the others).
     std::vector<CQTask> b;
     int lo = 0;
     while (lo < rcholqr_kmax()) {
         const int hi = rcholqr_bucket(lo + 1);
-        b.clear();
         for (auto &t : v)
             if (t.k1 + t.k2 > lo && t.k1 + t.k2 <= hi) b.push_back(t);
+        size_t next = 0;
+        const int up = hi < rcholqr_kmax() ? rcholqr_bucket(hi + 1) : hi;
+        for (auto &t : v) next += t.k1 + t.k2 > hi && t.k1 + t.k2 <= up;
         lo = hi;
         if (b.empty()) continue;
+        if (next && 2 * (b.size() + next) <= (size_t)c->nsm) continue;
+        const int cap = c->nsm * 3 / 4, cluster = 4 * (int)b.size() <= cap ? 4 : 2 * (int)b.size() <= cap ? 2 : 1;
         CQTask *d = stage(c, b.data(), b.size());
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
         double fl = 0, by = 0;
@@ -572,9 +580,10 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
         }
         {
             Prof pf(c, P_CHOLQR, fl, by);
-            launch_rcholqr_batched(d, (int)b.size(), hi, form_q, c->d_flags + 5, c->cur);
+            launch_rcholqr_batched(d, (int)b.size(), hi, form_q, cluster, c->d_flags + 5, c->cur);
         }
         TRY(check_launch(c));
+        b.clear();
     }
     v.clear();
     return 0;

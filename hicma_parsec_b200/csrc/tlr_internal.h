@@ -274,9 +274,13 @@ struct CQTask {
 };
 int rcholqr_kmax();
 int rcholqr_bucket(int K);   // width of the kernel instance that takes K
-// form_q: every task of the launch sets Q (and none sets Rinv); otherwise none sets Q
-void launch_rcholqr_batched(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags,
+// form_q: every task of the launch sets Q (and none sets Rinv); otherwise none sets Q.
+// cluster: CTAs per matrix (1, 2 or 4).
+void launch_rcholqr_batched(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int cluster, int *flags,
                             cudaStream_t st);
+void launch_rcholqr_cs1(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags, cudaStream_t st);
+void launch_rcholqr_cs2(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags, cudaStream_t st);
+void launch_rcholqr_cs4(const CQTask *d_tasks, int ntasks, int kmax, bool form_q, int *flags, cudaStream_t st);
 
 // ------------------------------------------------------------- core SVD -----
 // M = RU RV^T (RU, RV: K x K upper from the QRs; RU == nullptr means I),

@@ -88,3 +88,22 @@ def test_core_svd_fixed_rank(ctx, K, fixed):
     assert r == fixed
     s = np.linalg.svd(Cu @ Cv.T - Au @ Y.T, compute_uv=False)
     assert abs(np.linalg.norm(U @ V.T) - np.sqrt((s[:fixed] ** 2).sum())) <= 100 * K * EPS * np.linalg.norm(s[:fixed])
+
+
+@pytest.mark.parametrize("nb", [21, 33, 64, 100, 257, 1030])
+@pytest.mark.parametrize("K", [5, 17, 40, 64])
+def test_narrow_qr_row_slices(ctx, nb, K):
+    """Stacks up to 64 columns with few rows: the clusters of CTAs that share a
+    matrix when a launch has few of them get partial, single or no row chunks."""
+    K = min(K, nb - 1)
+    rng = np.random.default_rng(nb * 100 + K)
+    rc = K // 2
+    Cu, Au, Av = orth(rng, nb, rc), orth(rng, nb, K - rc), orth(rng, nb, K - rc)
+    Cv, Y = orth(rng, nb, rc) * np.linspace(3.0, 1.0, rc), orth(rng, nb, K - rc)
+    ref = Cu @ Cv.T - Au @ Y.T
+    s = np.linalg.svd(ref, compute_uv=False)
+    r, U, V = update(ctx, nb, Cu, Cv, Au, Av, Y, Av, 1e-6, max(K, 1))
+    assert r == int((s >= 1e-6).sum())
+    # backward stable QRs and core: 100 K eps sigma_1, plus what the truncation at 1e-6 may drop
+    assert np.linalg.norm(U @ V.T - ref, 2) <= 100 * K * EPS * s[0] + (s[r] if r < len(s) else 0.0)
+    assert np.abs(U.T @ U - np.eye(r)).max() <= 100 * K * EPS
