@@ -128,7 +128,8 @@ struct hicma_tlr_ctx_s {
     int device = 0;
     cudaStream_t stream = nullptr;      // bulk work
     cudaStream_t stream_hi = nullptr;   // critical path (high priority): SYRK(k,k+1) + POTRF(k+1)
-    cudaStream_t stream_side = nullptr; // wide recompressions (Householder chain) beside the CholeskyQR chain
+    cudaStream_t stream_side = nullptr; // wide recompressions beside the narrow ones
+    cudaStream_t stream_core = nullptr; // their narrower core SVDs beside the widest
     cudaStream_t stream_copy = nullptr; // copy-out of final factor columns during a factorization
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t cur = nullptr;         // stream the helpers launch on
@@ -209,6 +210,7 @@ size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 int ctx_sync(hicma_tlr_ctx *c) {
     CUDA_TRY(cudaStreamSynchronize(c->stream_hi));
+    CUDA_TRY(cudaStreamSynchronize(c->stream_core));
     CUDA_TRY(cudaStreamSynchronize(c->stream_side));
     CUDA_TRY(cudaStreamSynchronize(c->stream_copy));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -268,6 +270,7 @@ T *stage(hicma_tlr_ctx *c, const T *src, size_t n) {
     if (bytes > c->stage_bytes) return nullptr;
     if (c->stage_off + bytes > c->stage_bytes) {
         if (cudaStreamSynchronize(c->stream_hi) != cudaSuccess) return nullptr;
+        if (cudaStreamSynchronize(c->stream_core) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream_side) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) return nullptr;
         c->stage_off = 0;
@@ -985,13 +988,14 @@ size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
 // no more tasks than SMs: it is then one CTA per SM either way, and a launch
 // lasts as long as its slowest core.  Cores of 65 to 96 columns run on clusters of
 // four CTAs, with the wider ones, while those clusters fit the device at once.
-int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreParams &cp) {
+int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreParams &cp, bool spread = false) {
     int mid = 0;
     for (auto &t : cores) mid += t.K > core_smem_kmax() && t.K <= core_one_cta_kmax();
     const bool cluster = 4 * mid <= c->nsm;
     auto bucket_of = [&](const CoreTask &t) { return core_bucket(t.K, cluster); };
     std::stable_sort(cores.begin(), cores.end(),
                      [&](const CoreTask &a, const CoreTask &b) { return bucket_of(a) < bucket_of(b); });
+    std::vector<std::pair<size_t, size_t>> launches;
     size_t i = 0;
     while (i < cores.size()) {
         size_t e = i;
@@ -1004,11 +1008,30 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
             if (f - i > (size_t)c->nsm) break;
             e = f;
         }
-        std::vector<CoreTask> bucket(cores.begin() + (long)i, cores.begin() + (long)e);
+        launches.emplace_back(i, e);
+        i = e;
+    }
+    // Widest first; with `spread` the others beside it on a stream of their own: each
+    // launch lasts as long as its slowest core (0.5 to 0.9 ms) and few of them fill the
+    // device (36 x 36 tiles of 2700 330 -> 322 ms, 3D N = 16000 110 -> 107).
+    spread = spread && launches.size() > 1;
+    cudaStream_t st = c->cur;
+    if (spread) {
+        CUDA_TRY(cudaEventRecord(c->ev_fork, st));
+        CUDA_TRY(cudaStreamWaitEvent(c->stream_core, c->ev_fork, 0));
+    }
+    for (size_t q = launches.size(); q-- > 0;) {
+        std::vector<CoreTask> bucket(cores.begin() + (long)launches[q].first, cores.begin() + (long)launches[q].second);
         int kmax = 0;
         for (auto &t : bucket) kmax = std::max(kmax, t.K);
-        TRY(run_core(c, bucket, kmax, cp, cluster));
-        i = e;
+        c->cur = spread && q + 1 < launches.size() ? c->stream_core : st;
+        const int rc = run_core(c, bucket, kmax, cp, cluster);
+        c->cur = st;
+        TRY(rc);
+    }
+    if (spread) {
+        CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_core));
+        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0));
     }
     cores.clear();
     return 0;
@@ -1220,7 +1243,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             TRY(check_launch(c));
         }
         CoreParams cp{0, acc, maxrank, fixed_rank, nb, c->d_flags + 1, c->d_flags + 2};
-        TRY(run_core_buckets(c, coresS, cp));
+        TRY(run_core_buckets(c, coresS, cp, side));
         TRY(run_qapply(c, apps, nb));
         TRY(run_gemms(c, gUS));
         TRY(run_gemms(c, g3S));
@@ -1529,6 +1552,7 @@ static void ctx_release(hicma_tlr_ctx *c) {
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream_side) cudaStreamDestroy(c->stream_side);
+    if (c->stream_core) cudaStreamDestroy(c->stream_core);
     if (c->stream_copy) cudaStreamDestroy(c->stream_copy);
     if (c->stream_hi) cudaStreamDestroy(c->stream_hi);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1553,7 +1577,12 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
     e = cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->stream_hi, cudaStreamNonBlocking, prio_hi);
     if (e != cudaSuccess) return fail(e, "priority stream");
-    e = cudaStreamCreateWithFlags(&c->stream_side, cudaStreamNonBlocking);
+    // The wide chain of a panel is a long series of launches that hold few tasks: it goes
+    // before the bulk, whose launches then fill the SMs it leaves, but after the next
+    // panel's POTRF (60 x 60 tiles of 2700: 409 ms at the bulk's priority, 390 so).
+    const int prio_side = std::min(prio_lo, prio_hi + 1);
+    e = cudaStreamCreateWithPriority(&c->stream_side, cudaStreamNonBlocking, prio_side);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->stream_core, cudaStreamNonBlocking, prio_side);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream_copy, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
