@@ -141,6 +141,9 @@ struct hicma_tlr_ctx_s {
     Arena *ar = nullptr;                // arena of `cur`
     char *h_stage = nullptr, *d_stage = nullptr;
     size_t stage_bytes = 0, stage_off = 0;
+    bool batching = false;                          // launches wait for one upload of their tasks (Batch)
+    size_t held_from = 0;                           // staged bytes from here on are not uploaded yet
+    std::vector<std::function<int()>> held;         // the launches, in order
     int *d_flags = nullptr;     // [0] info, [1] overflow, [2] Jacobi sweeps, [3] wait timed out, [4] FP32 updates,
                                 // [5] CholeskyQR null pivots, [6] CholeskyQR passes repeated
     int nsm = 148;              // SM count of the device
@@ -265,21 +268,74 @@ struct OnHi {
     ~OnHi() { c->cur = c->stream; c->ar = &c->main_ar; }
 };
 
+// Uploads what is staged on the current stream and makes the held launches.  `wait`:
+// also for streams that are not ordered after it.
+int issue_held(hicma_tlr_ctx *c, bool wait = false) {
+    if (c->stage_off > c->held_from)
+        CUDA_TRY(cudaMemcpyAsync(c->d_stage + c->held_from, c->h_stage + c->held_from, c->stage_off - c->held_from,
+                                 cudaMemcpyHostToDevice, c->cur));
+    if (wait) CUDA_TRY(cudaStreamSynchronize(c->cur));
+    c->held_from = c->stage_off;
+    std::vector<std::function<int()>> q;
+    q.swap(c->held);
+    cudaStream_t st = c->cur;
+    int rc = 0;
+    for (size_t i = 0; i < q.size() && !rc; ++i) rc = q[i]();
+    c->cur = st;
+    return rc;
+}
+
+// A launch (or an event call) on the current stream: made now, or held inside a Batch.
+template <class F>
+int issue(hicma_tlr_ctx *c, F f) {
+    if (!c->batching) return f();
+    cudaStream_t st = c->cur;
+    c->held.push_back([c, st, f]() {
+        c->cur = st;
+        return f();
+    });
+    return 0;
+}
+
+// While a Batch lives, the helpers stage their task arrays and hold their launches;
+// flush() uploads all arrays in one copy on the current stream, then launches.  A copy
+// per launch sits in the stream before it: 3 us of copy and 6 us of gaps to a launch of
+// 20 to 200 us in the chains of a late panel.  One copy a batch: 2D requests of 27,000
+// and 97,200 unknowns 77.3, 314 ms -> 73.3, 299; 60 x 60 tiles 390 -> 377.
+struct Batch {
+    hicma_tlr_ctx *c;
+    bool mine;
+    explicit Batch(hicma_tlr_ctx *ctx) : c(ctx), mine(!ctx->batching) {
+        if (!mine) return;
+        c->batching = true;
+        c->held_from = c->stage_off;
+    }
+    int flush() { return mine ? issue_held(c) : 0; }
+    ~Batch() {
+        if (!mine) return;
+        c->held.clear();       // left only by an error
+        c->batching = false;
+    }
+    Batch(const Batch &) = delete;
+    Batch &operator=(const Batch &) = delete;
+};
+
 template <class T>
 T *stage(hicma_tlr_ctx *c, const T *src, size_t n) {
     const size_t raw = n * sizeof(T);
     const size_t bytes = align_up(raw + 1);
     if (bytes > c->stage_bytes) return nullptr;
     if (c->stage_off + bytes > c->stage_bytes) {
+        if (c->batching && issue_held(c, true)) return nullptr;
         if (cudaStreamSynchronize(c->stream_hi) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream_core) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream_side) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) return nullptr;
-        c->stage_off = 0;
+        c->stage_off = c->held_from = 0;
     }
     std::memcpy(c->h_stage + c->stage_off, src, raw);
-    if (cudaMemcpyAsync(c->d_stage + c->stage_off, c->h_stage + c->stage_off, raw,
-                        cudaMemcpyHostToDevice, c->cur) != cudaSuccess)
+    if (!c->batching && cudaMemcpyAsync(c->d_stage + c->stage_off, c->h_stage + c->stage_off, raw,
+                                        cudaMemcpyHostToDevice, c->cur) != cudaSuccess)
         return nullptr;
     T *d = (T *)(c->d_stage + c->stage_off);
     c->stage_off += bytes;
@@ -522,12 +578,13 @@ int run_qr(hicma_tlr_ctx *c, std::vector<QRTask> &v, int m_max) {
         fl += 2.0 * t.m * (double)t.K * t.K - 2.0 / 3.0 * (double)t.K * t.K * t.K;
         by += 16.0 * t.m * (double)t.K;
     }
-    {
-        Prof pf(c, P_QR, fl, by);
-        launch_qr_batched(d, (int)v.size(), m_max, c->cur);
-    }
+    const int n = (int)v.size();
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        Prof pf(c, P_QR, fl, by);
+        launch_qr_batched(d, n, m_max, c->cur);
+        return check_launch(c);
+    });
 }
 
 int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
@@ -583,11 +640,12 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
             // X read twice; Y written when kept; Y read and Q written when Q is formed
             by += 8.0 * t.nb * K * (t.plain ? 3.0 : 2.0 + (t.Q || t.Rinv ? 1.0 : 0.0) + (t.Q ? 2.0 : 0.0));
         }
-        {
+        const int n = (int)b.size();
+        TRY(issue(c, [=]() {
             Prof pf(c, P_CHOLQR, fl, by);
-            launch_rcholqr_batched(d, (int)b.size(), hi, form_q, cluster, c->d_flags + 5, c->cur);
-        }
-        TRY(check_launch(c));
+            launch_rcholqr_batched(d, n, hi, form_q, cluster, c->d_flags + 5, c->cur);
+            return check_launch(c);
+        }));
         b.clear();
     }
     v.clear();
@@ -601,12 +659,13 @@ int run_qapply(hicma_tlr_ctx *c, std::vector<QApplyTask> &v, int m_max) {
     if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
     double by = 0;
     for (auto &t : v) by += 8.0 * t.m * (double)t.K;
-    {
-        Prof pf(c, P_QAPPLY, 0, by);
-        launch_qapply_batched(d, (int)v.size(), m_max, c->cur);
-    }
+    const int n = (int)v.size();
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        Prof pf(c, P_QAPPLY, 0, by);
+        launch_qapply_batched(d, n, m_max, c->cur);
+        return check_launch(c);
+    });
 }
 
 int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CoreParams &cp, bool cluster) {
@@ -614,12 +673,13 @@ int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CorePar
     TRY(bc_cores(v));
     CoreTask *d = stage(c, v.data(), v.size());
     if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-    {
-        Prof pf(c, P_CORE, 0, 0);
-        launch_core_svd_batched(d, (int)v.size(), std::max(kmax, 1), cp, cluster, c->cur);
-    }
+    const int n = (int)v.size();
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        Prof pf(c, P_CORE, 0, 0);
+        launch_core_svd_batched(d, n, std::max(kmax, 1), cp, cluster, c->cur);
+        return check_launch(c);
+    });
 }
 
 int run_gemms_narrow(hicma_tlr_ctx *c, std::vector<GemmTask> &v, int cls);
@@ -678,13 +738,16 @@ int run_gemms(hicma_tlr_ctx *c, std::vector<GemmTask> &v, bool fp32 = false, int
     if (!dt || !doff) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
     double fl = 0, by = 0;
     bool ndev = gemm_work(v, fl, by);
-    {
-        Prof pf(c, cls, fl, by);
-        launch_gemm_batched(dt, doff, (int)v.size(), off[v.size()], c->cur, fp32);
-    }
-    if (ndev && c->prof) launch_gemm_devcount(dt, (int)v.size(), c->d_profacc + 2 * cls, c->cur);
+    const int n = (int)v.size(), tiles = off[v.size()];
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        {
+            Prof pf(c, cls, fl, by);
+            launch_gemm_batched(dt, doff, n, tiles, c->cur, fp32);
+        }
+        if (ndev && c->prof) launch_gemm_devcount(dt, n, c->d_profacc + 2 * cls, c->cur);
+        return check_launch(c);
+    });
 }
 
 int run_gemms_narrow(hicma_tlr_ctx *c, std::vector<GemmTask> &v, int cls) {
@@ -702,13 +765,16 @@ int run_gemms_narrow(hicma_tlr_ctx *c, std::vector<GemmTask> &v, int cls) {
     if (!dt || !doff) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
     double fl = 0, by = 0;
     bool ndev = gemm_work(v, fl, by);
-    {
-        Prof pf(c, cls, fl, by);
-        launch_gemm_batched_narrow(dt, doff, (int)v.size(), off[v.size()], c->cur);
-    }
-    if (ndev && c->prof) launch_gemm_devcount(dt, (int)v.size(), c->d_profacc + 2 * cls, c->cur);
+    const int n = (int)v.size(), tiles = off[v.size()];
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        {
+            Prof pf(c, cls, fl, by);
+            launch_gemm_batched_narrow(dt, doff, n, tiles, c->cur);
+        }
+        if (ndev && c->prof) launch_gemm_devcount(dt, n, c->d_profacc + 2 * cls, c->cur);
+        return check_launch(c);
+    });
 }
 
 // Batched inner products P = C^T W of nb-long columns (split-K DMMA, one CTA
@@ -734,11 +800,11 @@ int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
         for (size_t q = i; q < i + n; ++q) blocks = std::max(blocks, gram_blocks(v[q].rc, v[q].ra));
         GramTask *d = stage(c, v.data() + i, n);
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-        {
+        TRY(issue(c, [=]() {
             Prof pf(c, cls, i ? 0.0 : fl, i ? 0.0 : by);
             launch_gram_batched(d, (int)n, blocks, c->cur);
-        }
-        TRY(check_launch(c));
+            return check_launch(c);
+        }));
     }
     v.clear();
     return 0;
@@ -800,8 +866,11 @@ int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
         }
         RInitTask *d = stage(c, ri.data(), ri.size());
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-        launch_rinit(d, (int)ri.size(), kmax, c->cur);
-        TRY(check_launch(c));
+        const int n = (int)ri.size();
+        TRY(issue(c, [=]() {
+            launch_rinit(d, n, kmax, c->cur);
+            return check_launch(c);
+        }));
     }
     for (int b = 0;; ++b) {
         std::vector<GramTask> g1, g2;
@@ -850,10 +919,13 @@ int run_copies(hicma_tlr_ctx *c, std::vector<CopyTask> &v) {
     if (!dt) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
     double by = 0;
     for (auto &t : v) by += 16.0 * t.rows * (double)t.cols;
-    Prof pf(c, P_COPY, 0, by);
-    launch_copy_batched(dt, (int)v.size(), maxc, c->cur);
+    const int n = (int)v.size();
     v.clear();
-    return check_launch(c);
+    return issue(c, [=]() {
+        Prof pf(c, P_COPY, 0, by);
+        launch_copy_batched(dt, n, maxc, c->cur);
+        return check_launch(c);
+    });
 }
 
 CopyTask make_copy(const double *src, int lds, double *dst, int ldd, int rows, int cols, double alpha = 1.0,
@@ -1019,8 +1091,8 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
     spread = spread && launches.size() > 1;
     cudaStream_t st = c->cur;
     if (spread) {
-        CUDA_TRY(cudaEventRecord(c->ev_fork, st));
-        CUDA_TRY(cudaStreamWaitEvent(c->stream_core, c->ev_fork, 0));
+        TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_fork, st)); return 0; }));
+        TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(c->stream_core, c->ev_fork, 0)); return 0; }));
     }
     for (size_t q = launches.size(); q-- > 0;) {
         std::vector<CoreTask> bucket(cores.begin() + (long)launches[q].first, cores.begin() + (long)launches[q].second);
@@ -1032,8 +1104,8 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
         TRY(rc);
     }
     if (spread) {
-        CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_core));
-        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0));
+        TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_core)); return 0; }));
+        TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0)); return 0; }));
     }
     cores.clear();
     return 0;
@@ -1203,23 +1275,29 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             (cq ? g4 : g4S).push_back(b);
         }
         TRY(bc_recompress_parts(sels, grams, projs, asm_));
+        Batch batch(c);
         TRY(run_copies(c, copies));
         if (!sels.empty()) {
             SelTask *d = stage(c, sels.data(), sels.size());
             if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-            launch_precision_select(d, (int)sels.size(), thr2, c->d_flags + 4, c->cur);
-            TRY(check_launch(c));
+            const int n = (int)sels.size();
+            TRY(issue(c, [=]() {
+                launch_precision_select(d, n, thr2, c->d_flags + 4, c->cur);
+                return check_launch(c);
+            }));
         }
         TRY(run_grams(c, grams, P_GRAM));
         TRY(run_gemms(c, g1, false, P_GEMM_Y));
         TRY(run_gemms(c, g1s, true, P_GEMM_Y));
         TRY(run_gemms(c, g2, false, P_GEMM_Y));
         TRY(run_gemms(c, g2s, true, P_GEMM_Y));
+        // the device starts on these while the host prepares the rest
+        TRY(batch.flush());
         const bool side = !coresS.empty();
         cudaStream_t bulk = c->cur;
         if (side) {
-            CUDA_TRY(cudaEventRecord(c->ev_fork, bulk));
-            CUDA_TRY(cudaStreamWaitEvent(c->stream_side, c->ev_fork, 0));
+            TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_fork, bulk)); return 0; }));
+            TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(c->stream_side, c->ev_fork, 0)); return 0; }));
             c->cur = c->stream_side;
         }
         TRY(run_copies(c, copiesS));
@@ -1230,19 +1308,25 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 fl += 8.0 * p.nb * p.rc * p.ra;             // two rounds of C^T W and C P
                 by += 8.0 * p.nb * (p.rc + 2.0 * p.ra);     // C and W read once, W written once
             }
-            Prof pr(c, P_PROJ, fl, by);
             ProjTask *d = stage(c, projs.data(), projs.size());
             if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-            launch_bcgs2(d, (int)projs.size(), c->cur);
-            TRY(check_launch(c));
+            const int n = (int)projs.size();
+            TRY(issue(c, [=]() {
+                Prof pr(c, P_PROJ, fl, by);
+                launch_bcgs2(d, n, c->cur);
+                return check_launch(c);
+            }));
         }
         TRY(run_qr(c, qrs, nb));
         TRY(run_block_qr(c, bqs));
         if (!asm_.empty()) {
             AssembleTask *d = stage(c, asm_.data(), asm_.size());
             if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-            launch_assemble_r(d, (int)asm_.size(), c->cur);
-            TRY(check_launch(c));
+            const int n = (int)asm_.size();
+            TRY(issue(c, [=]() {
+                launch_assemble_r(d, n, c->cur);
+                return check_launch(c);
+            }));
         }
         CoreParams cp{0, acc, maxrank, fixed_rank, nb, c->d_flags + 1, c->d_flags + 2};
         TRY(run_core_buckets(c, coresS, cp, side));
@@ -1251,7 +1335,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         TRY(run_gemms(c, g3S));
         TRY(run_gemms(c, g4S));
         if (side) {
-            CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_side));
+            TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_side)); return 0; }));
             c->cur = bulk;
         }
         TRY(run_rcholqr(c, vrs, 0));
@@ -1261,7 +1345,8 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         TRY(run_gemms(c, g3));
         TRY(run_gemms(c, g4));
         // the next chunk reuses the workspace: it starts after both chains
-        if (side) CUDA_TRY(cudaStreamWaitEvent(bulk, c->ev_join, 0));
+        if (side) TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(bulk, c->ev_join, 0)); return 0; }));
+        TRY(batch.flush());
         i0 = i;
     }
     c->ar->off = mark;
@@ -2576,6 +2661,7 @@ static int stream_column(hicma_tlr_ctx *c, hicma_tlr_desc *A, int k, cudaEvent_t
 // dense T -= A A^T (CORE_dsyrk), low rank T -= U (V^T V) U^T (HCORE_dsyrk),
 // HiCMA_dpotrf_L_2flow.jdf:503-565; rank 0 skips (:511-513).
 static int run_syrk(hicma_tlr_ctx *c, hicma_tlr_desc *A, int k, const std::vector<int> &ms) {
+    Batch batch(c);
     const int NB = A->NB;
     const size_t mark = c->ar->off;
     std::vector<GemmTask> g1, g2, g3;
@@ -2608,7 +2694,7 @@ static int run_syrk(hicma_tlr_ctx *c, hicma_tlr_desc *A, int k, const std::vecto
     TRY(run_gemms(c, g2, false, P_GEMM_SYRK));
     TRY(run_gemms(c, g3, false, P_GEMM_SYRK));
     c->ar->off = mark;
-    return 0;
+    return batch.flush();
 }
 
 // The low-rank SYRK contributions of columns j in [j0, j1) to diagonal tile m
@@ -2620,6 +2706,7 @@ static int run_syrk(hicma_tlr_ctx *c, hicma_tlr_desc *A, int k, const std::vecto
 // critical path, and only column m-1 right before POTRF(m).  Chunked to the
 // free workspace.
 static int run_syrk_lazy(hicma_tlr_ctx *c, hicma_tlr_desc *A, int m, int j0, int j1) {
+    Batch batch(c);
     const int NB = A->NB;
     const size_t mark = c->ar->off;
     std::vector<int> js;
@@ -2663,7 +2750,7 @@ static int run_syrk_lazy(hicma_tlr_ctx *c, hicma_tlr_desc *A, int m, int j0, int
         p = q;
     }
     c->ar->off = mark;
-    return 0;
+    return batch.flush();
 }
 
 static unsigned long syrk_ops(const hicma_tlr_desc *A, int k, int m) {
@@ -2780,6 +2867,7 @@ static int factorize(hicma_tlr_ctx *c, hicma_tlr_desc *A, double acc, int fixed_
             // arena bytes of the gathered block and its product for w columns
             auto lr_need = [&](size_t w) { return w ? 2 * align_up(sizeof(double) * NB * w + 1) : 0; };
             auto flush = [&]() -> int {
+                Batch batch(c);
                 TRY(run_gemms(c, g, false, P_GEMM_TRSM));
                 TRY(run_copies(c, cp));
                 if (!lr.empty()) {
@@ -2801,7 +2889,7 @@ static int factorize(hicma_tlr_ctx *c, hicma_tlr_desc *A, double acc, int fixed_
                     sumr = 0;
                 }
                 c->ar->off = base_mark;
-                return 0;
+                return batch.flush();
             };
             for (int m = k + 1; m < NT; ++m) {
                 if (m == k + 2) {
@@ -2971,9 +3059,13 @@ static int factorize(hicma_tlr_ctx *c, hicma_tlr_desc *A, double acc, int fixed_
                     }
                 }
             }
-            TRY(run_gemms(c, g1, false, P_GEMM_DENSE));
-            TRY(run_gemms(c, g2, false, P_GEMM_DENSE));
-            TRY(run_gemms(c, g3, false, P_GEMM_DENSE));
+            {
+                Batch batch(c);
+                TRY(run_gemms(c, g1, false, P_GEMM_DENSE));
+                TRY(run_gemms(c, g2, false, P_GEMM_DENSE));
+                TRY(run_gemms(c, g3, false, P_GEMM_DENSE));
+                TRY(batch.flush());
+            }
             c->ar->off = base_mark;
             TRY(run_recompress(c, NB, rec, acc, maxrank, fixed_rank, rtask, thr2));
             CUDA_TRY(cudaEventRecord(ev[G1], c->stream));
