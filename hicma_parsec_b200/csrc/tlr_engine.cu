@@ -130,7 +130,7 @@ struct hicma_tlr_ctx_s {
     cudaStream_t stream = nullptr;      // bulk work
     cudaStream_t stream_hi = nullptr;   // critical path (high priority): SYRK(k,k+1) + POTRF(k+1)
     cudaStream_t stream_side = nullptr; // wide recompressions beside the narrow ones
-    cudaStream_t stream_core = nullptr; // their narrower core SVDs beside the widest
+    cudaStream_t stream_core = nullptr; // their narrower QRs and core SVDs beside the widest
     cudaStream_t stream_copy = nullptr; // copy-out of final factor columns during a factorization
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t cur = nullptr;         // stream the helpers launch on
@@ -587,6 +587,22 @@ int run_qr(hicma_tlr_ctx *c, std::vector<QRTask> &v, int m_max) {
     });
 }
 
+// stream_core starts after what `st` holds; `st` goes on after what stream_core holds.
+int fork_core(hicma_tlr_ctx *c, cudaStream_t st) {
+    return issue(c, [=]() {
+        CUDA_TRY(cudaEventRecord(c->ev_fork, st));
+        CUDA_TRY(cudaStreamWaitEvent(c->stream_core, c->ev_fork, 0));
+        return 0;
+    });
+}
+int join_core(hicma_tlr_ctx *c, cudaStream_t st) {
+    return issue(c, [=]() {
+        CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_core));
+        CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0));
+        return 0;
+    });
+}
+
 int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
     if (v.empty()) return 0;
 #ifdef TLR_BOUNDS_CHECK
@@ -614,6 +630,12 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
     // launch then lasts as long as its widest matrix instead of one after the other.
     // Few matrices share clusters of CTAs while those fit three quarters of the SMs
     // (the tile POTRF holds the others).
+    struct Launch {
+        CQTask *d;
+        int n, hi, cluster;
+        double fl, by;
+    };
+    std::vector<Launch> ls;
     std::vector<CQTask> b;
     int lo = 0;
     while (lo < rcholqr_kmax()) {
@@ -640,15 +662,28 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
             // X read twice; Y written when kept; Y read and Q written when Q is formed
             by += 8.0 * t.nb * K * (t.plain ? 3.0 : 2.0 + (t.Q || t.Rinv ? 1.0 : 0.0) + (t.Q ? 2.0 : 0.0));
         }
-        const int n = (int)b.size();
-        TRY(issue(c, [=]() {
-            Prof pf(c, P_CHOLQR, fl, by);
-            launch_rcholqr_batched(d, n, hi, form_q, cluster, c->d_flags + 5, c->cur);
-            return check_launch(c);
-        }));
+        ls.push_back({d, (int)b.size(), hi, cluster, fl, by});
         b.clear();
     }
     v.clear();
+    // Widest first.  In the chain of the wide updates, which is bound by the latency of
+    // its launches, the narrower ones run beside it on the cores' stream
+    // (36 x 36 tiles of 2700 299.2 -> 295.2 ms, 20 x 20 of 1350 73.3 -> 72.4).
+    const bool spread = c->cur == c->stream_side && ls.size() > 1;
+    cudaStream_t st = c->cur;
+    if (spread) TRY(fork_core(c, st));
+    for (size_t q = ls.size(); q-- > 0;) {
+        const Launch l = ls[q];
+        c->cur = spread && q + 1 < ls.size() ? c->stream_core : st;
+        const int rc = issue(c, [=]() {
+            Prof pf(c, P_CHOLQR, l.fl, l.by);
+            launch_rcholqr_batched(l.d, l.n, l.hi, form_q, l.cluster, c->d_flags + 5, c->cur);
+            return check_launch(c);
+        });
+        c->cur = st;
+        TRY(rc);
+    }
+    if (spread) TRY(join_core(c, st));
     return 0;
 }
 
@@ -1090,10 +1125,7 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
     // device (36 x 36 tiles of 2700 330 -> 322 ms, 3D N = 16000 110 -> 107).
     spread = spread && launches.size() > 1;
     cudaStream_t st = c->cur;
-    if (spread) {
-        TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_fork, st)); return 0; }));
-        TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(c->stream_core, c->ev_fork, 0)); return 0; }));
-    }
+    if (spread) TRY(fork_core(c, st));
     for (size_t q = launches.size(); q-- > 0;) {
         std::vector<CoreTask> bucket(cores.begin() + (long)launches[q].first, cores.begin() + (long)launches[q].second);
         int kmax = 0;
@@ -1103,10 +1135,7 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
         c->cur = st;
         TRY(rc);
     }
-    if (spread) {
-        TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_core)); return 0; }));
-        TRY(issue(c, [=]() { CUDA_TRY(cudaStreamWaitEvent(st, c->ev_join, 0)); return 0; }));
-    }
+    if (spread) TRY(join_core(c, st));
     cores.clear();
     return 0;
 }
