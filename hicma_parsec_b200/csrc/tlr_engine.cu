@@ -142,6 +142,7 @@ struct hicma_tlr_ctx_s {
     char *h_stage = nullptr, *d_stage = nullptr;
     size_t stage_bytes = 0, stage_off = 0;
     bool batching = false;                          // launches wait for one upload of their tasks (Batch)
+    bool batch_split = false;                       // the ring wrapped inside the Batch: part of it is launched
     size_t held_from = 0;                           // staged bytes from here on are not uploaded yet
     std::vector<std::function<int()>> held;         // the launches, in order
     int *d_flags = nullptr;     // [0] info, [1] overflow, [2] Jacobi sweeps, [3] wait timed out, [4] FP32 updates,
@@ -268,13 +269,14 @@ struct OnHi {
     ~OnHi() { c->cur = c->stream; c->ar = &c->main_ar; }
 };
 
-// Uploads what is staged on the current stream and makes the held launches.  `wait`:
-// also for streams that are not ordered after it.
-int issue_held(hicma_tlr_ctx *c, bool wait = false) {
+// Uploads what is staged on the current stream and makes the held launches.  Other
+// streams join the current one by an event held among them, so after the upload; once
+// a part of the Batch with such an event is launched, the host waits for the upload.
+int issue_held(hicma_tlr_ctx *c) {
     if (c->stage_off > c->held_from)
         CUDA_TRY(cudaMemcpyAsync(c->d_stage + c->held_from, c->h_stage + c->held_from, c->stage_off - c->held_from,
                                  cudaMemcpyHostToDevice, c->cur));
-    if (wait) CUDA_TRY(cudaStreamSynchronize(c->cur));
+    if (c->batch_split) CUDA_TRY(cudaStreamSynchronize(c->cur));
     c->held_from = c->stage_off;
     std::vector<std::function<int()>> q;
     q.swap(c->held);
@@ -308,6 +310,7 @@ struct Batch {
     explicit Batch(hicma_tlr_ctx *ctx) : c(ctx), mine(!ctx->batching) {
         if (!mine) return;
         c->batching = true;
+        c->batch_split = false;
         c->held_from = c->stage_off;
     }
     int flush() { return mine ? issue_held(c) : 0; }
@@ -326,7 +329,10 @@ T *stage(hicma_tlr_ctx *c, const T *src, size_t n) {
     const size_t bytes = align_up(raw + 1);
     if (bytes > c->stage_bytes) return nullptr;
     if (c->stage_off + bytes > c->stage_bytes) {
-        if (c->batching && issue_held(c, true)) return nullptr;
+        if (c->batching) {
+            c->batch_split = true;
+            if (issue_held(c)) return nullptr;
+        }
         if (cudaStreamSynchronize(c->stream_hi) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream_core) != cudaSuccess) return nullptr;
         if (cudaStreamSynchronize(c->stream_side) != cudaSuccess) return nullptr;

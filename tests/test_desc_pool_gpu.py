@@ -1,5 +1,8 @@
 """Descriptor memory from the device's pool: reused regions are zero-filled, contexts
 on threads share the pool, the last context gives it back."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -8,6 +11,8 @@ import pytest
 from hicma_parsec_b200 import tlr
 
 pytestmark = pytest.mark.gpu
+
+REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("nt, nb, cap, band", [(1, 64, 8, 1), (3, 96, 40, 1), (4, 64, 16, 2)])
@@ -49,13 +54,20 @@ def test_threads_share_the_pool():
         assert out[q] == out["alone"]
 
 
+GIVES_BACK = """
+import torch
+from hicma_parsec_b200 import tlr
+keep = tlr.Context(0, 256 << 20)
+free0 = torch.cuda.mem_get_info(0)[0]
+tlr.TLRMatrix(keep, 8 * 2048, 2048, 2048, 1).close()     # 8 dense tiles + 28 full slots: 2.1 GB
+assert free0 - torch.cuda.mem_get_info(0)[0] >= 1 << 30  # kept for the next descriptor
+keep.close()
+torch.cuda.synchronize()
+assert torch.cuda.mem_get_info(0)[0] >= free0
+"""
+
+
 def test_last_context_gives_the_memory_back():
-    import torch
-    held = 1 << 30
-    keep = tlr.Context(0, 256 << 20)
-    free0 = torch.cuda.mem_get_info(0)[0]
-    tlr.TLRMatrix(keep, 8 * 2048, 2048, 2048, 1).close()     # 8 dense tiles + 28 full slots: 2.1 GB
-    assert free0 - torch.cuda.mem_get_info(0)[0] >= held     # kept for the next descriptor
-    keep.close()
-    torch.cuda.synchronize()
-    assert torch.cuda.mem_get_info(0)[0] >= free0
+    # in a process of its own: contexts of other tests share this process's pool
+    r = subprocess.run([sys.executable, "-c", GIVES_BACK], cwd=REPO, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
