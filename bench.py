@@ -441,7 +441,7 @@ def run_ours(args, cfg):
         return {f: sum(prof[n][f] for n in names) for f in ("launches", "seconds", "flops", "bytes")}
     kernels = {"k_gemm_batched": (agg([n for n in prof if n.startswith("gemm")]), "tensor"),
                "k_qr": (prof["qr"], "fp64"), "k_qapply": (prof["qapply"], "fp64"),
-               "k_core_svd": (prof["core_svd"], "fp64"), "k_bcgs2": (prof["proj"], "tensor"),
+               "core_svd": (prof["core_svd"], "fp64"), "projections": (prof["proj"], "tensor"),
                "k_copy_batched": (prof["copy"], "hbm"), "k_gram_batched": (prof["gram"], "tensor"),
                "k_rcholqr": (prof["rcholqr"], "tensor")}
     dom = max(kernels, key=lambda k: kernels[k][0]["seconds"])

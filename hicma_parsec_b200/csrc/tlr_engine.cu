@@ -353,7 +353,7 @@ enum {
     // batched DMMA GEMMs by call site (P_GEMM: recompression outputs and the rest)
     P_GEMM_Y, P_GEMM_TRSM, P_GEMM_SYRK, P_GEMM_DENSE, P_GEMM_GEN,
     P_GRAM,   // split-K inner products B_V^T A_V of the recompressions
-    P_CHOLQR,     // QR factors by randomized CholeskyQR
+    P_CHOLQR,     // QR factors by randomized CholeskyQR (the blocks of wider stacks: P_QR)
     P_NCLASS
 };
 static_assert(P_NCLASS <= 32, "two device counters per class in d_profacc");
@@ -609,7 +609,8 @@ int join_core(hicma_tlr_ctx *c, cudaStream_t st) {
     });
 }
 
-int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
+// cls: the profiling class, P_QR for the blocks of wide stacks.
+int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
     if (v.empty()) return 0;
 #ifdef TLR_BOUNDS_CHECK
     for (size_t i = 0; i < v.size(); ++i) {
@@ -623,7 +624,6 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
         if (t.Rinv) BC(t.Rinv, bc_span(K, K, K), "cholqr R3 inverse", i);
     }
 #endif
-    (void)kmax;
     // all tasks form Q or none does (the kernel is instantiated both ways)
     const bool form_q = v[0].Q != nullptr;
     for (auto &t : v)
@@ -682,7 +682,7 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int kmax) {
         const Launch l = ls[q];
         c->cur = spread && q + 1 < ls.size() ? c->stream_core : st;
         const int rc = issue(c, [=]() {
-            Prof pf(c, P_CHOLQR, l.fl, l.by);
+            Prof pf(c, cls, l.fl, l.by);
             launch_rcholqr_batched(l.d, l.n, l.hi, form_q, l.cluster, c->d_flags + 5, c->cur);
             return check_launch(c);
         });
@@ -941,10 +941,10 @@ int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
         if (q1.empty()) break;
         TRY(run_grams(c, g1, P_PROJ));
         TRY(run_gemms(c, u1, false, P_PROJ));
-        TRY(run_rcholqr(c, q1, 0));
+        TRY(run_rcholqr(c, q1, P_QR));
         TRY(run_grams(c, g2, P_PROJ));
         TRY(run_gemms(c, u2, false, P_PROJ));
-        TRY(run_rcholqr(c, q2, 0));
+        TRY(run_rcholqr(c, q2, P_QR));
         TRY(run_gemms(c, r2, false, P_PROJ));
     }
     v.clear();
@@ -1373,7 +1373,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             TRY(issue(c, [=]() { CUDA_TRY(cudaEventRecord(c->ev_join, c->stream_side)); return 0; }));
             c->cur = bulk;
         }
-        TRY(run_rcholqr(c, vrs, 0));
+        TRY(run_rcholqr(c, vrs));
         TRY(run_core_buckets(c, cores, cp));
         TRY(run_gemms(c, gTU));
         TRY(run_gemms(c, gU));
@@ -2373,7 +2373,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         }
         TRY(run_gemms(c, gy, false, P_GEMM_GEN));
         TRY(run_qr(c, qy, nb));
-        TRY(run_rcholqr(c, cqy, 0));
+        TRY(run_rcholqr(c, cqy));
         TRY(run_block_qr(c, bqy));
         if (!gq.empty()) {
             // Q^T Q of every formed Q, then the orthogonality flags of this sub-batch
@@ -2388,7 +2388,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         TRY(run_gemms(c, gw, false, P_GEMM_GEN));
         TRY(run_copies(c, keeps));
         TRY(run_qr(c, qw, nb));
-        TRY(run_rcholqr(c, cqw, 0));
+        TRY(run_rcholqr(c, cqw));
         TRY(run_block_qr(c, bqw));
         CoreParams cp{1, tol, maxrank, 0, nb, nullptr, nullptr};
         TRY(run_core_buckets(c, cores, cp));
