@@ -818,8 +818,8 @@ int run_gemms_narrow(hicma_tlr_ctx *c, std::vector<GemmTask> &v, int cls) {
     });
 }
 
-// Batched inner products P = C^T W of nb-long columns (split-K DMMA, one CTA
-// per product; k_gram_batched).
+// Batched inner products P = C^T W of nb-long columns (split-K DMMA, one CTA per
+// 32 x 32 block of a product; k_gram_batched).
 int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
     if (v.empty()) return 0;
 #ifdef TLR_BOUNDS_CHECK
@@ -1148,7 +1148,7 @@ int run_core_buckets(hicma_tlr_ctx *c, std::vector<CoreTask> &cores, const CoreP
 
 // Recompression of a batch of low-rank updates C = [Cu Au][Cv -Y]^T.
 // Both stacks get a QR: up to rcholqr_kmax() columns by the randomized
-// CholeskyQR in one CTA, wider ones by block Gram-Schmidt (run_block_qr).  There
+// CholeskyQR, wider ones by block Gram-Schmidt (run_block_qr).  There
 // the old U is orthonormal, so on that side only the new columns are factored,
 // R_U = [[I, P], [0, R]]; the old V = V Sigma is orthogonal only up to the core
 // solver's tolerance relative to its largest singular value, which is not enough
@@ -1165,7 +1165,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
     while (i0 < tasks.size()) {
         c->ar->off = mark;
         // common prefix (Y products, V-side stacks) on the bulk stream; then the
-        // CholeskyQR chain (F) there and the Householder chain of the wide
+        // CholeskyQR chain (F) there and the block Gram-Schmidt chain of the wide
         // updates (S) on the side stream, joined at the end of the chunk
         std::vector<CopyTask> copies, copiesS, keeps;
         std::vector<GemmTask> g1, g2, g1s, g2s, gTU, gU, g3, g4, gUS, g3S, g4S;
