@@ -36,7 +36,10 @@
 // 16-column blocks, one pair per CTA and round (Gram product and the product
 // with the accumulated rotations on DMMA, the rotations of the 32 x 32 Gram
 // matrix in shared memory).
+#include "core_layout.h"
 #include "tlr_internal.h"
+
+#include <algorithm>
 
 #include <cooperative_groups.h>
 
@@ -529,17 +532,6 @@ __global__ void __launch_bounds__(4 * KM) k_core_small(const CoreTask *__restric
 // One core of K = 96, 256, 400: 0.52, 2.4, 9.0 ms.  Two launches of three cores and
 // one of K about 650 (k about 430): 470 -> 32 ms against one warp per column pair
 // reading its columns through L2.
-constexpr int WB = 16;                        // columns of a block
-constexpr int WP = 2 * WB;                    // columns of a pair problem
-constexpr int WLD = WP + 4;                   // pitch of its J (conflict-free DMMA fragments)
-constexpr int WGD = WP + 1;                   // pitch of its G (rows and columns read alike)
-constexpr int W_CT = 256;
-constexpr int W_NW = W_CT / 32;
-constexpr int W_TILES = 10;                   // lower 8 x 8 tiles of the 32 x 32 Gram matrix
-constexpr int W_CSMAX = 16;
-constexpr size_t W_JACOBI_DOUBLES = 2 * WP * WLD + W_NW * W_TILES * 64;
-constexpr size_t W_SMEM_MAX = 220 * 1024;
-
 __device__ __forceinline__ double ldg2(const double *p) { return __ldcg(p); }
 __device__ __forceinline__ int ldg2(const int *p) { return __ldcg(p); }
 
@@ -548,10 +540,9 @@ struct WidePub {
     int col, pad;
 };
 
-// columns of T a CTA holds
-__host__ __device__ __forceinline__ int wide_ncl(int K, int cs) { return (K + cs - 1) / cs; }
-
-__global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__ tasks, CoreParams p, int t_in_smem) {
+// HV: the pivot column is in shared memory (W_HV_SHARED)
+template <bool HV>
+__global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__ tasks, CoreParams p, int place) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) double sm[];
@@ -573,17 +564,16 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
         }
         return;
     }
-    // task scratch: X (K x (K + 32)), sigma, T when it does not fit, flags
-    double *X = t.work;
-    double *sig = X + (size_t)K * (K + WP);
-    double *Tg = sig + K;
-    int *rotf = (int *)(Tg + (size_t)K * (K + W_CSMAX));  // [sweep]: a pair was rotated
+    const bool t_in_smem = place & W_T_SHARED;
+    const WideLayout L = wide_layout(K, CS, crank, place);
+    double *X = t.work + L.X;
+    double *sig = t.work + L.sig;
+    int *rotf = (int *)(t.work + L.flags);    // [sweep]: a pair was rotated
     const int ncl = wide_ncl(K, CS), lcs = __ffs(CS) - 1;   // CS is a power of two
-    double *hv = sm;                          // K
-    double *sigl = hv + K;                    // ncl: squared norms of the CTA's columns, -1 once pivots
-    double *Ts = sigl + ncl + ((K + ncl) & 1);
+    double *sigl = sm + L.sigl;               // squared norms of the CTA's columns, -1 once pivots
+    double *hv = (HV ? sm : t.work) + L.hv;   // the pivot column
+    double *Tl = (t_in_smem ? sm : t.work) + L.T;   // the CTA's columns of T
     const int nc = crank < K ? (K - crank + CS - 1) / CS : 0;   // columns this CTA holds
-    double *Tl = t_in_smem ? Ts : Tg + (size_t)crank * ncl * K;
 
     if (gt < 64) rotf[gt] = 0;
     // 1. the CTA's columns of T = M^T: T(i, c) = sum_{l >= max(i, c)} RU(c, l) RV(i, l);
@@ -680,10 +670,10 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
         n2 = pub[par][owner].norm;
         const double sn = sqrt(n2);
         if (t_in_smem) {
-            const double *src = cl.map_shared_rank(Ts, owner) + (size_t)lp * K;
+            const double *src = cl.map_shared_rank(Tl, owner) + (size_t)lp * K;
             for (int r = j + tid; r < K; r += W_CT) hv[r] = src[r];
         } else {
-            const double *src = Tg + ((size_t)owner * ncl + lp) * K;
+            const double *src = Tl + ((ptrdiff_t)(owner - crank) * ncl + lp) * K;
             for (int r = j + tid; r < K; r += W_CT) hv[r] = ldg2(src + r);
         }
         __syncthreads();
@@ -736,6 +726,7 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
         }
         __syncthreads();
     }
+    if (!HV) cl.sync();                       // hv lies in columns that are zeroed now
     // blocks past k: zero columns
     const int nblk = max(2, (k + WB - 1) / WB), nbp = nblk + (nblk & 1);
     for (long long idx = (long long)k * K + gt; idx < (long long)nblk * WB * K && idx < (long long)K * (K + WP); idx += GT)
@@ -872,8 +863,9 @@ __global__ void __launch_bounds__(W_CT) k_core_wide(const CoreTask *__restrict__
         if (lane == 0) sig[c] = sqrt(s);
     }
     cl.sync();
-    // every CTA orders them and finds the rank (one reports it)
-    double *sg = sm;
+    // every CTA orders them (in T's place, where that is free) and finds the rank (one
+    // reports it)
+    double *sg = (t_in_smem ? sm : t.work) + L.sort;
     int *order = (int *)(sg + K);
     int nge = 0;
     for (int c0 = 0; c0 < k; c0 += W_CT) {
@@ -924,17 +916,6 @@ void launch_small(const CoreTask *d, int n, const CoreParams &p, cudaStream_t st
     k_core_small<KM><<<n, S::NT, S::bytes, st>>>(d, p);
 }
 
-size_t wide_smem(int K, int cs, bool t_in_smem) {
-    const size_t ncl = wide_ncl(K, cs);
-    const size_t qr = (size_t)K + ncl + 1 + (t_in_smem ? ncl * K : 0);
-    return sizeof(double) * (qr > W_JACOBI_DOUBLES ? qr : W_JACOBI_DOUBLES);
-}
-
-// CTAs of a cluster: about one per pair problem of the Jacobi rounds (k / 32
-// pairs, k about K / 2) and enough shared memory for T: 4 up to K = 160, 8 up
-// to 448, then 16 (the non-portable maximum).
-int wide_cluster(int K) { return K <= 160 ? 4 : K <= 448 ? 8 : W_CSMAX; }
-
 }  // namespace
 
 // One CTA beats a cluster at any width when the launch fills the device, but its
@@ -942,7 +923,7 @@ int wide_cluster(int K) { return K <= 160 ? 4 : K <= 448 ? 8 : W_CSMAX; }
 // 65 to SMALL_KMAX columns take either kernel, so they bring scratch.
 int core_smem_kmax() { return 64; }
 
-size_t core_work_doubles(int K) { return (size_t)K * (K + WP) + (size_t)K * (K + W_CSMAX) + (size_t)K + 64; }
+size_t core_work_doubles(int K) { return wide_work_doubles(K); }
 
 int core_bucket(int K, bool cluster) {
     if (K <= 64) return K <= 16 ? 16 : K <= 32 ? 32 : K <= 48 ? 48 : 64;
@@ -952,7 +933,7 @@ int core_bucket(int K, bool cluster) {
 int core_one_cta_kmax() { return SMALL_KMAX; }
 
 void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p, bool cluster,
-                             cudaStream_t st) {
+                             size_t smem_limit, cudaStream_t st) {
     if (ntasks <= 0) return;
     if (kmax <= 16) return launch_small<16>(d_tasks, ntasks, p, st);
     if (kmax <= 32) return launch_small<32>(d_tasks, ntasks, p, st);
@@ -962,11 +943,11 @@ void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, cons
     if (kmax <= SMALL_KMAX && !cluster) return launch_small<96>(d_tasks, ntasks, p, st);
     int cs = wide_cluster(kmax);
     for (;;) {
-    // T in the cluster's shared memory where a CTA's share fits
-        const bool in_smem = wide_smem(kmax, cs, true) <= W_SMEM_MAX;
-        const size_t smem = wide_smem(kmax, cs, in_smem);
-        cudaFuncSetAttribute(k_core_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(k_core_wide, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        const int place = wide_place(kmax, cs, std::min(smem_limit, W_SMEM_MAX));
+        const size_t smem = wide_smem(kmax, cs, place);
+        auto *kernel = place & W_HV_SHARED ? k_core_wide<true> : k_core_wide<false>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ntasks * cs);
         cfg.blockDim = dim3(W_CT);
@@ -982,13 +963,13 @@ void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, cons
         if (cs > 8) {
             // 16 CTAs need a GPC with that many SMs free: take 8 where none has them
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, k_core_wide, &cfg) != cudaSuccess || n < 1) {
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
                 cudaGetLastError();
                 cs = 8;
                 continue;
             }
         }
-        cudaLaunchKernelEx(&cfg, k_core_wide, d_tasks, p, in_smem ? 1 : 0);
+        cudaLaunchKernelEx(&cfg, kernel, d_tasks, p, place);
         return;
     }
 }

@@ -155,6 +155,7 @@ struct hicma_tlr_ctx_s {
     // ranks up to rcholqr_kmax() and the generation range finder up to that many samples
     // (1), the Householder pipeline for all (0; HICMA_TLR_QR=householder)
     int cholqr = 1;
+    size_t core_smem = (size_t)-1;   // shared memory limit of the wide core SVD (HICMA_TLR_CORE_SMEM, bytes)
     double *d_scal = nullptr;   // device scalars
     double *d_profacc = nullptr;   // per profiling class: flops, bytes counted on the device
     int precision = HICMA_TLR_PREC_FP64;
@@ -718,7 +719,7 @@ int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CorePar
     v.clear();
     return issue(c, [=]() {
         Prof pf(c, P_CORE, 0, 0);
-        launch_core_svd_batched(d, n, std::max(kmax, 1), cp, cluster, c->cur);
+        launch_core_svd_batched(d, n, std::max(kmax, 1), cp, cluster, c->core_smem, c->cur);
         return check_launch(c);
     });
 }
@@ -1755,6 +1756,7 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
     if (e != cudaSuccess) return fail(e, "side stream");
     c->cur = c->stream;
     if (const char *q = std::getenv("HICMA_TLR_QR")) c->cholqr = std::strcmp(q, "householder") != 0;
+    if (const char *q = std::getenv("HICMA_TLR_CORE_SMEM")) c->core_smem = (size_t)std::strtoull(q, nullptr, 10);
     size_t free_b = 0, total_b = 0;
     e = cudaMemGetInfo(&free_b, &total_b);
     if (e != cudaSuccess) return fail(e, "memory info");

@@ -314,8 +314,9 @@ size_t core_work_doubles(int K);
 int core_bucket(int K, bool cluster);
 int core_one_cta_kmax();
 // All tasks of one launch have K <= kmax; kernel and shared memory are chosen from kmax.
+// smem_limit: bytes of shared memory a cluster's CTA may take for its pivoted QR.
 void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, const CoreParams &p, bool cluster,
-                             cudaStream_t st);
+                             size_t smem_limit, cudaStream_t st);
 
 // ---------------------------------------------------------------- misc ------
 // sum of 2*log(diag) over n diagonal entries of ntiles tiles, into *out
