@@ -281,11 +281,16 @@ size_t qr_smem(int m) { return sizeof(double) * ((size_t)PB * m + QW_MAX * PB + 
 template <int PB>
 constexpr int qr_threads() { return PB <= 16 ? 512 : 256; }
 
+// The dynamic shared memory limit belongs to the function, for all threads of the
+// process: always the most a block can have, so that a launch of another context with
+// shorter stacks never lowers it in between.
+constexpr int QR_SMEM_LIMIT = 227 * 1024;
+
 template <int PB>
 void launch_qr_pb(const QRTask *d_tasks, int ntasks, int m_max, cudaStream_t st) {
     const size_t smem = qr_smem<PB>(m_max);
     constexpr int T = qr_threads<PB>();
-    cudaFuncSetAttribute(k_qr<PB, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_qr<PB, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, QR_SMEM_LIMIT);
     k_qr<PB, T><<<ntasks, T, smem, st>>>(d_tasks);
 }
 
@@ -293,7 +298,7 @@ template <int PB>
 void launch_qapply_pb(const QApplyTask *d_tasks, int ntasks, int m_max, cudaStream_t st) {
     const size_t smem = sizeof(double) * ((size_t)PB * m_max + PB * PB);
     constexpr int T = qr_threads<PB>();
-    cudaFuncSetAttribute(k_qapply<PB, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_qapply<PB, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, QR_SMEM_LIMIT);
     k_qapply<PB, T><<<ntasks, T, smem, st>>>(d_tasks);
 }
 

@@ -946,7 +946,9 @@ void launch_core_svd_batched(const CoreTask *d_tasks, int ntasks, int kmax, cons
         const int place = wide_place(kmax, cs, std::min(smem_limit, W_SMEM_MAX));
         const size_t smem = wide_smem(kmax, cs, place);
         auto *kernel = place & W_HV_SHARED ? k_core_wide<true> : k_core_wide<false>;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the limit belongs to the function, for all threads of the process: always the same
+        // value, so that a launch of another context never lowers it in between
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W_SMEM_MAX);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ntasks * cs);
