@@ -11,6 +11,7 @@
 // write disjoint tiles), so batching them preserves the reference's data
 // flow.  The host reads the rank map once per panel (the sizes of the next
 // panel's tasks depend on the ranks the recompressions produced).
+#include "staging.h"
 #include "tlr_internal.h"
 
 #include <nvtx3/nvToolsExt.h>
@@ -139,12 +140,19 @@ struct hicma_tlr_ctx_s {
     size_t ws_bytes = 0;
     Arena main_ar, hi_ar;               // workspace of `stream` / `stream_hi`
     Arena *ar = nullptr;                // arena of `cur`
-    char *h_stage = nullptr, *d_stage = nullptr;
-    size_t stage_bytes = 0, stage_off = 0;
-    bool batching = false;                          // launches wait for one upload of their tasks (Batch)
-    bool batch_split = false;                       // the ring wrapped inside the Batch: part of it is launched
-    size_t held_from = 0;                           // staged bytes from here on are not uploaded yet
-    std::vector<std::function<int()>> held;         // the launches, in order
+    Ring ring;                          // task arrays on their way to the device
+    int ring_upload(size_t off, size_t n) {
+        CUDA_TRY(cudaMemcpyAsync(ring.d + off, ring.h + off, n, cudaMemcpyHostToDevice, cur));
+        return 0;
+    }
+    int ring_wait_current() {
+        CUDA_TRY(cudaStreamSynchronize(cur));
+        return 0;
+    }
+    int ring_wait_all() {
+        for (cudaStream_t st : {stream_hi, stream_core, stream_side, stream}) CUDA_TRY(cudaStreamSynchronize(st));
+        return 0;
+    }
     int *d_flags = nullptr;     // [0] info, [1] overflow, [2] Jacobi sweeps, [3] wait timed out, [4] FP32 updates,
                                 // [5] CholeskyQR null pivots, [6] CholeskyQR passes repeated
     int nsm = 148;              // SM count of the device
@@ -221,7 +229,7 @@ int ctx_sync(hicma_tlr_ctx *c) {
     CUDA_TRY(cudaStreamSynchronize(c->stream_side));
     CUDA_TRY(cudaStreamSynchronize(c->stream_copy));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
-    c->stage_off = 0;
+    c->ring.off = 0;
     return 0;
 }
 
@@ -270,84 +278,7 @@ struct OnHi {
     ~OnHi() { c->cur = c->stream; c->ar = &c->main_ar; }
 };
 
-// Uploads what is staged on the current stream and makes the held launches.  Other
-// streams join the current one by an event held among them, so after the upload; once
-// a part of the Batch with such an event is launched, the host waits for the upload.
-int issue_held(hicma_tlr_ctx *c) {
-    if (c->stage_off > c->held_from)
-        CUDA_TRY(cudaMemcpyAsync(c->d_stage + c->held_from, c->h_stage + c->held_from, c->stage_off - c->held_from,
-                                 cudaMemcpyHostToDevice, c->cur));
-    if (c->batch_split) CUDA_TRY(cudaStreamSynchronize(c->cur));
-    c->held_from = c->stage_off;
-    std::vector<std::function<int()>> q;
-    q.swap(c->held);
-    cudaStream_t st = c->cur;
-    int rc = 0;
-    for (size_t i = 0; i < q.size() && !rc; ++i) rc = q[i]();
-    c->cur = st;
-    return rc;
-}
-
-// A launch (or an event call) on the current stream: made now, or held inside a Batch.
-template <class F>
-int issue(hicma_tlr_ctx *c, F f) {
-    if (!c->batching) return f();
-    cudaStream_t st = c->cur;
-    c->held.push_back([c, st, f]() {
-        c->cur = st;
-        return f();
-    });
-    return 0;
-}
-
-// While a Batch lives, the helpers stage their task arrays and hold their launches;
-// flush() uploads all arrays in one copy on the current stream, then launches.  A copy
-// per launch sits in the stream before it: 3 us of copy and 6 us of gaps to a launch of
-// 20 to 200 us in the chains of a late panel.  One copy a batch: 2D requests of 27,000
-// and 97,200 unknowns 77.3, 314 ms -> 73.3, 299; 60 x 60 tiles 390 -> 377.
-struct Batch {
-    hicma_tlr_ctx *c;
-    bool mine;
-    explicit Batch(hicma_tlr_ctx *ctx) : c(ctx), mine(!ctx->batching) {
-        if (!mine) return;
-        c->batching = true;
-        c->batch_split = false;
-        c->held_from = c->stage_off;
-    }
-    int flush() { return mine ? issue_held(c) : 0; }
-    ~Batch() {
-        if (!mine) return;
-        c->held.clear();       // left only by an error
-        c->batching = false;
-    }
-    Batch(const Batch &) = delete;
-    Batch &operator=(const Batch &) = delete;
-};
-
-template <class T>
-T *stage(hicma_tlr_ctx *c, const T *src, size_t n) {
-    const size_t raw = n * sizeof(T);
-    const size_t bytes = align_up(raw + 1);
-    if (bytes > c->stage_bytes) return nullptr;
-    if (c->stage_off + bytes > c->stage_bytes) {
-        if (c->batching) {
-            c->batch_split = true;
-            if (issue_held(c)) return nullptr;
-        }
-        if (cudaStreamSynchronize(c->stream_hi) != cudaSuccess) return nullptr;
-        if (cudaStreamSynchronize(c->stream_core) != cudaSuccess) return nullptr;
-        if (cudaStreamSynchronize(c->stream_side) != cudaSuccess) return nullptr;
-        if (cudaStreamSynchronize(c->stream) != cudaSuccess) return nullptr;
-        c->stage_off = c->held_from = 0;
-    }
-    std::memcpy(c->h_stage + c->stage_off, src, raw);
-    if (!c->batching && cudaMemcpyAsync(c->d_stage + c->stage_off, c->h_stage + c->stage_off, raw,
-                                        cudaMemcpyHostToDevice, c->cur) != cudaSuccess)
-        return nullptr;
-    T *d = (T *)(c->d_stage + c->stage_off);
-    c->stage_off += bytes;
-    return d;
-}
+using Batch = BatchOf<hicma_tlr_ctx>;
 
 enum {
     P_GEMM = 0, P_QR, P_QAPPLY, P_CORE, P_POTRF, P_COV, P_COPY, P_OTHER, P_PROJ,
@@ -638,8 +569,8 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
     // Few matrices share clusters of CTAs while those fit three quarters of the SMs
     // (the tile POTRF holds the others).
     struct Launch {
-        CQTask *d;
-        int n, hi, cluster;
+        std::vector<CQTask> tasks;
+        int hi, cluster;
         double fl, by;
     };
     std::vector<Launch> ls;
@@ -656,8 +587,6 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
         if (b.empty()) continue;
         if (next && 2 * (b.size() + next) <= (size_t)c->nsm) continue;
         const int cap = c->nsm * 3 / 4, cluster = 4 * (int)b.size() <= cap ? 4 : 2 * (int)b.size() <= cap ? 2 : 1;
-        CQTask *d = stage(c, b.data(), b.size());
-        if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
         double fl = 0, by = 0;
         for (auto &t : b) {
             // the sketch (nb K FMAs); shifted CholeskyQR3 of the 256 sketch rows (three Gram
@@ -669,7 +598,7 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
             // X read twice; Y written when kept; Y read and Q written when Q is formed
             by += 8.0 * t.nb * K * (t.plain ? 3.0 : 2.0 + (t.Q || t.Rinv ? 1.0 : 0.0) + (t.Q ? 2.0 : 0.0));
         }
-        ls.push_back({d, (int)b.size(), hi, cluster, fl, by});
+        ls.push_back({std::move(b), hi, cluster, fl, by});
         b.clear();
     }
     v.clear();
@@ -680,11 +609,15 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
     cudaStream_t st = c->cur;
     if (spread) TRY(fork_core(c, st));
     for (size_t q = ls.size(); q-- > 0;) {
-        const Launch l = ls[q];
+        const Launch &l = ls[q];
         c->cur = spread && q + 1 < ls.size() ? c->stream_core : st;
+        CQTask *d = stage(c, l.tasks.data(), l.tasks.size());
+        if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
+        const int n = (int)l.tasks.size(), hi = l.hi, cluster = l.cluster;
+        const double fl = l.fl, by = l.by;
         const int rc = issue(c, [=]() {
-            Prof pf(c, cls, l.fl, l.by);
-            launch_rcholqr_batched(l.d, l.n, l.hi, form_q, l.cluster, c->d_flags + 5, c->cur);
+            Prof pf(c, cls, fl, by);
+            launch_rcholqr_batched(d, n, hi, form_q, cluster, c->d_flags + 5, c->cur);
             return check_launch(c);
         });
         c->cur = st;
@@ -775,9 +708,9 @@ int run_gemms(hicma_tlr_ctx *c, std::vector<GemmTask> &v, bool fp32 = false, int
     for (size_t i = 0; i < v.size(); ++i) off[i + 1] = off[i] + gemm_tiles(v[i]);
     if (off.back() == 0) { v.clear(); return 0; }
     gemm_groups(off);
-    GemmTask *dt = stage(c, v.data(), v.size());
-    int *doff = stage(c, off.data(), off.size());
-    if (!dt || !doff) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
+    GemmTask *dt;
+    int *doff;
+    if (!stage_both(c, v, off, &dt, &doff)) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
     double fl = 0, by = 0;
     bool ndev = gemm_work(v, fl, by);
     const int n = (int)v.size(), tiles = off[v.size()];
@@ -802,9 +735,9 @@ int run_gemms_narrow(hicma_tlr_ctx *c, std::vector<GemmTask> &v, int cls) {
     }
     if (off.back() == 0) { v.clear(); return 0; }
     gemm_groups(off);
-    GemmTask *dt = stage(c, v.data(), v.size());
-    int *doff = stage(c, off.data(), off.size());
-    if (!dt || !doff) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
+    GemmTask *dt;
+    int *doff;
+    if (!stage_both(c, v, off, &dt, &doff)) { set_err("task staging failed"); return HICMA_TLR_ERR_CUDA; }
     double fl = 0, by = 0;
     bool ndev = gemm_work(v, fl, by);
     const int n = (int)v.size(), tiles = off[v.size()];
@@ -1706,13 +1639,13 @@ static void ctx_release(hicma_tlr_ctx *c) {
     }
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
     bc_remove(c->d_ws);
-    bc_remove(c->d_stage);
+    bc_remove(c->ring.d);
     bc_remove(c->d_flags);
     bc_remove(c->d_scal);
     if (c->pool) pool_release(c->device);
     if (c->d_ws) cudaFree(c->d_ws);
-    if (c->d_stage) cudaFree(c->d_stage);
-    if (c->h_stage) cudaFreeHost(c->h_stage);
+    if (c->ring.d) cudaFree(c->ring.d);
+    if (c->ring.h) cudaFreeHost(c->ring.h);
     if (c->d_flags) cudaFree(c->d_flags);
     if (c->d_scal) cudaFree(c->d_scal);
     if (c->d_profacc) cudaFree(c->d_profacc);
@@ -1781,15 +1714,16 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
         c->main_ar.bytes = c->ws_bytes - hi;
         c->ar = &c->main_ar;
     }
-    c->stage_bytes = (size_t)64 << 20;
-    if ((e = cudaMallocHost(&c->h_stage, c->stage_bytes)) != cudaSuccess) { c->h_stage = nullptr; return fail(e, "pinned staging"); }
-    if ((e = cudaMalloc(&c->d_stage, c->stage_bytes)) != cudaSuccess) { c->d_stage = nullptr; return fail(e, "device staging"); }
+    c->ring.bytes = (size_t)64 << 20;
+    if (const char *q = std::getenv("HICMA_TLR_STAGE_BYTES")) c->ring.bytes = std::max(std::strtoull(q, nullptr, 10), 4096ull) / 256 * 256;
+    if ((e = cudaMallocHost(&c->ring.h, c->ring.bytes)) != cudaSuccess) { c->ring.h = nullptr; return fail(e, "pinned staging"); }
+    if ((e = cudaMalloc(&c->ring.d, c->ring.bytes)) != cudaSuccess) { c->ring.d = nullptr; return fail(e, "device staging"); }
     if ((e = cudaMalloc(&c->d_flags, 64 * sizeof(int))) != cudaSuccess) { c->d_flags = nullptr; return fail(e, "flags"); }
     if ((e = cudaMalloc(&c->d_scal, 64 * sizeof(double))) != cudaSuccess) { c->d_scal = nullptr; return fail(e, "scalars"); }
     if ((e = cudaMalloc(&c->d_profacc, 64 * sizeof(double))) != cudaSuccess) { c->d_profacc = nullptr; return fail(e, "profiling counters"); }
     if ((e = xclear(c, c->d_profacc, 64 * sizeof(double))) != cudaSuccess) return fail(e, "profiling counters reset");
     bc_add(c->d_ws, c->ws_bytes);
-    bc_add(c->d_stage, c->stage_bytes);
+    bc_add(c->ring.d, c->ring.bytes);
     bc_add(c->d_flags, 64 * sizeof(int));
     bc_add(c->d_scal, 64 * sizeof(double));
     if ((e = xclear(c, c->d_flags, 64 * sizeof(int))) != cudaSuccess) return fail(e, "flags reset");
@@ -3500,7 +3434,7 @@ static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, 
     }
 #endif
     // staged in pieces of whole steps where the ring is too small for all of them
-    const size_t cap = c->stage_bytes / 2 / sizeof(SkinnyTask);
+    const size_t cap = c->ring.bytes / 2 / sizeof(SkinnyTask);
     for (size_t s = 0; s < steps.size();) {
         size_t e = s, cnt = 0;
         while (e < steps.size() && (e == s || cnt + steps[e].cnt <= cap)) cnt += steps[e++].cnt;
@@ -3817,7 +3751,7 @@ int hicma_tlr_check(hicma_tlr_ctx *c, hicma_tlr_desc *L, const hicma_tlr_problem
     }
     cudaError_t e = cudaMemcpyAsync(h, sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    c->stage_off = 0;
+    c->ring.off = 0;
     cleanup();
     if (e != cudaSuccess) { set_err("check: %s", cudaGetErrorString(e)); return HICMA_TLR_ERR_CUDA; }
     if (res_llt) *res_llt = std::sqrt(h[1]) / std::sqrt(h[0]);
