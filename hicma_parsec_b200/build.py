@@ -30,7 +30,7 @@ SOURCES = ["k_gemm.cu", "k_tile.cu", "k_potrf.cu", "k_potrf_tile.cu", "k_qr.cu",
            "k_rcholqr_c4.cu", "k_proj.cu", "k_svd.cu",
            "k_skinny.cu",
            "tlr_engine.cu", "serve.cu"]
-HEADERS = ["tlr_internal.h", "core_layout.h", "staging.h"]
+HEADERS = ["tlr_internal.h", "core_layout.h", "regions.h", "staging.h"]
 INCLUDED = {"k_rcholqr_c2.cu": "k_rcholqr.cu", "k_rcholqr_c4.cu": "k_rcholqr.cu"}   # sources that include another
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -836,7 +836,7 @@ const ItemList *get_items(int nblk, bool inv, cudaStream_t st) {
     if (f != g_items.end()) return &f->second;
     std::vector<PItem> h = build_items(nblk, inv);
     ItemList L;
-    if (cudaMalloc(&L.d, h.size() * sizeof(PItem)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (device_malloc((void **)&L.d, h.size() * sizeof(PItem))) return nullptr;
     // ordered on the launch stream and complete before the list is used (a
     // legacy-stream copy from pageable memory may land after the kernel reads it)
     if (cudaMemcpyAsync(L.d, h.data(), h.size() * sizeof(PItem), cudaMemcpyHostToDevice, st) != cudaSuccess ||

@@ -11,6 +11,7 @@
 // write disjoint tiles), so batching them preserves the reference's data
 // flow.  The host reads the rank map once per panel (the sizes of the next
 // panel's tasks depend on the ranks the recompressions produced).
+#include "regions.h"
 #include "staging.h"
 #include "tlr_internal.h"
 
@@ -24,6 +25,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <set>
@@ -120,6 +122,33 @@ struct BcScope {
         }                                         \
     } while (0)
 
+// ----------------------------------------------------------- device memory ---
+struct CudaRegions {
+    static int alloc(void **p, size_t bytes) {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+        return (int)e;
+    }
+    static bool is_oom(int e) { return e == (int)cudaErrorMemoryAllocation; }
+    static void release(void *p) { cudaFree(p); }
+};
+using DeviceRegions = Regions<CudaRegions>;
+
+// The regions of a device, for the life of the process.
+static DeviceRegions *device_regions(int device) {
+    static std::mutex mu;
+    static auto *all = new std::map<int, DeviceRegions>();
+    std::lock_guard<std::mutex> lk(mu);
+    return &(*all)[device];
+}
+
+// cudaMalloc on the current device that gets what destroyed descriptors left.
+int tlr::device_malloc(void **p, size_t bytes) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return device_regions(dev)->alloc(p, bytes);
+}
+
 // --------------------------------------------------------------- context ---
 struct Arena {
     char *base = nullptr;
@@ -135,7 +164,7 @@ struct hicma_tlr_ctx_s {
     cudaStream_t stream_copy = nullptr; // copy-out of final factor columns during a factorization
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t cur = nullptr;         // stream the helpers launch on
-    cudaMemPool_t pool = nullptr;       // matrix storage of the descriptors (the device's pool)
+    DeviceRegions *regions = nullptr;   // matrix storage of the descriptors (shared by the device's contexts)
     char *d_ws = nullptr;
     size_t ws_bytes = 0;
     Arena main_ar, hi_ar;               // workspace of `stream` / `stream_hi`
@@ -1586,49 +1615,6 @@ int hicma_tlr_points_mesh(const hicma_tlr_problem *prob, const char *mesh_file, 
     return 0;
 }
 
-// Memory pool of a device for the matrix storage of all its contexts.  It keeps up to
-// an eighth of the device, 16 GiB at most, of what destroyed descriptors held for the
-// next ones; it gives that back when an allocation fails and with the last context.
-struct DevicePool {
-    cudaMemPool_t pool = nullptr;
-    int users = 0;
-};
-static std::mutex pools_mu;
-static std::map<int, DevicePool> pools;
-
-static cudaError_t pool_acquire(int device, size_t device_bytes, cudaMemPool_t *out) {
-    std::lock_guard<std::mutex> lk(pools_mu);
-    DevicePool &d = pools[device];
-    if (!d.pool) {
-        cudaMemPoolProps pp = {};
-        pp.allocType = cudaMemAllocationTypePinned;
-        pp.location.type = cudaMemLocationTypeDevice;
-        pp.location.id = device;
-        cudaMemPool_t p = nullptr;
-        cudaError_t e = cudaMemPoolCreate(&p, &pp);
-        if (e != cudaSuccess) return e;
-        unsigned long long keep = std::min<size_t>(device_bytes / 8, (size_t)16 << 30);
-        e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) {
-            cudaMemPoolDestroy(p);
-            return e;
-        }
-        d.pool = p;
-    }
-    ++d.users;
-    *out = d.pool;
-    return cudaSuccess;
-}
-
-static void pool_release(int device) {
-    std::lock_guard<std::mutex> lk(pools_mu);
-    DevicePool &d = pools[device];
-    if (--d.users == 0) {
-        cudaMemPoolDestroy(d.pool);   // regions still in use stay until they are freed
-        d.pool = nullptr;
-    }
-}
-
 // Releases whatever a context holds (also a partly built one from init).
 static void ctx_release(hicma_tlr_ctx *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
@@ -1642,7 +1628,7 @@ static void ctx_release(hicma_tlr_ctx *c) {
     bc_remove(c->ring.d);
     bc_remove(c->d_flags);
     bc_remove(c->d_scal);
-    if (c->pool) pool_release(c->device);
+    if (c->regions) c->regions->leave();
     if (c->d_ws) cudaFree(c->d_ws);
     if (c->ring.d) cudaFree(c->ring.d);
     if (c->ring.h) cudaFreeHost(c->ring.h);
@@ -1693,13 +1679,17 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
     size_t free_b = 0, total_b = 0;
     e = cudaMemGetInfo(&free_b, &total_b);
     if (e != cudaSuccess) return fail(e, "memory info");
-    if ((e = pool_acquire(device, total_b, &c->pool)) != cudaSuccess) { c->pool = nullptr; return fail(e, "memory pool"); }
+    // an eighth of a device's memory, 8 GiB at most, is kept for the next descriptors
+    c->regions = device_regions(device);
+    c->regions->enter(std::min<size_t>(total_b / 8, (size_t)8 << 30));
+    free_b += c->regions->held();
     if (workspace_bytes == 0) {
         workspace_bytes = std::min<size_t>(free_b / 8, (size_t)8 << 30);
         workspace_bytes = std::max<size_t>(workspace_bytes, (size_t)256 << 20);
     }
     c->ws_bytes = workspace_bytes;
-    e = cudaMalloc(&c->d_ws, c->ws_bytes);
+    auto dmalloc = [&](void *pp, size_t n) { return (cudaError_t)device_malloc((void **)pp, n); };
+    e = dmalloc(&c->d_ws, c->ws_bytes);
     if (e != cudaSuccess) {
         c->d_ws = nullptr;
         char what[96];
@@ -1717,10 +1707,10 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
     c->ring.bytes = (size_t)64 << 20;
     if (const char *q = std::getenv("HICMA_TLR_STAGE_BYTES")) c->ring.bytes = std::max(std::strtoull(q, nullptr, 10), 4096ull) / 256 * 256;
     if ((e = cudaMallocHost(&c->ring.h, c->ring.bytes)) != cudaSuccess) { c->ring.h = nullptr; return fail(e, "pinned staging"); }
-    if ((e = cudaMalloc(&c->ring.d, c->ring.bytes)) != cudaSuccess) { c->ring.d = nullptr; return fail(e, "device staging"); }
-    if ((e = cudaMalloc(&c->d_flags, 64 * sizeof(int))) != cudaSuccess) { c->d_flags = nullptr; return fail(e, "flags"); }
-    if ((e = cudaMalloc(&c->d_scal, 64 * sizeof(double))) != cudaSuccess) { c->d_scal = nullptr; return fail(e, "scalars"); }
-    if ((e = cudaMalloc(&c->d_profacc, 64 * sizeof(double))) != cudaSuccess) { c->d_profacc = nullptr; return fail(e, "profiling counters"); }
+    if ((e = dmalloc(&c->ring.d, c->ring.bytes)) != cudaSuccess) { c->ring.d = nullptr; return fail(e, "device staging"); }
+    if ((e = dmalloc(&c->d_flags, 64 * sizeof(int))) != cudaSuccess) { c->d_flags = nullptr; return fail(e, "flags"); }
+    if ((e = dmalloc(&c->d_scal, 64 * sizeof(double))) != cudaSuccess) { c->d_scal = nullptr; return fail(e, "scalars"); }
+    if ((e = dmalloc(&c->d_profacc, 64 * sizeof(double))) != cudaSuccess) { c->d_profacc = nullptr; return fail(e, "profiling counters"); }
     if ((e = xclear(c, c->d_profacc, 64 * sizeof(double))) != cudaSuccess) return fail(e, "profiling counters reset");
     bc_add(c->d_ws, c->ws_bytes);
     bc_add(c->ring.d, c->ring.bytes);
@@ -1734,18 +1724,10 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
 }
 
 // Matrix storage: zero-filled regions (one per array), so no result depends on what the
-// memory held before.  A program that creates a descriptor per likelihood evaluation
-// would map and unmap its memory each time with cudaMalloc: creating one of 1.1 GB took
-// 15 ms (up to 1 s when the host was busy), now 0.24 ms (the zero fill); requests of
-// 2,700, 27,000, 97,200 unknowns 12.6, 81.5, 322 ms -> 10.3, 78.3, 314.
+// memory held before.
 static cudaError_t dev_alloc(hicma_tlr_ctx *c, void **p, size_t bytes) {
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        cudaStreamSynchronize(c->stream);
-        cudaMemPoolTrimTo(c->pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-    }
+    cudaError_t e = cudaSetDevice(c->device);
+    if (e == cudaSuccess) e = (cudaError_t)c->regions->take(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
         return e;
@@ -1755,21 +1737,20 @@ static cudaError_t dev_alloc(hicma_tlr_ctx *c, void **p, size_t bytes) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return e;
 }
-// Work of any stream on the region is over before it is reused (the caller's streams too).
-static void dev_free(hicma_tlr_ctx *c, void *p) {
-    if (!p) return;
-    cudaDeviceSynchronize();
-    bc_remove(p);
-    cudaFreeAsync(p, c->stream);
+// Work of any stream of the context's device on the regions is over before they are
+// reused (the caller's streams too); after an error they are not reused.
+static void dev_free(hicma_tlr_ctx *c, std::initializer_list<void *> ps) {
+    cudaSetDevice(c->device);
+    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+    for (void *p : ps) {
+        if (!p) continue;
+        bc_remove(p);
+        c->regions->give(p, ok);
+    }
 }
 
 static void desc_free_device(hicma_tlr_desc *A) {
-    hicma_tlr_ctx *c = A->ctx;
-    dev_free(c, A->d_pts);
-    dev_free(c, A->d_band);
-    dev_free(c, A->d_lr);
-    dev_free(c, A->d_rank);
-    dev_free(c, A->d_linv);
+    dev_free(A->ctx, {A->d_pts, A->d_band, A->d_lr, A->d_rank, A->d_linv});
     A->d_pts = A->d_band = A->d_lr = A->d_linv = nullptr;
     A->d_rank = nullptr;
 }
@@ -1958,7 +1939,7 @@ int hicma_tlr_desc_create(hicma_tlr_ctx *c, int N, int NB, int maxrank, int band
         dev_alloc(c, (void **)&A->d_rank, (size_t)NT * NT * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         set_err("descriptor allocation failed (band %zu B, low-rank slots %zu B)", band_bytes, lr_bytes);
-        dev_free(c, A->d_band); dev_free(c, A->d_lr); dev_free(c, A->d_rank);
+        dev_free(c, {A->d_band, A->d_lr, A->d_rank});
         delete A;
         return HICMA_TLR_ERR_OOM;
     }
@@ -1968,7 +1949,7 @@ int hicma_tlr_desc_create(hicma_tlr_ctx *c, int N, int NB, int maxrank, int band
     const cudaError_t e = xfer(c, A->d_rank, A->h_rank.data(), (size_t)NT * NT * sizeof(int), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         set_err("rank map upload: %s", cudaGetErrorString(e));
-        dev_free(c, A->d_band); dev_free(c, A->d_lr); dev_free(c, A->d_rank);
+        dev_free(c, {A->d_band, A->d_lr, A->d_rank});
         delete A;
         return HICMA_TLR_ERR_CUDA;
     }
@@ -2007,10 +1988,11 @@ int hicma_tlr_desc_copy(hicma_tlr_ctx *c, const hicma_tlr_desc *src, hicma_tlr_d
                   src->slot_band == dst->slot_band,
               "descriptor shapes differ (N, NB, maxrank and the band it was created with must match)");
     std::lock_guard<std::recursive_mutex> lk(c->mu);
+    CUDA_TRY(cudaSetDevice(c->device));
     const size_t NB = src->NB, NT = src->NT;
     if (dst->band_alloc != src->band_alloc) {
         // the source's band was widened (band regeneration): the copy adopts it
-        dev_free(c, dst->d_band);
+        dev_free(c, {dst->d_band});
         dst->d_band = nullptr;
         const size_t bytes = NT * src->band_alloc * NB * NB * sizeof(double);
         if (dev_alloc(c, (void **)&dst->d_band, bytes) != cudaSuccess) {
@@ -2031,7 +2013,7 @@ int hicma_tlr_desc_copy(hicma_tlr_ctx *c, const hicma_tlr_desc *src, hicma_tlr_d
     dst->factored = src->factored;
     if (src->d_pts) {
         if (!dst->d_pts || dst->ndim != src->ndim) {
-            dev_free(c, dst->d_pts);
+            dev_free(c, {dst->d_pts});
             CUDA_TRY(dev_alloc(c, (void **)&dst->d_pts, (size_t)src->ndim * src->N * sizeof(double)));
         }
         dst->ndim = src->ndim;
@@ -2109,7 +2091,7 @@ static int set_points(hicma_tlr_ctx *c, hicma_tlr_desc *A, const hicma_tlr_probl
         points = h.data();
     }
     if (!A->d_pts || A->ndim != ndim) {
-        dev_free(c, A->d_pts);
+        dev_free(c, {A->d_pts});
         A->d_pts = nullptr;
         CUDA_TRY(dev_alloc(c, (void **)&A->d_pts, (size_t)ndim * A->N * sizeof(double)));
     }
@@ -2569,7 +2551,7 @@ int hicma_tlr_band_regenerate(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, con
     band_size = std::min(band_size, NT);
     TRY(ctx_sync(c));
     if (band_size > A->band_alloc) {
-        dev_free(c, A->d_band);
+        dev_free(c, {A->d_band});
         A->d_band = nullptr;
         const size_t bytes = (size_t)NT * band_size * NB * (size_t)NB * sizeof(double);
         if (dev_alloc(c, (void **)&A->d_band, bytes) != cudaSuccess) {
@@ -3708,9 +3690,9 @@ int hicma_tlr_check(hicma_tlr_ctx *c, hicma_tlr_desc *L, const hicma_tlr_problem
         }
     };
     const int nblk = 1024;
-    if (cudaMalloc(&DL, N * N * sizeof(double)) != cudaSuccess || cudaMalloc(&DA, N * N * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&part, nblk * sizeof(double)) != cudaSuccess || cudaMalloc(&sc, 8 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&dinfo, sizeof(int)) != cudaSuccess) {
+    if (device_malloc((void **)&DL, N * N * sizeof(double)) || device_malloc((void **)&DA, N * N * sizeof(double)) ||
+        device_malloc((void **)&part, nblk * sizeof(double)) || device_malloc((void **)&sc, 8 * sizeof(double)) ||
+        device_malloc((void **)&dinfo, sizeof(int))) {
         cudaGetLastError();
         cleanup();
         set_err("check: allocation of dense N x N buffers failed (N = %zu)", N);
@@ -3733,7 +3715,7 @@ int hicma_tlr_check(hicma_tlr_ctx *c, hicma_tlr_desc *L, const hicma_tlr_problem
     launch_sumsq(DA, nullptr, (int)N, (int)N, (long long)N, 0, part, nblk, sc + 1, c->stream);
     double h[4] = {0, 0, 0, 0};
     if (A0 && res_diff) {
-        if (cudaMalloc(&D0, N * N * sizeof(double)) != cudaSuccess) {
+        if (device_malloc((void **)&D0, N * N * sizeof(double))) {
             cudaGetLastError();
             D0 = nullptr;
             cleanup();
@@ -3771,7 +3753,15 @@ int hicma_tlr_k_cov(const hicma_tlr_problem *prob, const double *d_points, int N
     CovTask t{d_out, ld, r0, c0, nr, nc};
     CovTask *dt = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
-    CUDA_TRY(cudaMallocAsync(&dt, sizeof(CovTask), st));
+    cudaError_t e = cudaMallocAsync(&dt, sizeof(CovTask), st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        int dev = 0;
+        cudaGetDevice(&dev);
+        device_regions(dev)->trim();
+        e = cudaMallocAsync(&dt, sizeof(CovTask), st);
+    }
+    CUDA_TRY(e);
     CUDA_TRY(cudaMemcpyAsync(dt, &t, sizeof t, cudaMemcpyHostToDevice, st));
     launch_cov_batched(p, dt, 1, nr, nc, st);
     CUDA_TRY(cudaGetLastError());
@@ -3831,7 +3821,7 @@ int hicma_tlr_k_wait_probe(long long polls0, long long polls1, int nblocks, doub
               "wait probe: 1..2^26 polls");
     cudaStream_t st = (cudaStream_t)stream;
     int *buf = nullptr;   // [0] timeout flag, then cnt: [1] ticket, [2] abort, [3..] counters
-    CUDA_TRY(cudaMalloc(&buf, (3 + 64) * sizeof(int)));
+    CUDA_TRY((cudaError_t)device_malloc((void **)&buf, (3 + 64) * sizeof(int)));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int flags[3] = {0, 0, 0};
     float ms = 0.f;

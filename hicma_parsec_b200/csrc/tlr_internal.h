@@ -100,6 +100,11 @@ struct SkinnyTask {
 constexpr int SKINNY_MAX_TASKS = 32768;   // grid.y
 void launch_skinny_batched(const SkinnyTask *d_tasks, int ntasks, int mmax, int nmax, int kmax, cudaStream_t st);
 
+// -------------------------------------------------------- device memory ----
+// cudaMalloc on the current device; when memory is short, the regions kept for the next
+// descriptors are freed first.  0, or the cudaError_t.
+int device_malloc(void **p, size_t bytes);
+
 // ------------------------------------------------------------ generation ----
 struct CovTask {
     double *out;
