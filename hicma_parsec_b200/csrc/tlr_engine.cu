@@ -825,7 +825,10 @@ int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
 // well enough conditioned for; R takes both rounds.  The products are batched
 // DMMA launches over all tasks, so a few wide stacks still fill the device (one
 // CTA per stack and SIMT reflectors before: 3 stacks of nb 1350 and K about 650
-// took 28 ms for the QRs and 18 ms for the Q application).
+// took 28 ms for the QRs and 18 ms for the Q application).  A stack wider than
+// tall has a full basis after nb columns: the others are only projected on it.  (As
+// blocks they would become unit vectors of rounding errors inside the basis, and the
+// projection of the next block would take those directions out twice.)
 // Scratch per task: Z nb x BQ_W, S2 K x BQ_W, R1 and R2 BQ_W x BQ_W.
 constexpr int BQ_W = 64;
 struct BQTask {
@@ -881,9 +884,9 @@ int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
         std::vector<GemmTask> u1, u2, r2;
         std::vector<CQTask> q1, q2;
         for (const BQTask &t : v) {
-            const int bw = bq_width(t.K - t.k0), j = t.k0 + b * bw;
-            if (j >= t.K) continue;
-            const int w = std::min(bw, t.K - j), nb = t.nb, K = t.K;
+            const int kq = std::min(t.K, t.nb), bw = bq_width(kq - t.k0), j = t.k0 + b * bw;
+            if (j >= kq) continue;
+            const int w = std::min(bw, kq - j), nb = t.nb, K = t.K;
             double *W = t.Q + (size_t)nb * j, *Rj = t.R + (size_t)j * K;
             CQTask f{W, nullptr, t.Z, j ? t.R1 : Rj, W, nb, w, 0, nb, nb};
             f.ldr = j ? w : K;
@@ -910,6 +913,11 @@ int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
         TRY(run_rcholqr(c, q2, P_QR));
         TRY(run_gemms(c, r2, false, P_PROJ));
     }
+    std::vector<GramTask> rest;
+    for (const BQTask &t : v)
+        if (t.K > t.nb)
+            rest.push_back(GramTask{t.Q, t.Q + (size_t)t.nb * t.nb, t.R + (size_t)t.nb * t.K, t.nb, t.nb, t.K - t.nb, t.K});
+    TRY(run_grams(c, rest, P_PROJ));
     v.clear();
     return 0;
 }
@@ -1040,20 +1048,30 @@ struct RecompTask {
     const double *na = nullptr, *nb = nullptr;
 };
 
+// QRs of an update of K stacked columns: one randomized CholeskyQR a side, by blocks, or
+// Householder.  Only the blocks stop at a full basis: a CholeskyQR forms K columns, and
+// past nb of them a reflector has no rows.
+enum QRPath { QR_CHOL, QR_BLOCK, QR_HOUSEHOLDER };
+QRPath recomp_path(const hicma_tlr_ctx *c, int nb, int K) {
+    if (K > nb) return QR_BLOCK;
+    return !c->cholqr ? QR_HOUSEHOLDER : K <= rcholqr_kmax() ? QR_CHOL : QR_BLOCK;
+}
+
 // Workspace of one low-rank update (K = rc + ra).
 size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
     const int K = t.rc + t.ra, rc = t.rc, ra = t.ra;
     auto A = [](size_t n) { return align_up(sizeof(double) * n + 1); };
+    const QRPath path = recomp_path(c, nb, K);
     size_t b = 0;
     b += A((size_t)nb * K) * 2;                          // Us (U side's Q), Vs = [Cv | -Y]
     b += A((size_t)K * K) * 6;                           // RU, SU, T1, RV, Rc^-1 and Rc^-1 U_r
-    if (!c->cholqr) {                                    // Householder QRs
+    if (path == QR_HOUSEHOLDER) {
         const int pb = qr_panel_width(nb);
         const size_t npk = (size_t)(K + pb - 1) / pb + 1, npa = (size_t)(ra + pb - 1) / pb + 1;
         b += A((size_t)nb * K);                          // Vk
         b += A(ra) + A(K) + A(npa * pb * pb) + A(npk * pb * pb);  // tau, T factors of Wu and Vs
         b += A((size_t)rc * ra) * 2;                     // Pu, Pu2
-    } else if (K > rcholqr_kmax()) {
+    } else if (path == QR_BLOCK) {
         b += A((size_t)nb * K) + 2 * bq_ws_bytes(nb, K); // Vk, block QRs
     }
     if (K > core_smem_kmax()) b += A(core_work_doubles(K));
@@ -1159,11 +1177,12 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             if (K == 0) { cores.push_back(ct); continue; }
             // Stacks up to rcholqr_kmax() columns: both QRs by randomized
             // CholeskyQR (U side [Cu, Au] read in place, Q_U = Y Rc^-1 kept
-            // factored; V side R only); wider stacks: block Gram-Schmidt QRs, on the
-            // U side starting from the orthonormal Cu.  With HICMA_TLR_QR=householder:
-            // Au projected on Cu + Householder on the U side, Householder on the V side.
-            const bool cq = c->cholqr && K <= rcholqr_kmax();
-            const bool bq = c->cholqr && !cq;
+            // factored; V side R only); wider stacks, and those wider than tall: block
+            // Gram-Schmidt QRs, on the U side starting from the orthonormal Cu.  With
+            // HICMA_TLR_QR=householder: Au projected on Cu + Householder on the U side,
+            // Householder on the V side.
+            const QRPath path = recomp_path(c, nb, K);
+            const bool cq = path == QR_CHOL, bq = path == QR_BLOCK;
             double *Vs = ws_alloc<double>(c, (size_t)nb * K);
             double *Us = ws_alloc<double>(c, (size_t)nb * K);    // CholeskyQR path: Y of the U side
             double *RU = ws_alloc<double>(c, (size_t)K * K);
