@@ -29,8 +29,8 @@ TLR_HD int wide_ncl(int K, int cs) { return (K + cs - 1) / cs; }
 
 // Offsets in doubles.  Shared memory: sigl (ncl: squared norms of the CTA's columns),
 // then, as `place` says, hv (K: the pivot column) and T (ncl x K).  Scratch of the task:
-// X (K x (K + WP)), sig (K), T (K x (K + W_CSMAX), its columns by CTA), the rotation
-// flags (64).  Without W_HV_SHARED, hv lies in X's columns past K, which are free until
+// X (K x (K + WP)), sig (K), T if it is here (K x (K + W_CSMAX), its columns by CTA), the
+// rotation flags (64).  Without W_HV_SHARED, hv lies in X's columns past K, which are free until
 // the QR is over.  The sorted values (K doubles and K ints) come last: over the CTA's T
 // in shared memory, or over T in the scratch.
 struct WideLayout {
@@ -43,17 +43,12 @@ TLR_HD WideLayout wide_layout(int K, int cs, int rank, int place) {
     w.X = 0;
     w.sig = k * (k + WP);
     const size_t Tg = w.sig + k;
-    w.flags = Tg + k * (k + W_CSMAX);
+    w.flags = place & W_T_SHARED ? Tg : Tg + k * (k + W_CSMAX);
     w.sigl = 0;
     w.hv = place & W_HV_SHARED ? ncl : k * k + r * k;
     w.T = place & W_T_SHARED ? ncl + k + ((ncl + k) & 1) : Tg + r * ncl * k;
     w.sort = place & W_T_SHARED ? 0 : Tg + r * 2 * k;
     return w;
-}
-
-// Scratch of a core (doubles).
-TLR_HD size_t wide_work_doubles(int K) {
-    return (size_t)K * (K + WP) + (size_t)K * (K + W_CSMAX) + (size_t)K + 64;
 }
 
 // Shared memory of a launch whose widest core has K columns (bytes): the pivoted QR's
@@ -78,5 +73,17 @@ TLR_HD int wide_place(int K, int cs, size_t limit) {
 // pairs, k about K / 2) and enough shared memory for T: 4 up to K = 160, 8 up
 // to 448, then 16 (the non-portable maximum).
 TLR_HD int wide_cluster(int K) { return K <= 160 ? 4 : K <= 448 ? 8 : W_CSMAX; }
+
+// Launches hold cores of one of the widths up to 160, up to 448 and above.
+constexpr int W_EDGE1 = 160, W_EDGE2 = 448;
+
+// Scratch of a core (doubles) under a shared memory limit: without T where every launch
+// that the core can be part of has it in shared memory.
+TLR_HD size_t wide_work_doubles(int K, size_t limit) {
+    const size_t k = (size_t)K;
+    const int edge = K <= W_EDGE1 ? W_EDGE1 : W_EDGE2;
+    const bool t_shared = K <= W_EDGE2 && (wide_place(edge, wide_cluster(edge), limit) & W_T_SHARED);
+    return k * (k + WP) + k + 64 + (t_shared ? 0 : k * (k + W_CSMAX));
+}
 
 }  // namespace tlr

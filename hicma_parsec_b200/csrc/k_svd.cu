@@ -923,12 +923,12 @@ void launch_small(const CoreTask *d, int n, const CoreParams &p, cudaStream_t st
 // 65 to SMALL_KMAX columns take either kernel, so they bring scratch.
 int core_smem_kmax() { return 64; }
 
-size_t core_work_doubles(int K) { return wide_work_doubles(K); }
+size_t core_work_doubles(int K, size_t smem_limit) { return wide_work_doubles(K, std::min(smem_limit, W_SMEM_MAX)); }
 
 int core_bucket(int K, bool cluster) {
     if (K <= 64) return K <= 16 ? 16 : K <= 32 ? 32 : K <= 48 ? 48 : 64;
     if (K <= SMALL_KMAX && !cluster) return K <= 80 ? 80 : SMALL_KMAX;
-    return K <= 160 ? 160 : K <= 448 ? 448 : 1 << 30;
+    return K <= W_EDGE1 ? W_EDGE1 : K <= W_EDGE2 ? W_EDGE2 : 1 << 30;
 }
 int core_one_cta_kmax() { return SMALL_KMAX; }
 

@@ -453,7 +453,7 @@ static int bc_qapply(const std::vector<QApplyTask> &v, int m_max) {
     return 0;
 }
 
-static int bc_cores(const std::vector<CoreTask> &v) {
+static int bc_cores(const hicma_tlr_ctx *c, const std::vector<CoreTask> &v) {
 #ifdef TLR_BOUNDS_CHECK
     for (size_t i = 0; i < v.size(); ++i) {
         const CoreTask &t = v[i];
@@ -461,12 +461,12 @@ static int bc_cores(const std::vector<CoreTask> &v) {
         if (t.RU) BC(t.RU, bc_span(t.K, t.K, t.ldru), "core RU", i);
         BC(t.RV, bc_span(t.K, t.K, t.ldrv), "core RV", i);
         BC(t.SU, bc_span(t.K, t.K, t.K), "core SU", i);
-        if (t.work) BC(t.work, core_work_doubles(t.K) * sizeof(double), "core scratch", i);
+        if (t.work) BC(t.work, core_work_doubles(t.K, c->core_smem) * sizeof(double), "core scratch", i);
         if (t.rank_out) BC(t.rank_out, sizeof(int), "core rank", i);
         if (t.rank_task) BC(t.rank_task, sizeof(int), "core task rank", i);
     }
 #else
-    (void)v;
+    (void)c; (void)v;
 #endif
     return 0;
 }
@@ -641,6 +641,7 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
         const Launch &l = ls[q];
         c->cur = spread && q + 1 < ls.size() ? c->stream_core : st;
         CQTask *d = stage(c, l.tasks.data(), l.tasks.size());
+        if (!d) c->cur = st;
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
         const int n = (int)l.tasks.size(), hi = l.hi, cluster = l.cluster;
         const double fl = l.fl, by = l.by;
@@ -674,7 +675,7 @@ int run_qapply(hicma_tlr_ctx *c, std::vector<QApplyTask> &v, int m_max) {
 
 int run_core(hicma_tlr_ctx *c, std::vector<CoreTask> &v, int kmax, const CoreParams &cp, bool cluster) {
     if (v.empty()) return 0;
-    TRY(bc_cores(v));
+    TRY(bc_cores(c, v));
     CoreTask *d = stage(c, v.data(), v.size());
     if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
     const int n = (int)v.size();
@@ -1058,13 +1059,13 @@ QRPath recomp_path(const hicma_tlr_ctx *c, int nb, int K) {
 }
 
 // Workspace of one low-rank update (K = rc + ra).
-size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
+size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t, QRPath path) {
     const int K = t.rc + t.ra, rc = t.rc, ra = t.ra;
     auto A = [](size_t n) { return align_up(sizeof(double) * n + 1); };
-    const QRPath path = recomp_path(c, nb, K);
     size_t b = 0;
     b += A((size_t)nb * K) * 2;                          // Us (U side's Q), Vs = [Cv | -Y]
-    b += A((size_t)K * K) * 6;                           // RU, SU, T1, RV, Rc^-1 and Rc^-1 U_r
+    // RU, SU, T1; RV; Rc^-1 and Rc^-1 U_r
+    b += A((size_t)K * K) * (path == QR_HOUSEHOLDER ? 3 : path == QR_BLOCK ? 4 : 6);
     if (path == QR_HOUSEHOLDER) {
         const int pb = qr_panel_width(nb);
         const size_t npk = (size_t)(K + pb - 1) / pb + 1, npa = (size_t)(ra + pb - 1) / pb + 1;
@@ -1074,7 +1075,7 @@ size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t) {
     } else if (path == QR_BLOCK) {
         b += A((size_t)nb * K) + 2 * bq_ws_bytes(nb, K); // Vk, block QRs
     }
-    if (K > core_smem_kmax()) b += A(core_work_doubles(K));
+    if (K > core_smem_kmax()) b += A(core_work_doubles(K, c->core_smem));
     if (t.Bv) b += A((size_t)t.rb * t.ra);
     return b + 1024;
 }
@@ -1165,11 +1166,17 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         int *rank_task = d_rank_task_base;
         for (; i < tasks.size(); ++i) {
             const RecompTask &t = tasks[i];
-            if (recomp_ws_bytes(c, nb, t) > ws_free(c)) {
-                if (i == i0) { set_err("workspace too small for one recompression (K=%d)", t.rc + t.ra); return HICMA_TLR_ERR_OOM; }
-                break;
-            }
             const int rc = t.rc, ra = t.ra, K = rc + ra;
+            QRPath path = recomp_path(c, nb, K);
+            if (recomp_ws_bytes(c, nb, t, path) > ws_free(c)) {
+                if (i != i0) break;
+                // the block QRs need some 128 (nb + K) doubles more than the Householder ones
+                if (path == QR_BLOCK && K <= nb) path = QR_HOUSEHOLDER;
+                if (recomp_ws_bytes(c, nb, t, path) > ws_free(c)) {
+                    set_err("workspace too small for one recompression (K=%d)", K);
+                    return HICMA_TLR_ERR_OOM;
+                }
+            }
             CoreTask ct{};
             ct.rank_out = t.rank_dst;
             ct.rank_task = rank_task + (i - i0);
@@ -1181,13 +1188,12 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             // Gram-Schmidt QRs, on the U side starting from the orthonormal Cu.  With
             // HICMA_TLR_QR=householder: Au projected on Cu + Householder on the U side,
             // Householder on the V side.
-            const QRPath path = recomp_path(c, nb, K);
             const bool cq = path == QR_CHOL, bq = path == QR_BLOCK;
             double *Vs = ws_alloc<double>(c, (size_t)nb * K);
             double *Us = ws_alloc<double>(c, (size_t)nb * K);    // CholeskyQR path: Y of the U side
             double *RU = ws_alloc<double>(c, (size_t)K * K);
             double *SU = ws_alloc<double>(c, (size_t)K * K), *T1 = ws_alloc<double>(c, (size_t)K * K);
-            double *work = K > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(K)) : nullptr;
+            double *work = K > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(K, c->core_smem)) : nullptr;
             double *Yb = Vs + (size_t)nb * rc;
             if (rc > 0) copies.push_back(make_copy(t.Cv, nb, Vs, nb, nb, rc));
             if (ra > 0) {
@@ -2174,17 +2180,27 @@ struct CompressTask {
     int *rank_dst;
 };
 
-static size_t compress_ws_bytes(int nb, int s) {
-    const int pb = qr_panel_width(nb);
-    const size_t npan = (size_t)(s + pb - 1) / pb + 1;
-    size_t b = 0;
-    b += align_up(sizeof(double) * (size_t)nb * s + 1) * 4;   // Y, Q, W, Wkeep
-    b += align_up(sizeof(double) * (size_t)s + 1) * 2;
-    b += align_up(sizeof(double) * npan * pb * pb + 1) * 2;
-    b += align_up(sizeof(double) * (size_t)s * s + 1) * 4;    // SU (+ R_Y, R_W, Q^T Q of the CholeskyQR path)
-    if (s > rcholqr_kmax()) b += 2 * bq_ws_bytes(nb, s);      // block QRs
-    if (s > core_smem_kmax()) b += align_up(sizeof(double) * core_work_doubles(s) + 1);
+static size_t compress_ws_bytes(const hicma_tlr_ctx *c, int nb, int s, bool householder) {
+    auto A = [](size_t n) { return align_up(sizeof(double) * n + 1); };
+    size_t b = A((size_t)nb * s) * (householder ? 4 : 3);    // Y, Q, W, Wkeep
+    b += A((size_t)s * s) * (householder ? 1 : 4);           // SU; R_Y, R_W, Q^T Q
+    if (householder) {
+        const int pb = qr_panel_width(nb);
+        const size_t npan = (size_t)(s + pb - 1) / pb + 1;
+        b += A(s) * 2 + A(npan * pb * pb) * 2;
+    } else if (s > rcholqr_kmax()) {
+        b += 2 * bq_ws_bytes(nb, s);                         // block QRs
+    }
+    if (s > core_smem_kmax()) b += A(core_work_doubles(s, c->core_smem));
     return b + 1024;
+}
+
+// QRs of a compression with s samples, `other` bytes of the workspace besides: Householder
+// where they are asked for, and where the block QRs' scratch (128 (nb + s) doubles) does not
+// fit.
+static bool compress_householder(const hicma_tlr_ctx *c, int nb, int s, size_t other) {
+    if (!c->cholqr) return true;
+    return s > rcholqr_kmax() && compress_ws_bytes(c, nb, s, false) + other > c->ar->bytes - c->ar->off;
 }
 
 // Largest entry of |Q^T Q - I| accepted from the randomized CholeskyQR range
@@ -2195,11 +2211,10 @@ static size_t compress_ws_bytes(int nb, int s) {
 constexpr double GEN_ORTH_THR = 1e-10;
 
 // d_fail (optional, one int per task): the CholeskyQR path writes 1 where the
-// range finder's Q fails the orthogonality check, else 0.  force_hh: take the
-// Householder path whatever s is.
+// range finder's Q fails the orthogonality check, else 0 (null with householder).
 static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const double *Omega, int s,
                         std::vector<CompressTask> &tasks, const double *d_identity, int *d_rank_task_base,
-                        int *d_fail = nullptr, bool force_hh = false) {
+                        int *d_fail, bool householder) {
     const int pb = qr_panel_width(nb);
     const size_t npan = (size_t)(s + pb - 1) / pb + 1;
     const size_t mark = c->ar->off;
@@ -2216,11 +2231,11 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
         std::vector<GramTask> gq;
         // both QRs by randomized CholeskyQR (Q of Y formed, R of W only; above
         // rcholqr_kmax() samples by block Gram-Schmidt), U = Q_Y U_r as a GEMM
-        const bool cq = c->cholqr && !force_hh;
+        const bool cq = !householder;
         std::vector<BQTask> bqy, bqw;
         size_t i = i0;
         for (; i < tasks.size(); ++i) {
-            if (compress_ws_bytes(nb, s) > ws_free(c)) {
+            if (compress_ws_bytes(c, nb, s, householder) > ws_free(c)) {
                 if (i == i0) { set_err("workspace too small for one tile compression"); return HICMA_TLR_ERR_OOM; }
                 break;
             }
@@ -2245,7 +2260,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
                 CoreTask ct{};
                 ct.RU = nullptr; ct.RV = RW; ct.ldru = s; ct.ldrv = s;
                 ct.SU = SU;
-                ct.work = s > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(s)) : nullptr;
+                ct.work = s > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(s, c->core_smem)) : nullptr;
                 ct.rank_out = t.rank_dst; ct.rank_task = rt; ct.K = s;
                 cores.push_back(ct);
                 GemmTask gU = make_gemm(0, 0, nb, std::min(s, maxrank), s, 1.0, Y, nb, SU, s, 0.0, t.outU, nb);
@@ -2289,7 +2304,7 @@ static int run_compress(hicma_tlr_ctx *c, int nb, int maxrank, double tol, const
             double *tauY = ws_alloc<double>(c, s), *tauW = ws_alloc<double>(c, s);
             double *TY = ws_alloc<double>(c, npan * pb * pb), *TW = ws_alloc<double>(c, npan * pb * pb);
             double *SU = ws_alloc<double>(c, (size_t)s * s);
-            double *work = s > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(s)) : nullptr;
+            double *work = s > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(s, c->core_smem)) : nullptr;
             int *rt = d_rank_task_base + (i - i0);
             gy.push_back(make_gemm(0, 0, nb, s, nb, 1.0, t.A, nb, Omega, nb, 0.0, Y, nb));
             qy.push_back(QRTask{Y, tauY, TY, nb, s, nb});
@@ -2384,12 +2399,13 @@ int hicma_tlr_generate(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, int *Ar, c
     bool force_hh = false;
     while (!pending.empty()) {
         const size_t mark_round = c->ar->off;
-        const bool cq_round = c->cholqr && !force_hh;
-        int *dfail = cq_round ? ws_alloc<int>(c, pending.size()) : nullptr;
-        if (cq_round && !dfail) { set_err("workspace too small"); return HICMA_TLR_ERR_OOM; }
+        const size_t tile_bytes = align_up(sizeof(double) * (size_t)NB * NB + 1);
+        const bool hh = force_hh || compress_householder(c, NB, s, tile_bytes + align_up(sizeof(int) * pending.size() + 1));
+        int *dfail = hh ? nullptr : ws_alloc<int>(c, pending.size());
+        if (!hh && !dfail) { set_err("workspace too small"); return HICMA_TLR_ERR_OOM; }
         launch_set_identity(Ident, s, s, c->stream);
         TRY(check_launch(c));
-        const size_t per_tile = align_up(sizeof(double) * (size_t)NB * NB + 1) + compress_ws_bytes(NB, s);
+        const size_t per_tile = tile_bytes + compress_ws_bytes(c, NB, s, hh);
         const size_t chunk = std::max<size_t>(1, ws_free(c) / (per_tile + 4096));
         for (size_t t0 = 0; t0 < pending.size(); t0 += chunk) {
             const size_t t1 = std::min(pending.size(), t0 + chunk);
@@ -2410,8 +2426,7 @@ int hicma_tlr_generate(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, int *Ar, c
                 launch_cov_batched(cp, dcov, (int)cov.size(), NB, NB, c->stream);
             }
             TRY(check_launch(c));
-            TRY(run_compress(c, NB, maxrank, tol, Omega, s, comp, Ident, rtask, dfail ? dfail + t0 : nullptr,
-                             force_hh));
+            TRY(run_compress(c, NB, maxrank, tol, Omega, s, comp, Ident, rtask, dfail ? dfail + t0 : nullptr, hh));
             c->ar->off = mark;
         }
         std::vector<int> fails;
@@ -3939,7 +3954,8 @@ int hicma_tlr_k_compress(hicma_tlr_ctx *c, int nb, const double *d_A, double *d_
     int *d_fail = ws_alloc<int>(c, 1);
     if (!d_fail) { set_err("workspace too small"); return HICMA_TLR_ERR_OOM; }
     CUDA_TRY(cudaMemsetAsync(d_fail, 0, sizeof(int), c->stream));
-    TRY(run_compress(c, nb, maxrank, tol, Omega, s, v, Ident, d_r + 1, d_fail));
+    const bool hh = compress_householder(c, nb, s, 0);
+    TRY(run_compress(c, nb, maxrank, tol, Omega, s, v, Ident, d_r + 1, hh ? nullptr : d_fail, hh));
     int fail = 0;
     CUDA_TRY(cudaMemcpyAsync(&fail, d_fail, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     TRY(ctx_sync(c));

@@ -295,7 +295,7 @@ struct CoreTask {
     const double *RU;    // K x K upper (ld ldru), nullptr = identity
     const double *RV;    // K x K upper (ld ldrv)
     double *SU;          // out: left singular vectors sorted by decreasing sigma, rank columns (ld K)
-    double *work;        // core_work_doubles(K) doubles when K > core_smem_kmax()
+    double *work;        // core_work_doubles() doubles when K > core_smem_kmax()
     int *rank_out;       // rank map entry (may be null)
     int *rank_task;      // per-task rank for the apply steps
     int K, ldru, ldrv;
@@ -311,8 +311,8 @@ struct CoreParams {
 };
 // Cores up to this K need no scratch in global memory.
 int core_smem_kmax();
-// Global scratch (doubles) of one core with K > core_smem_kmax().
-size_t core_work_doubles(int K);
+// Global scratch (doubles) of one core with K > core_smem_kmax(); smem_limit as for the launch.
+size_t core_work_doubles(int K, size_t smem_limit);
 // Launch bucket of a core (the widest K of its kernel instance or cluster size).
 // Cores between core_smem_kmax() and core_one_cta_kmax() run on a cluster of
 // CTAs each if `cluster` is set, else on one CTA.

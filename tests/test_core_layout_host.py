@@ -32,9 +32,9 @@ static int check(int K, int cs, const char *what, size_t limit, const std::vecto
     return 0;
 }
 // a task of K columns in a launch whose widest has kmax, laid out as `place` says
-static int task(int K, int kmax, int cs, int place, size_t bytes) {
+static int task(int K, int cs, int place, size_t bytes, size_t limit) {
     const bool hv = place & W_HV_SHARED, t = place & W_T_SHARED;
-    const size_t k = (size_t)K, ncl = (size_t)wide_ncl(K, cs), sm = bytes / 8, work = wide_work_doubles(K);
+    const size_t k = (size_t)K, ncl = (size_t)wide_ncl(K, cs), sm = bytes / 8, work = wide_work_doubles(K, limit);
     std::vector<Part> qr_sm, qr_work, sort_sm, sort_work;
     qr_work = {{"X", 0, k * k}, {"sigma", wide_layout(K, cs, 0, place).sig, k}, {"flags", wide_layout(K, cs, 0, place).flags, 64}};
     sort_work = {{"X", 0, k * (k + WP)}, qr_work[1], qr_work[2]};
@@ -57,15 +57,18 @@ static int task(int K, int kmax, int cs, int place, size_t bytes) {
 }
 int main() {
     int bad = 0, seen = 0;
-    for (int kmax = 65; kmax <= 40000 && !bad; kmax += kmax < 9000 ? 1 : 37)
-        for (int cs : {4, 8, 16}) {
-            if (cs != wide_cluster(kmax) && !(cs == 8 && wide_cluster(kmax) == 16)) continue;   // 16 falls back to 8
-            const int place = wide_place(kmax, cs, W_SMEM_MAX);
-            const size_t bytes = wide_smem(kmax, cs, place);
-            seen |= 1 << place;
-            if (bytes > W_SMEM_MAX) { printf("K %d: %zu bytes\n", kmax, bytes); return 1; }
-            for (int K : {65, kmax / 2 > 65 ? kmax / 2 : 65, kmax - 1 > 65 ? kmax - 1 : 65, kmax}) bad |= task(K, kmax, cs, place, bytes);
-        }
+    for (size_t limit : {W_SMEM_MAX, (size_t)100000, (size_t)0})
+        for (int kmax = 65; kmax <= 40000 && !bad; kmax += kmax < 9000 ? 1 : 37)
+            for (int cs : {4, 8, 16}) {
+                if (cs != wide_cluster(kmax) && !(cs == 8 && wide_cluster(kmax) == 16)) continue;   // 16 falls back to 8
+                const int place = wide_place(kmax, cs, limit);
+                const size_t bytes = wide_smem(kmax, cs, place);
+                seen |= 1 << place;
+                if (bytes > W_SMEM_MAX) { printf("K %d: %zu bytes\n", kmax, bytes); return 1; }
+                // the narrowest, a middle and the widest core that this launch can hold
+                const int lo = kmax <= W_EDGE1 ? 65 : kmax <= W_EDGE2 ? W_EDGE1 + 1 : W_EDGE2 + 1;
+                for (int K : {lo, (lo + kmax) / 2, kmax}) bad |= task(K, cs, place, bytes, limit);
+            }
     if (seen != ((1 << 0) | (1 << W_HV_SHARED) | (1 << (W_HV_SHARED | W_T_SHARED)))) { printf("places %x\n", seen); return 1; }
     return bad;
 }
