@@ -1722,7 +1722,7 @@ int hicma_tlr_init(int device, size_t workspace_bytes, hicma_tlr_ctx **out) {
         return fail(e, what);
     }
     {
-        const size_t hi = std::min<size_t>(c->ws_bytes / 8, (size_t)512 << 20);
+        const size_t hi = std::min<size_t>(c->ws_bytes / 8, (size_t)512 << 20) / 256 * 256;   // main_ar's alignment
         c->hi_ar.base = c->d_ws;
         c->hi_ar.bytes = hi;
         c->main_ar.base = c->d_ws + hi;

@@ -98,3 +98,19 @@ def test_generate_in_the_smallest_workspace(nb, cap, acc, beta):
         assert abs(U0.shape[1] - U1.shape[1]) <= 1
         T = U0 @ V0.T
         assert np.linalg.norm(T - U1 @ V1.T) <= 2.0 * acc * np.linalg.norm(T)
+
+
+@pytest.mark.parametrize("odd", [1, 8, 100, 1234])
+def test_workspace_of_any_size(odd):
+    """A workspace that is no multiple of anything: its two parts start aligned."""
+    from hicma_parsec_b200 import tlr
+    prob = tlr.Problem(kind=2, beta=0.1, noise=0.1)
+    out = []
+    for ws in (64 << 20, (64 << 20) + odd):
+        with tlr.Context(0, ws) as ctx:
+            A = tlr.TLRMatrix(ctx, 1280, 256, 120, 1)
+            assert A.generate(prob, 1e-8) == 0
+            assert A.potrf(1e-8) == 0
+            out.append((A.logdet(), A.rank_map()))
+            A.close()
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
