@@ -8,7 +8,8 @@
 // straight into DMMA fragments (mma.sync m8n8k4 f64, four quads of loads in
 // flight per lane), then add their partials in warp order (deterministic).  A
 // triangular A is read only where it has entries.  Two warps a CTA for inner
-// dimensions up to 64 (the rank-wide factors), eight above.
+// dimensions up to 64 (the rank-wide factors); above, eight with 8 columns of C and
+// four with 32.
 // The batched GEMM used before walked a tile column's 2700-long inner dimension
 // in one CTA (about 170 us a step).  Device time of a log-likelihood with the 36 x
 // 36-tile factor of tile 2700: 41 -> 5 ms; a solve call of the 30 x 30-tile factor

@@ -3396,14 +3396,16 @@ int hicma_tlr_logdet(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *logdet) {
 // T: NT x maxrank x n scratch).  Three launches a step: the diagonal solve (into
 // the other of X and Z, so nothing is copied), the products V^T z of the column's
 // low-rank tiles with the dense tiles' updates, and the low-rank updates.  The
-// tasks of all steps are staged at once: their sizes are known on the host.
-static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, double *T, int n) {
+// tasks of all steps are staged at once: their sizes are known on the host.  With Z
+// null (too small a workspace) a diagonal solve goes to block (NB x n) and is copied
+// back: a fourth operation in each of the 2 NT steps.
+static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, double *block, double *T, int n) {
     const int NT = A->NT, NB = A->NB, N = A->N;
-    struct Step { size_t first; int cnt, mmax, kmax; };
+    struct Step { size_t first; int cnt, mmax, kmax, back; };   // back: block row to copy back, -1: none
     std::vector<SkinnyTask> all;
     std::vector<Step> steps;
-    auto close = [&](size_t first) {
-        Step s{first, (int)(all.size() - first), 0, 0};
+    auto close = [&](size_t first, int back = -1) {
+        Step s{first, (int)(all.size() - first), 0, 0, back};
         for (size_t i = first; i < all.size(); ++i) {
             s.mmax = std::max(s.mmax, all[i].m);
             s.kmax = std::max(s.kmax, all[i].k);
@@ -3412,14 +3414,14 @@ static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, 
     };
     for (int sweep = 0; sweep < 2; ++sweep) {
         const bool fw = sweep == 0;
-        double *src = fw ? X : Z, *dst = fw ? Z : X;   // updated right-hand sides, solved blocks
+        double *src = fw || !Z ? X : Z, *dst = fw && Z ? Z : X;   // updated right-hand sides, solved blocks
         for (int q = 0; q < NT; ++q) {
             const int k = fw ? q : NT - 1 - q;
             const double *yk = dst + (size_t)k * NB;
             size_t first = all.size();
-            all.push_back(SkinnyTask{A->linv(k), src + (size_t)k * NB, dst + (size_t)k * NB, NB, n, NB, NB, N, N,
-                                     fw ? 0 : 1, fw ? 1 : 2, 1.0, 0.0});
-            close(first);
+            all.push_back(SkinnyTask{A->linv(k), src + (size_t)k * NB, Z ? dst + (size_t)k * NB : block, NB, n, NB, NB, N,
+                                     Z ? N : NB, fw ? 0 : 1, fw ? 1 : 2, 1.0, 0.0});
+            close(first, Z ? -1 : k);
             std::vector<SkinnyTask> upd;
             first = all.size();
             for (int o = fw ? k + 1 : 0; o < (fw ? NT : k); ++o) {
@@ -3472,6 +3474,9 @@ static int solve_dev(hicma_tlr_ctx *c, hicma_tlr_desc *A, double *X, double *Z, 
                                       st.kmax, c->cur);
                 TRY(check_launch(c));
             }
+            if (st.back >= 0)
+                CUDA_TRY(cudaMemcpy2DAsync(X + (size_t)st.back * NB, (size_t)N * sizeof(double), block, NB * sizeof(double),
+                                           NB * sizeof(double), n, cudaMemcpyDeviceToDevice, c->cur));
         }
     }
     return 0;
@@ -3487,19 +3492,12 @@ int hicma_tlr_solve(hicma_tlr_ctx *c, hicma_tlr_desc *A, int nrhs, double *B, lo
     const size_t N = A->N;
     double *X = ws_alloc<double>(c, N * nrhs);
     double *T = ws_alloc<double>(c, (size_t)A->NT * A->maxrank * nrhs + 1);
-    if (!X || !T || !ws_alloc<double>(c, (size_t)A->NB * nrhs)) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
-    // the second right-hand-side buffer: as many columns as the arena has left (the
-    // critical-path arena, idle here, when that is not one)
-    int cols = (int)std::min<size_t>((size_t)nrhs, ws_free(c) / (N * sizeof(double) + 256));
-    double *Z = cols > 0 ? ws_alloc<double>(c, N * cols) : nullptr;
-    if (!Z) {
-        cols = (int)std::min<size_t>((size_t)nrhs, c->hi_ar.bytes / (N * sizeof(double)));
-        Z = (double *)c->hi_ar.base;
-        if (cols < 1) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
-    }
+    double *Z = ws_alloc<double>(c, N * nrhs);
+    double *block = Z ? nullptr : ws_alloc<double>(c, (size_t)A->NB * nrhs);
+    if (!X || !T || (!Z && !block)) { set_err("workspace too small (solve)"); return HICMA_TLR_ERR_OOM; }
     CUDA_TRY(cudaMemcpy2DAsync(X, N * sizeof(double), B, ldb * sizeof(double), N * sizeof(double), nrhs,
                                cudaMemcpyHostToDevice, c->stream));
-    for (int j = 0; j < nrhs; j += cols) TRY(solve_dev(c, A, X + N * j, Z, T, std::min(cols, nrhs - j)));
+    TRY(solve_dev(c, A, X, Z, block, T, nrhs));
     CUDA_TRY(cudaMemcpy2DAsync(B, ldb * sizeof(double), X, N * sizeof(double), N * sizeof(double), nrhs,
                                cudaMemcpyDeviceToHost, c->stream));
     TRY(ctx_sync(c));

@@ -114,3 +114,31 @@ def test_workspace_of_any_size(odd):
             out.append((A.logdet(), A.rank_map()))
             A.close()
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("nt, nb, band, nrhs", [(1, 96, 1, 1), (2, 100, 1, 3), (6, 128, 1, 1), (6, 128, 2, 8), (6, 130, 1, 9),
+                                                (5, 200, 3, 70)])
+def test_solve_in_the_smallest_workspace(nt, nb, band, nrhs):
+    """The right-hand sides, one block row of them and the low-rank products: what a solve
+    needs without a second copy of the right-hand sides.  Same products in the same
+    order as with one, so the same bits."""
+    from hicma_parsec_b200 import tlr
+    prob = tlr.Problem(kind=2, beta=0.1, noise=0.1)
+    n, cap = nt * nb, nb // 2 - 1
+    b = np.random.default_rng(n).standard_normal((n, nrhs))
+    small = workspace(arrays(n * nrhs, nt * cap * nrhs + 1, nb * nrhs))
+    with tlr.Context(0, 64 << 20) as ctx, tlr.Context(0, small) as tight:
+        A, B = tlr.TLRMatrix(ctx, n, nb, cap, band), tlr.TLRMatrix(tight, n, nb, cap, band)
+        info = A.generate(prob, 1e-7)
+        if info:
+            A.band_regenerate(prob, max(m - k for m, k in A.rejected_tiles()) + 1)
+        assert A.potrf(1e-7) == 0
+        B.copy_from(A)
+        x, y = A.solve(b.copy()), B.solve(b.copy())
+        assert np.array_equal(x, y)
+        # and it is the solution: the factor holds A to acc, the nugget 0.1 bounds its inverse
+        D = A.uncompress()
+        L = np.tril(D)
+        assert np.linalg.norm(L @ (L.T @ x) - b) <= 1e-9 * np.linalg.norm(b)
+        A.close()
+        B.close()
