@@ -978,7 +978,10 @@ int potrf_tile(hicma_tlr_ctx *c, double *A, int n, int lda, double *Linv, int ld
         // CTAs hold 106 KB of shared memory, which keeps the CholeskyQR kernels off their
         // SMs, and the tile is on the critical path of small panels only (2D, tile 2700:
         // 60 x 60 tiles 449 ms with 148 CTAs, 428 to 430 with 48 to 80, 447 with 24;
-        // 36 x 36 tiles 380, 365, 373; the tile alone 1.13, 1.7 to 1.5, 4.1 ms).
+        // 36 x 36 tiles 380, 365, 373; the tile alone 1.13, 1.7 to 1.5, 4.1 ms).  To the last
+        // panel: with all SMs for the last 6, 12 or 24 tiles 12 x 12 tiles take 44.9, 48.2, 48.2
+        // ms instead of 42.3, 36 x 36 179.5, 182.5, 187.2 instead of 177.1.  Without
+        // lookahead nothing runs beside it: 12 x 12 tiles 53.3 ms on all SMs, 57.3 on half.
         const int grid = c->potrf_grid > 0 ? c->potrf_grid : overlapped ? c->nsm / 2 : c->nsm;
         if (launch_potrf_tile(A, lda, n, Linv, ldl, D, cnt, d_info, info_base, c->d_flags + 3, grid, st)) {
             set_err("tile POTRF launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -2952,7 +2955,7 @@ static int factorize(hicma_tlr_ctx *c, hicma_tlr_desc *A, double acc, int fixed_
                 syrk_from[k + 1] = k + 1;
                 CUDA_TRY(cudaEventRecord(ev[P0], c->cur));
                 TRY(potrf_tile(c, A->dense(k + 1, k + 1), NB, NB, A->linv(k + 1), NB, d_info, (k + 1) * NB,
-                               NT - (k + 1) >= 6));
+                               lookahead));
                 CUDA_TRY(cudaEventRecord(ev[P1], c->cur));
                 CUDA_TRY(cudaEventRecord(evP, c->cur));
                 // the next diagonal tile's low-rank contributions of columns 0..k (all
