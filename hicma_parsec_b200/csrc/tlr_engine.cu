@@ -264,6 +264,19 @@ int ctx_sync(hicma_tlr_ctx *c) {
 
 void ws_reset(hicma_tlr_ctx *c) { c->ar->off = 0; }
 
+// After an error (rc < 0) that may have left launches on several streams and another
+// stream current: they are waited for, so that the next call starts on the context's
+// stream and has the workspace to itself.
+int settle(hicma_tlr_ctx *c, int rc) {
+    if (rc >= 0) return rc;
+    const std::string msg = g_err;
+    ctx_sync(c);
+    g_err = msg;
+    c->cur = c->stream;
+    c->ar = &c->main_ar;
+    return rc;
+}
+
 // Host <-> device transfers and clears, ordered on the context stream and
 // complete on return.  (cudaMemcpy and cudaMemset run on the legacy default
 // stream, which the context's non-blocking streams do not wait for, and a
@@ -641,7 +654,6 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
         const Launch &l = ls[q];
         c->cur = spread && q + 1 < ls.size() ? c->stream_core : st;
         CQTask *d = stage(c, l.tasks.data(), l.tasks.size());
-        if (!d) c->cur = st;
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
         const int n = (int)l.tasks.size(), hi = l.hi, cluster = l.cluster;
         const double fl = l.fl, by = l.by;
@@ -3189,7 +3201,8 @@ int hicma_tlr_dpotrf_L(hicma_tlr_ctx *c, int uplo, hicma_tlr_desc *A, int *Ar, d
     NvtxRange nv("HiCMA_dpotrf_L");
     CUDA_TRY(cudaSetDevice(c->device));
     const bool la = !(lookahead && *lookahead == 0);
-    const int info = factorize(c, A, acc, fixed_rank, maxrank, tileopcounters, opcounters, critical_path_time, verbose, la);
+    const int info = settle(c, factorize(c, A, acc, fixed_rank, maxrank, tileopcounters, opcounters, critical_path_time,
+                                         verbose, la));
     if (Ar) std::memcpy(Ar, A->h_rank.data(), (size_t)A->NT * A->NT * sizeof(int));
     return info;
 }
@@ -3926,7 +3939,7 @@ int hicma_tlr_k_lr_update(hicma_tlr_ctx *c, int nb, const double *d_Au, const do
     if (!d_r) { set_err("workspace too small"); return HICMA_TLR_ERR_OOM; }
     std::vector<RecompTask> v{RecompTask{d_Cu, d_Cv, *rc, d_Au, d_Av, ra, d_Bu, d_Bv, rb, d_Cu, d_Cv, d_r}};
     CUDA_TRY(cudaMemsetAsync(c->d_flags + 1, 0, sizeof(int), c->stream));
-    TRY(run_recompress(c, nb, v, acc, maxrank, fixed_rank, d_r + 1, 0.0));
+    TRY(settle(c, run_recompress(c, nb, v, acc, maxrank, fixed_rank, d_r + 1, 0.0)));
     int r = 0;
     CUDA_TRY(cudaMemcpyAsync(&r, d_r, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     TRY(ctx_sync(c));

@@ -34,3 +34,38 @@ def test_wrapping_ring_changes_nothing(monkeypatch, kind, n, nb, cap, acc, prec)
     for other in out[1:]:
         for x, y in zip(out[0], other):
             assert np.array_equal(np.asarray(x), np.asarray(y))
+
+
+def test_a_failed_factorization_leaves_the_context_usable(monkeypatch):
+    """Rings too small for the task arrays of one launch or another of a panel: the
+    factorization fails there, on the bulk or on the side stream, and the next solve is as
+    ever."""
+    from hicma_parsec_b200 import tlr
+    prob = tlr.Problem(kind=4, beta=0.1, noise=0.1)
+    n, nb, cap = 4800, 200, 99
+    b = np.random.default_rng(0).standard_normal((n, 2))
+    monkeypatch.delenv("HICMA_TLR_STAGE_BYTES", raising=False)
+    with tlr.Context(0, 1 << 30) as ctx:
+        A, F = tlr.TLRMatrix(ctx, n, nb, cap, 1), tlr.TLRMatrix(ctx, n, nb, cap, 1)
+        if A.generate(prob, 1e-6):
+            A.band_regenerate(prob, max(m - k for m, k in A.rejected_tiles()) + 1)
+        F.copy_from(A)
+        assert F.potrf(1e-6) == 0
+        x = F.solve(b.copy())
+        failed = 0
+        for size in range(4096, 49152, 4096):
+            monkeypatch.setenv("HICMA_TLR_STAGE_BYTES", str(size))
+            with tlr.Context(0, 1 << 30) as tight:
+                B, G = tlr.TLRMatrix(tight, n, nb, cap, 1), tlr.TLRMatrix(tight, n, nb, cap, 1)
+                B.copy_from(A)
+                G.copy_from(F)
+                try:
+                    assert B.potrf(1e-6) == 0
+                except tlr.TLRError as e:
+                    assert "staging failed" in str(e)
+                    failed += 1
+                assert np.array_equal(G.solve(b.copy()), x)
+                B.copy_from(A)
+                B.close()
+                G.close()
+        assert failed >= 3
