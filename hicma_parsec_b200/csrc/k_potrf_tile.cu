@@ -20,8 +20,9 @@
 // take tasks from it with an atomic ticket, so every task waits only on the
 // chain or on tasks already held by running CTAs, and the chain waits only on
 // tasks of earlier block columns, which the other CTAs take in list order: the
-// kernel makes progress with two or more CTAs, whether or not they are resident
-// together, and needs no cooperative launch.  Dependencies are per-block flags
+// kernel makes progress with two or more CTAs and needs no cooperative launch.  A CTA
+// that waits holds its place on an SM, so beside the chain a second one has to become
+// resident; it does when any block of another kernel ends.  Dependencies are per-block flags
 // released with a fence after the block is written and acquired by one thread
 // before the CTA reads (through L2: ld.global.cg).  Every wait is bounded; a wait
 // that gives up sets the timeout flag and the abort flag, and every CTA leaves

@@ -608,8 +608,10 @@ int run_rcholqr(hicma_tlr_ctx *c, std::vector<CQTask> &v, int cls = P_CHOLQR) {
     // one launch per width bucket (the kernel is instantiated per bucket); a bucket
     // joins the next wider one while both together leave half of the SMs free: the
     // launch then lasts as long as its widest matrix instead of one after the other.
-    // Few matrices share clusters of CTAs while those fit three quarters of the SMs
-    // (the tile POTRF holds the others).
+    // Few matrices share clusters of CTAs while those fit three quarters of the SMs: a
+    // cluster needs its SMs free within one GPC, so that about 32 clusters of 4 with 205 KB
+    // a CTA run at once (36 matrices of K = 64: 449 us in two waves of clusters of 4, 345 on
+    // clusters of 2).
     struct Launch {
         std::vector<CQTask> tasks;
         int hi, cluster;
@@ -988,7 +990,8 @@ int potrf_tile(hicma_tlr_ctx *c, double *A, int n, int lda, double *Linv, int ld
         if (Linv) CUDA_TRY(cudaMemset2DAsync(Linv, (size_t)ldl * sizeof(double), 0, sizeof(double) * n, n, st));
         // One CTA per SM when it runs alone.  Beside a panel's updates half of that: its
         // CTAs hold 106 KB of shared memory, which keeps the CholeskyQR kernels off their
-        // SMs, and the tile is on the critical path of small panels only (2D, tile 2700:
+        // SMs, and the tile is on the critical path of small panels only (2D, tile 2700,
+        // before the later changes to the chains beside it:
         // 60 x 60 tiles 449 ms with 148 CTAs, 428 to 430 with 48 to 80, 447 with 24;
         // 36 x 36 tiles 380, 365, 373; the tile alone 1.13, 1.7 to 1.5, 4.1 ms).  To the last
         // panel: with all SMs for the last 6, 12 or 24 tiles 12 x 12 tiles take 44.9, 48.2, 48.2
