@@ -840,10 +840,9 @@ int run_grams(hicma_tlr_ctx *c, std::vector<GramTask> &v, int cls) {
 // well enough conditioned for; R takes both rounds.  The products are batched
 // DMMA launches over all tasks, so a few wide stacks still fill the device (one
 // CTA per stack and SIMT reflectors before: 3 stacks of nb 1350 and K about 650
-// took 28 ms for the QRs and 18 ms for the Q application).  A stack wider than
-// tall has a full basis after nb columns: the others are only projected on it.  (As
-// blocks they would become unit vectors of rounding errors inside the basis, and the
-// projection of the next block would take those directions out twice.)
+// took 28 ms for the QRs and 18 ms for the Q application).  K <= nb: past a full
+// basis a block would become unit vectors of rounding errors inside it, and the next
+// block's projection would take those directions out twice.
 // Scratch per task: Z nb x BQ_W, S2 K x BQ_W, R1 and R2 BQ_W x BQ_W.
 constexpr int BQ_W = 64;
 struct BQTask {
@@ -874,34 +873,40 @@ int bq_width(int n) {
     return nblk ? ((n + nblk - 1) / nblk + 7) / 8 * 8 : BQ_W;
 }
 
-int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
-    if (v.empty()) return 0;
+int run_rinits(hicma_tlr_ctx *c, std::vector<RInitTask> &v) {
     for (size_t i = 0; i < v.size(); i += GRAM_MAX_TASKS) {
-        std::vector<RInitTask> ri;
+        const int n = (int)std::min<size_t>(v.size() - i, GRAM_MAX_TASKS);
         int kmax = 1;
-        for (size_t q = i; q < std::min(v.size(), i + GRAM_MAX_TASKS); ++q) {
-            ri.push_back(RInitTask{v[q].R, v[q].K, v[q].k0});
-            kmax = std::max(kmax, v[q].K);
+        for (int q = 0; q < n; ++q) {
+            kmax = std::max(kmax, v[i + q].K);
 #ifdef TLR_BOUNDS_CHECK
-            BC(v[q].R, bc_span(v[q].K, v[q].K, v[q].K), "block QR R", q);
+            BC(v[i + q].R, bc_span(v[i + q].K, v[i + q].K, v[i + q].K), "block QR R", i + q);
 #endif
         }
-        RInitTask *d = stage(c, ri.data(), ri.size());
+        RInitTask *d = stage(c, v.data() + i, (size_t)n);
         if (!d) { set_err("staging failed"); return HICMA_TLR_ERR_CUDA; }
-        const int n = (int)ri.size();
         TRY(issue(c, [=]() {
             launch_rinit(d, n, kmax, c->cur);
             return check_launch(c);
         }));
     }
+    v.clear();
+    return 0;
+}
+
+int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
+    if (v.empty()) return 0;
+    std::vector<RInitTask> ri;
+    for (const BQTask &t : v) ri.push_back(RInitTask{t.R, t.K, t.k0});
+    TRY(run_rinits(c, ri));
     for (int b = 0;; ++b) {
         std::vector<GramTask> g1, g2;
         std::vector<GemmTask> u1, u2, r2;
         std::vector<CQTask> q1, q2;
         for (const BQTask &t : v) {
-            const int kq = std::min(t.K, t.nb), bw = bq_width(kq - t.k0), j = t.k0 + b * bw;
-            if (j >= kq) continue;
-            const int w = std::min(bw, kq - j), nb = t.nb, K = t.K;
+            const int bw = bq_width(t.K - t.k0), j = t.k0 + b * bw;
+            if (j >= t.K) continue;
+            const int w = std::min(bw, t.K - j), nb = t.nb, K = t.K;
             double *W = t.Q + (size_t)nb * j, *Rj = t.R + (size_t)j * K;
             CQTask f{W, nullptr, t.Z, j ? t.R1 : Rj, W, nb, w, 0, nb, nb};
             f.ldr = j ? w : K;
@@ -928,11 +933,6 @@ int run_block_qr(hicma_tlr_ctx *c, std::vector<BQTask> &v) {
         TRY(run_rcholqr(c, q2, P_QR));
         TRY(run_gemms(c, r2, false, P_PROJ));
     }
-    std::vector<GramTask> rest;
-    for (const BQTask &t : v)
-        if (t.K > t.nb)
-            rest.push_back(GramTask{t.Q, t.Q + (size_t)t.nb * t.nb, t.R + (size_t)t.nb * t.K, t.nb, t.nb, t.K - t.nb, t.K});
-    TRY(run_grams(c, rest, P_PROJ));
     v.clear();
     return 0;
 }
@@ -1068,11 +1068,12 @@ struct RecompTask {
 };
 
 // QRs of an update of K stacked columns: one randomized CholeskyQR a side, by blocks, or
-// Householder.  Only the blocks stop at a full basis: a CholeskyQR forms K columns, and
-// past nb of them a reflector has no rows.
-enum QRPath { QR_CHOL, QR_BLOCK, QR_HOUSEHOLDER };
+// Householder.  None of them factors a stack that is wider than tall.  There the update
+// is formed as one nb x nb product D = [Cv, -Y] [Cu, Au]^T, and C = I D^T is recompressed
+// with the identity as the U side's Q, so that only D gets a (block) QR.
+enum QRPath { QR_CHOL, QR_BLOCK, QR_HOUSEHOLDER, QR_PRODUCT };
 QRPath recomp_path(const hicma_tlr_ctx *c, int nb, int K) {
-    if (K > nb) return QR_BLOCK;
+    if (K > nb) return QR_PRODUCT;
     return !c->cholqr ? QR_HOUSEHOLDER : K <= rcholqr_kmax() ? QR_CHOL : QR_BLOCK;
 }
 
@@ -1081,6 +1082,13 @@ size_t recomp_ws_bytes(const hicma_tlr_ctx *c, int nb, const RecompTask &t, QRPa
     const int K = t.rc + t.ra, rc = t.rc, ra = t.ra;
     auto A = [](size_t n) { return align_up(sizeof(double) * n + 1); };
     size_t b = 0;
+    if (path == QR_PRODUCT) {
+        b += A((size_t)nb * K) * 2 + A((size_t)nb * nb) * 5;    // Us, Vs; D, its QR's Q and R, SU, identity
+        b += bq_ws_bytes(nb, nb);
+        if (nb > core_smem_kmax()) b += A(core_work_doubles(nb, c->core_smem));
+        if (t.Bv) b += A((size_t)t.rb * t.ra);
+        return b + 1024;
+    }
     b += A((size_t)nb * K) * 2;                          // Us (U side's Q), Vs = [Cv | -Y]
     // RU, SU, T1; RV; Rc^-1 and Rc^-1 U_r
     b += A((size_t)K * K) * (path == QR_HOUSEHOLDER ? 3 : path == QR_BLOCK ? 4 : 6);
@@ -1170,6 +1178,8 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         std::vector<CopyTask> copies, copiesS, keeps;
         std::vector<GemmTask> g1, g2, g1s, g2s, gTU, gU, g3, g4, gUS, g3S, g4S;
         std::vector<BQTask> bqs;   // block QRs of the wide updates
+        std::vector<GemmTask> gD;  // products of the updates that are wider than tall
+        std::vector<RInitTask> ids;
         std::vector<CoreTask> coresS;
         std::vector<ProjTask> projs;
         std::vector<SelTask> sels;
@@ -1189,7 +1199,7 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             if (recomp_ws_bytes(c, nb, t, path) > ws_free(c)) {
                 if (i != i0) break;
                 // the block QRs need some 128 (nb + K) doubles more than the Householder ones
-                if (path == QR_BLOCK && K <= nb) path = QR_HOUSEHOLDER;
+                if (path == QR_BLOCK) path = QR_HOUSEHOLDER;
                 if (recomp_ws_bytes(c, nb, t, path) > ws_free(c)) {
                     set_err("workspace too small for one recompression (K=%d)", K);
                     return HICMA_TLR_ERR_OOM;
@@ -1202,16 +1212,17 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
             if (K == 0) { cores.push_back(ct); continue; }
             // Stacks up to rcholqr_kmax() columns: both QRs by randomized
             // CholeskyQR (U side [Cu, Au] read in place, Q_U = Y Rc^-1 kept
-            // factored; V side R only); wider stacks, and those wider than tall: block
-            // Gram-Schmidt QRs, on the U side starting from the orthonormal Cu.  With
-            // HICMA_TLR_QR=householder: Au projected on Cu + Householder on the U side,
-            // Householder on the V side.
-            const bool cq = path == QR_CHOL, bq = path == QR_BLOCK;
+            // factored; V side R only); wider stacks: block Gram-Schmidt QRs, on the
+            // U side starting from the orthonormal Cu.  With HICMA_TLR_QR=householder:
+            // Au projected on Cu + Householder on the U side, Householder on the V side.
+            const bool cq = path == QR_CHOL, bq = path == QR_BLOCK, dq = path == QR_PRODUCT;
+            const int Kc = dq ? nb : K;                          // order of the core
             double *Vs = ws_alloc<double>(c, (size_t)nb * K);
             double *Us = ws_alloc<double>(c, (size_t)nb * K);    // CholeskyQR path: Y of the U side
-            double *RU = ws_alloc<double>(c, (size_t)K * K);
-            double *SU = ws_alloc<double>(c, (size_t)K * K), *T1 = ws_alloc<double>(c, (size_t)K * K);
-            double *work = K > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(K, c->core_smem)) : nullptr;
+            double *RU = ws_alloc<double>(c, (size_t)Kc * Kc);
+            double *SU = ws_alloc<double>(c, (size_t)Kc * Kc), *T1 = dq ? nullptr : ws_alloc<double>(c, (size_t)K * K);
+            double *work = Kc > core_smem_kmax() ? ws_alloc<double>(c, core_work_doubles(Kc, c->core_smem)) : nullptr;
+            ct.K = Kc;
             double *Yb = Vs + (size_t)nb * rc;
             if (rc > 0) copies.push_back(make_copy(t.Cv, nb, Vs, nb, nb, rc));
             if (ra > 0) {
@@ -1261,6 +1272,28 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
                 bqs.push_back(bu);
                 bqs.push_back(bv);
                 ct.RV = RV; ct.ldrv = K;
+            } else if (dq) {
+                double *D = ws_alloc<double>(c, (size_t)nb * nb), *Dk = ws_alloc<double>(c, (size_t)nb * nb);
+                double *RV = ws_alloc<double>(c, (size_t)nb * nb);
+                if (rc > 0) copies.push_back(make_copy(t.Cu, nb, Us, nb, nb, rc));
+                if (ra > 0) copies.push_back(make_copy(t.Au, nb, Us + (size_t)nb * rc, nb, nb, ra));
+                gD.push_back(make_gemm(0, 1, nb, nb, K, 1.0, Vs, nb, Us, nb, 0.0, D, nb));
+                keeps.push_back(make_copy(D, nb, Dk, nb, nb, nb));
+                ids.push_back(RInitTask{RU, nb, nb});
+                BQTask bv;
+                if (!bq_make(c, bv, Dk, nb, 0, nb, RV)) { set_err("workspace too small (block QR)"); return HICMA_TLR_ERR_OOM; }
+                bqs.push_back(bv);
+                ct.RV = RV; ct.ldrv = nb;
+                ct.RU = nullptr; ct.ldru = nb; ct.SU = SU; ct.work = work;
+                coresS.push_back(ct);
+                // new U = I U_r, new V = D U_r
+                GemmTask u = make_gemm(0, 0, nb, std::min(nb, maxrank), nb, 1.0, RU, nb, SU, nb, 0.0, t.outU, nb);
+                u.n_dev = ct.rank_task;
+                gUS.push_back(u);
+                GemmTask w = make_gemm(0, 0, nb, std::min(nb, maxrank), nb, 1.0, D, nb, SU, nb, 0.0, t.outV, nb);
+                w.n_dev = ct.rank_task;
+                g4S.push_back(w);
+                continue;
             } else {
                 double *Vk = ws_alloc<double>(c, (size_t)nb * K);
                 const int pbw = qr_panel_width(nb);
@@ -1332,6 +1365,8 @@ int run_recompress(hicma_tlr_ctx *c, int nb, std::vector<RecompTask> &tasks, dou
         TRY(run_gemms(c, g1s, true, P_GEMM_Y));
         TRY(run_gemms(c, g2, false, P_GEMM_Y));
         TRY(run_gemms(c, g2s, true, P_GEMM_Y));
+        TRY(run_gemms(c, gD, false, P_GEMM_Y));
+        TRY(run_rinits(c, ids));
         // the device starts on these while the host prepares the rest
         TRY(batch.flush());
         const bool side = !coresS.empty();

@@ -37,3 +37,28 @@ def test_update_wider_than_tall(monkeypatch, mode, nb, rc, ra, lo):
     assert r == i + 1
     assert np.linalg.norm(U @ V.T - ref, 2) <= s[r] + 100 * K * EPS * s[0]
     assert np.abs(U.T @ U - np.eye(r)).max() <= 100 * K * EPS * s[0] / s[r - 1]
+
+
+@pytest.mark.parametrize("nb, rc, ra, what", [(100, 70, 70, "zero"), (100, 70, 70, "dependent"), (60, 40, 40, "zero"),
+                                              (150, 100, 120, "dependent"), (150, 20, 150, "zero"), (200, 0, 200, "zero"),
+                                              (140, 70, 70, "dependent"), (128, 64, 64, "dependent"), (300, 150, 150, "dependent"),
+                                              (71, 35, 36, "dependent"), (141, 70, 70, "dependent")])
+def test_new_directions_after_a_gap(nb, rc, ra, what):
+    """The first new columns bring nothing (zero, or copies of old ones), the last ones do: with
+    K > nb the basis is not full when nb columns are through, with K = nb the rounding errors
+    of the copies fill it exactly."""
+    from hicma_parsec_b200 import tlr
+    rng = np.random.default_rng(nb + rc)
+    K = rc + ra
+    Cu, Au, Av = orth(rng, nb, rc), orth(rng, nb, ra), orth(rng, nb, ra)
+    gap = min(ra - 10, max(rc, 40))
+    Au[:, :gap] = 0.0 if what == "zero" else Cu[:, np.arange(gap) % max(rc, 1)]
+    Cv, Y = orth(rng, nb, rc) * np.linspace(3.0, 1.0, rc), orth(rng, nb, ra) * np.linspace(2.0, 1.0, ra)
+    ref = Cu @ Cv.T - Au @ Y.T
+    s = np.linalg.svd(ref, compute_uv=False)
+    acc = 1e-6
+    with tlr.Context(0, 512 << 20) as ctx:
+        r, U, V = update(ctx, nb, Cu, Cv, Au, Av, Y, Av, acc, max(K, 1))
+    assert r == int((s >= acc).sum())
+    assert np.linalg.norm(U @ V.T - ref, 2) <= 100 * K * EPS * s[0] + (s[r] if r < len(s) else 0.0)
+    assert np.abs(U.T @ U - np.eye(r)).max() <= 100 * K * EPS * s[0] / s[r - 1]
