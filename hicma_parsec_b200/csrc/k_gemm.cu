@@ -19,6 +19,12 @@
 // (2-way conflicts): 2700^3 NT 22.8 -> 30.0, NN 20.8 -> 29.7, TN 17.4 -> 30.5
 // TFLOP/s; 10800^3 27.5 -> 33.4, 23.6 -> 33.2, 20.1 -> 34.3; 1000^3 13 -> 23.
 // Larger tiles (128 x 64, 128 x 128, 96 x 96) were slower at every size.
+// A single product takes two stages and four CTAs an SM instead of three and three where
+// waves of CTAs count more than the depth of the pipeline: k up to 128, or fewer waves
+// and k up to 512, or one wave instead of two.  NT, three and four CTAs an SM: 24 x 24
+// tiles, k = 16, 200, 1600 42, 75, 326 and 32, 61, 299 us; 32 x 32 tiles, k = 16, 400,
+// 1600 54, 156, 453 and 43, 139, 458; 25 x 25 tiles (two waves either way), k = 16, 400
+// 41, 106 and 40, 118.
 // A batch is a list of tasks whose output tiles are flattened into one grid
 // (prefix sums in tile_off).
 #include "tlr_internal.h"
@@ -58,8 +64,8 @@ struct OpTile {
 };
 template <int BX>
 constexpr int op_doubles() { return OpTile<BX, true>::D > OpTile<BX, false>::D ? OpTile<BX, true>::D : OpTile<BX, false>::D; }
-template <int BM_, int BN_>
-constexpr size_t gemm_smem() { return sizeof(double) * STAGES * (op_doubles<BM_>() + op_doubles<BN_>()); }
+template <int BM_, int BN_, int ST = STAGES>
+constexpr size_t gemm_smem() { return sizeof(double) * ST * (op_doubles<BM_>() + op_doubles<BN_>()); }
 
 // Rows x0.. (below xe) and inner indices k0.. (below ke) of an operand into its stage.
 template <int BX, bool KC, bool V16>
@@ -83,7 +89,7 @@ __device__ __forceinline__ void load_operand(double *sm, const double *X, int ld
 // One BM_ x BN_ output tile; four warps of 32 x 32 (2 x 2 for 64 x 64,
 // 4 x 1 for the narrow 128 x 32 tile used when n is a rank).  AK / BKC: op(A) /
 // op(B) is contiguous along the inner dimension (opA = 1, opB = 0).
-template <int BM_, int BN_, bool AK, bool BKC, bool V16>
+template <int BM_, int BN_, int ST, bool AK, bool BKC, bool V16>
 __device__ __forceinline__ void gemm_tile_op(double *sm, const GemmTask &t, int n, int i0, int j0) {
     using OA = OpTile<BM_, AK>;
     using OB = OpTile<BN_, BKC>;
@@ -110,15 +116,15 @@ __device__ __forceinline__ void gemm_tile_op(double *sm, const GemmTask &t, int 
         load_operand<BN_, BKC, V16>(sa + OA::D, t.B, t.ldb, j0, n, kt * BK, t.k);
     };
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
+    for (int s = 0; s < ST - 1; ++s) {
         if (s < ktiles) load(s, s);
         cp_async_commit();
     }
     int s = 0;
     for (int kt = 0; kt < ktiles; ++kt) {
-        cp_async_wait<STAGES - 2>();
+        cp_async_wait<ST - 2>();
         __syncthreads();   // the stage is complete, and the one loaded next is no longer read
-        if (kt + STAGES - 1 < ktiles) load(s == 0 ? STAGES - 1 : s - 1, kt + STAGES - 1);
+        if (kt + ST - 1 < ktiles) load(s == 0 ? ST - 1 : s - 1, kt + ST - 1);
         cp_async_commit();
         const double *sa = sm + s * (OA::D + OB::D), *sb = sa + OA::D;
         const double *pa = sa + (wm * 32 + g) * SI + tig * SKA, *pb = sb + (wn * 32 + g) * SJ + tig * SKB;
@@ -134,7 +140,7 @@ __device__ __forceinline__ void gemm_tile_op(double *sm, const GemmTask &t, int 
 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
         }
-        s = s + 1 == STAGES ? 0 : s + 1;
+        s = s + 1 == ST ? 0 : s + 1;
     }
 
     const double alpha = t.alpha, beta = t.beta;
@@ -157,7 +163,7 @@ __device__ __forceinline__ void gemm_tile_op(double *sm, const GemmTask &t, int 
     }
 }
 
-template <int BM_, int BN_>
+template <int BM_, int BN_, int ST = STAGES>
 __device__ __forceinline__ void gemm_tile(double *sm, const GemmTask &t, int tm, int tn) {
     const int i0 = tm * BM_, j0 = tn * BN_;
     if (t.lower && j0 >= i0 + BM_) return;
@@ -166,14 +172,14 @@ __device__ __forceinline__ void gemm_tile(double *sm, const GemmTask &t, int tm,
     if (j0 >= n) return;
     const bool v16 = (((size_t)t.A | (size_t)t.B) & 15) == 0 && ((t.lda | t.ldb) & 1) == 0;
     switch ((t.opA ? 4 : 0) | (t.opB ? 2 : 0) | (v16 ? 1 : 0)) {
-        case 0: gemm_tile_op<BM_, BN_, false, true, false>(sm, t, n, i0, j0); break;
-        case 1: gemm_tile_op<BM_, BN_, false, true, true>(sm, t, n, i0, j0); break;
-        case 2: gemm_tile_op<BM_, BN_, false, false, false>(sm, t, n, i0, j0); break;
-        case 3: gemm_tile_op<BM_, BN_, false, false, true>(sm, t, n, i0, j0); break;
-        case 4: gemm_tile_op<BM_, BN_, true, true, false>(sm, t, n, i0, j0); break;
-        case 5: gemm_tile_op<BM_, BN_, true, true, true>(sm, t, n, i0, j0); break;
-        case 6: gemm_tile_op<BM_, BN_, true, false, false>(sm, t, n, i0, j0); break;
-        default: gemm_tile_op<BM_, BN_, true, false, true>(sm, t, n, i0, j0); break;
+        case 0: gemm_tile_op<BM_, BN_, ST, false, true, false>(sm, t, n, i0, j0); break;
+        case 1: gemm_tile_op<BM_, BN_, ST, false, true, true>(sm, t, n, i0, j0); break;
+        case 2: gemm_tile_op<BM_, BN_, ST, false, false, false>(sm, t, n, i0, j0); break;
+        case 3: gemm_tile_op<BM_, BN_, ST, false, false, true>(sm, t, n, i0, j0); break;
+        case 4: gemm_tile_op<BM_, BN_, ST, true, true, false>(sm, t, n, i0, j0); break;
+        case 5: gemm_tile_op<BM_, BN_, ST, true, true, true>(sm, t, n, i0, j0); break;
+        case 6: gemm_tile_op<BM_, BN_, ST, true, false, false>(sm, t, n, i0, j0); break;
+        default: gemm_tile_op<BM_, BN_, ST, true, false, true>(sm, t, n, i0, j0); break;
     }
 }
 
@@ -196,9 +202,18 @@ __global__ void __launch_bounds__(NT, 3) k_gemm_batched(const GemmTask *__restri
     gemm_tile<BM_, BN_>(sm, t, local % t.tiles_m, local / t.tiles_m);
 }
 
-__global__ void __launch_bounds__(NT, 3) k_gemm_single(GemmTask t) {
+template <int ST, int CTAS>
+__global__ void __launch_bounds__(NT, CTAS) k_gemm_single(GemmTask t) {
     extern __shared__ __align__(16) double sm[];
-    gemm_tile<BM, BN>(sm, t, blockIdx.x, blockIdx.y);
+    gemm_tile<BM, BN, ST>(sm, t, blockIdx.x, blockIdx.y);
+}
+
+template <int ST, int CTAS>
+void launch_single(const GemmTask &t, dim3 grid, cudaStream_t st) {
+    constexpr size_t smem = gemm_smem<BM, BN, ST>();
+    if constexpr (smem > 48 * 1024)   // the limit without it
+        cudaFuncSetAttribute(k_gemm_single<ST, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_gemm_single<ST, CTAS><<<grid, NT, smem, st>>>(t);
 }
 
 // ---------------------------------------------------------------------------
@@ -314,8 +329,14 @@ void launch_gemm_batched_narrow(const GemmTask *d_tasks, const int *d_tile_off, 
 void launch_gemm_single(const GemmTask &t, cudaStream_t st) {
     if (t.m <= 0 || t.n <= 0) return;
     dim3 grid((t.m + BM - 1) / BM, (t.n + BN - 1) / BN);
-    cudaFuncSetAttribute(k_gemm_single, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<BM, BN>());
-    k_gemm_single<<<grid, NT, gemm_smem<BM, BN>(), st>>>(t);
+    if (t.k <= 128) return launch_single<2, 4>(t, grid, st);
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const long long tiles = (long long)grid.x * grid.y;
+    const long long waves3 = (tiles + 3 * nsm - 1) / (3 * nsm), waves4 = (tiles + 4 * nsm - 1) / (4 * nsm);
+    if (waves4 < waves3 && (t.k <= 512 || waves4 == 1)) launch_single<2, 4>(t, grid, st);
+    else launch_single<STAGES, 3>(t, grid, st);
 }
 
 }  // namespace tlr
